@@ -51,11 +51,11 @@ typedef struct mgpu_scene mgpu_scene; /* device-resident scene: tree, triangles,
 /* kd-tree build parameters, Milton's SAH (kdTreeAccel.cpp:722-877) with its knobs; Milton's
  * defaults (kdTreeAccel.h:97-104) are min_prims 3, max_depth 24, cost_traversal 1, empty_bias 0.9.
  * threads 0 = all cores.  The renderer's default traversal cost is MGPU_KD_COST_TRAVERSAL (a scene
- * file's kdCostTraversal still sets it): SAH weighs a node step against a triangle test, and on
- * this GPU the traversal kernels test a leaf's triangles with all lanes of a warp but descend
- * nodes with the few lanes whose rays are still descending, so a node step costs about three
- * tests (mid frame: cost 1 / 2 / 3 / 4 / 6 -> 270 / 283 / 288 / 286 / 277 Mpaths/s).  The tree
- * never changes a closest hit (only which of two equal-t triangles is reported).              */
+ * file's kdCostTraversal still sets it): a quarter fewer references than at Milton's 1 on the
+ * 1 M-triangle scene, so a shorter build and upload (0.4 against 0.5 s, 446 against 560 MB).  Rays
+ * traverse the 8-wide hierarchy of mgpu_scene_create; the tree answers the counted queries and
+ * decides near ties.  It never changes a closest hit (only which of two equal-t triangles is
+ * reported).                                                                                 */
 #define MGPU_KD_COST_TRAVERSAL 3.0
 typedef struct {
   uint32_t min_prims;
@@ -230,7 +230,9 @@ int mgpu_accel_serialize(const mgpu_accel *accel, int32_t *kind, float *split, i
                          int64_t *n_nodes, int64_t *n_prims);
 int mgpu_accel_destroy(mgpu_accel *accel);
 
-/* Upload accel + scene to the current device.  The triangle arrays uploaded are the ones the
+/* Upload accel + scene to the current device and build the 8-wide hierarchy that rays traverse there
+ * (device scratch of about 170 bytes per triangle for the duration of the call; a scene whose
+ * scratch does not fit is traversed through its kd-tree).  The triangle arrays uploaded are the ones the
  * accel captured at build time (tree layout with leaf-ordered triangle records, triangles by id,
  * shading records; page-locked on the first upload); desc supplies the materials and lights and
  * must describe the same triangles.  Returns after the copies complete.                   */
@@ -245,8 +247,8 @@ int mgpu_scene_device_bytes(const mgpu_scene_desc *desc, const mgpu_accel *accel
 /* Texel values of texture tex as the device holds them (after filtering): width*height*4
  * floats (colour maps: rgb, 0; bump maps: gx, gy, 0, 0).  Synchronises.  For tests. */
 int mgpu_scene_read_texels(const mgpu_scene *scene, int32_t tex, float *out, void *stream);
-/* Tuning: how many of the breadth-first top 16-byte pairs the traversal kernels stage in
- * shared memory per block (0 = none; clamped to what the builder laid out breadth-first). */
+/* Tuning: how many of the breadth-first top 16-byte pairs the kd-tree ray queries (the counted
+ * one, and scenes without the 8-wide hierarchy) stage in shared memory per block (0 = none; clamped to what the builder laid out breadth-first). */
 int mgpu_scene_set_top_pairs(mgpu_scene *scene, uint32_t n);
 
 /* Ray queries on device buffers (Scene::getIntersection / Scene::intersects).
@@ -255,8 +257,8 @@ int mgpu_scene_set_top_pairs(mgpu_scene *scene, uint32_t n);
  *   occluded: n bytes   (1 if any hit with tmin < t < tmax)                               */
 int mgpu_trace_closest(const mgpu_scene *scene, const float *d_rays, float *d_hits, int64_t n, void *stream);
 int mgpu_trace_any(const mgpu_scene *scene, const float *d_rays, uint8_t *d_occluded, int64_t n, void *stream);
-/* Same queries with per-ray traversal counters written to d_counts (n * 4 uint32:
- * nodes visited, leaf refs read, triangles tested, max stack depth) -- measurement only. */
+/* Same queries through the kd-tree, with per-ray traversal counters written to d_counts (n * 4
+ * uint32: nodes visited, leaf refs read, triangles tested, max stack depth) -- measurement only. */
 int mgpu_trace_closest_counted(const mgpu_scene *scene, const float *d_rays, float *d_hits, uint32_t *d_counts,
                                int64_t n, void *stream);
 
@@ -351,7 +353,8 @@ int mgpu_render_stats_get(mgpu_render_stats *out); /* stats of the last render o
  * ext[b] = live paths traced at bounce b, shadow[b] = shadow rays queued at bounce b.       */
 int mgpu_render_wave_queues(uint32_t *ext, uint32_t *shadow, int32_t max_bounces);
 /* Render with traversal counters: counts8 = extension {nodes, leaf refs, triangles, rays},
- * shadow {nodes, leaf refs, triangles, rays} summed over the render (synchronises).
+ * shadow {nodes, leaf refs, triangles, rays} summed over the render (synchronises): 8-wide nodes
+ * (kd-tree nodes where the kd-tree is traversed); leaf refs stay 0.
  * Measurement helper for the memory roofline; slower than mgpu_render.                   */
 int mgpu_render_counted(const mgpu_scene *scene, const mgpu_render_params *params, mgpu_film *film, uint64_t *counts8,
                         void *stream);
@@ -362,12 +365,10 @@ int mgpu_render_counted(const mgpu_scene *scene, const mgpu_render_params *param
 int mgpu_profile_enable(int enable);
 int mgpu_profile_read(double *ms6, uint64_t *launches6);
 /* Process-wide tuning knobs (results do not depend on them):
- *   "persistent"     0/1  persistent warp-level traversal with per-lane ray refill (default 0)
- *   "coop_leaf"      0..3 warp-shared leaf tests: the triangles of all the lanes' current leaves
- *                    are tested by the whole warp, 32 at a time; bit 0 = shadow (any-hit)
- *                    kernel, bit 1 = extension (closest-hit) kernel (default 3: both)
- *   "trav_block"     64 / 128 / 256  threads per block of the grid-stride and warp-shared
- *                    traversal kernels, at the same threads (and registers) per SM (default 256)
+ *   "wide"           0/1  traversal of the 8-wide hierarchy that mgpu_scene_create builds on the
+ *                    device (default 1); 0 = the kd-tree, one ray per lane
+ *   "persistent" 0/1, "coop_leaf" 0..3, "trav_block" 64 / 128 / 256: shapes of earlier kd-tree
+ *                    kernels; accepted and read back, they select nothing
  *   "bin_shadow"     0/1  counting-sort shadow rays by (light, origin cell) (default 1)
  *   "bin_extension"  0/1  counting-sort extension rays by (direction octant, origin cell) (default 1)
  *   "bin_min_paths"  n    waves of fewer paths are not binned (default 2^22)

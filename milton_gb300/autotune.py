@@ -1,8 +1,9 @@
 """Autotuner for the wavefront renderer: picks the wave size (paths in flight, i.e. queue
-capacity), the traversal kernel shape (grid-stride or persistent warps), queue binning and the
-traversal block size by timing a short calibration render of the actual requests (wave size x
-shape first, then the block size of the best), and caches the choice per workload size class.  Results never depend on these knobs (every path draws its own counter-based random
-numbers and each film sums its samples in sample order), only speed does."""
+capacity) and queue binning by timing a short calibration render of the actual requests, and caches
+the choice per workload size class.  Results never depend on these knobs (every path draws its
+own counter-based random numbers and each film sums its samples in sample order), only speed does.
+The "persistent" and "trav_block" entries select nothing any more (include/mgpu.h); they are kept at
+one value so that a configuration still names them."""
 from __future__ import annotations
 
 import itertools
@@ -11,8 +12,8 @@ import math
 from . import pathtracer as pt
 
 WAVES = (1 << 21, 1 << 22, 1 << 23, 1 << 24, 1 << 25, 1 << 26)
-SHAPES = ((0, 1, 1), (0, 1, 0), (0, 0, 1), (1, 1, 1), (0, 0, 0))  # (persistent, bin_shadow, bin_extension)
-BLOCKS = (64, 128, 256)  # threads per traversal block (grid-stride shapes)
+SHAPES = ((0, 1, 1), (0, 1, 0), (0, 0, 1), (0, 0, 0))  # (persistent, bin_shadow, bin_extension)
+BLOCKS = (256,)
 
 _cache: dict = {}
 

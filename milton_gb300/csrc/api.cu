@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "hd_wide.h"
 
 namespace mgpu {
 
@@ -85,7 +86,7 @@ static void register_staging(mgpu_accel *a) {
 // Offsets of the arrays in a scene's one device allocation (256-byte aligned each).
 struct SceneLayout {
   size_t off_pairs, off_refs, off_tris, off_shade, off_mats, off_lights, off_uv, off_texrec, off_texels, off_sph,
-      off_err, total;
+      off_wnodes, off_wtris, off_wscratch, off_err, total;
 };
 // uv_tris: triangles with uploaded uvs (0 or all); ntex textures holding texels texels in all;
 // nsph analytic spheres (2 float4 each, and 3 shading records after the triangles')
@@ -103,7 +104,10 @@ static SceneLayout scene_layout(const mgpu_accel *a, int32_t nmat, int32_t nligh
   L.off_texrec = align_up(L.off_uv + (size_t)std::max<int64_t>(uv_tris, 0) * 3 * sizeof(float2), 256);
   L.off_texels = align_up(L.off_texrec + (size_t)std::max(ntex, 0) * 2 * sizeof(float4), 256);
   L.off_sph = align_up(L.off_texels + (size_t)texels * sizeof(float4), 256);
-  L.off_err = align_up(L.off_sph + (size_t)std::max(nsph, 0) * 2 * sizeof(float4), 256);
+  L.off_wnodes = align_up(L.off_sph + (size_t)std::max(nsph, 0) * 2 * sizeof(float4), 256);
+  L.off_wtris = align_up(L.off_wnodes + (size_t)wide_node_cap(a->ntri) * kWideWords * sizeof(uint32_t), 256);
+  L.off_wscratch = align_up(L.off_wtris + (size_t)a->ntri * 3 * sizeof(F4), 256);
+  L.off_err = align_up(L.off_wscratch + wide_scratch(a->ntri), 256);
   L.total = L.off_err + 256;
   return L;
 }
@@ -487,6 +491,16 @@ int mgpu_scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void
   s->d_lights = (float *)(base + off_lights);
   s->nmat = desc->nmat;
   s->nlight = desc->nlight;
+  bool wide = false;
+  uint32_t wide_nodes = 0;
+  if (int rc = wide_build(s->view.tris, T, base + L.off_wnodes, (F4 *)(base + L.off_wtris), base + L.off_wscratch, st,
+                          &wide_nodes, &wide)) {
+    cudaFree(s->d_block);
+    delete s;
+    return rc;
+  }
+  s->view.wnodes = wide ? (const uint4 *)(base + L.off_wnodes) : nullptr;
+  s->view.wtris = wide ? (const F4 *)(base + L.off_wtris) : nullptr;
   // staging the top of the tree in shared memory costs more occupancy than it saves on GB300
   // (the L1 keeps those pairs anyway); mgpu_scene_set_top_pairs turns it on
   s->top_pairs = 0;

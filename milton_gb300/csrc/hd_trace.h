@@ -51,6 +51,10 @@ struct SceneView {
   uint64_t npairs, nrefs;
   const F4 *spheres;       // 2 per analytic sphere: (center, radius), world-to-object quaternion
   int32_t nsphere;         // spheres are primitives ntri .. ntri + nsphere - 1
+#if defined(__CUDACC__)
+  const uint4 *wnodes;     // 8-wide hierarchy (hd_wide.h), nullptr: none
+  const F4 *wtris;         // its triangle records, 3 per triangle
+#endif
 };
 
 struct Ray {
@@ -460,215 +464,6 @@ __device__ __forceinline__ void grid_trace(View view, const Pair *top, uint32_t 
     while (!trav_step<ANY, COUNT>(s, st, stack, top, ntop, cnt)) {
     }
     store(i, st.best_prim >= 0, st);
-  }
-}
-
-// Persistent warp-level traversal (Aila and Laine, "Understanding the Efficiency of Ray
-// Traversal on GPUs", HPG 2009): every lane owns one ray; after each leaf step, lanes whose
-// ray finished take new rays from a global counter with one warp-aggregated atomicAdd, so a
-// warp never idles behind its slowest ray.  All 32 lanes of every warp must call this.
-template <bool ANY, bool COUNT, bool SPH, class View, class Load, class Store>
-__device__ __forceinline__ void persistent_trace(View view, const Pair *top, uint32_t ntop, uint32_t n,
-                                                 uint32_t *fetch, Load load, Store store, TraceCounts *cnt,
-                                                 uint32_t &rays_done) {
-  const unsigned kFull = 0xFFFFFFFFu;
-  const int lane = threadIdx.x & 31;
-  TravState st;
-  TravEntry stack[kMaxStack];
-  const SceneView *sv = nullptr;
-  uint32_t idx = 0;
-  bool have = false, exhausted = false;
-  for (;;) {
-    bool need = !have && !exhausted;
-    unsigned m = __ballot_sync(kFull, need);
-    if (m) {
-      int leader = __ffs(m) - 1;
-      uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(fetch, (uint32_t)__popc(m));
-      base = __shfl_sync(kFull, base, leader);
-      if (need) {
-        uint32_t my = base + (uint32_t)__popc(m & ((1u << lane) - 1u));
-        if (my < n) {
-          idx = my;
-          sv = &view(idx);
-          Ray r;
-          load(idx, r);
-          ++rays_done;
-          if (trav_init<SPH>(*sv, r, top, ntop, st, ANY)) have = true;
-          else store(idx, st.best_prim >= 0, st);
-        } else {
-          exhausted = true;
-        }
-      }
-    }
-    if (__all_sync(kFull, exhausted && !have)) break;
-    if (have && trav_step<ANY, COUNT>(*sv, st, stack, top, ntop, cnt)) {
-      store(idx, st.best_prim >= 0, st);
-      have = false;
-    }
-  }
-}
-
-// Grid-stride traversal with the leaf triangles shared by the warp.  Every lane descends its own
-// ray to its next leaf; then the warp tests the triangles of all the lanes' leaves together, 32
-// (ray, triangle) pairs at a time, each test with the owning lane's ray (its shear constants,
-// tmin and current best), and the results go back to the owners: for a closest hit the smallest
-// (t, index in the leaf) per owner through a shared-memory atomicMin on wkey[32] (a per-warp array
-// in shared memory; reducing each owner's run of lanes with __reduce_min_sync instead measured 45 %
-// slower), for an any hit a bit per owner.  Lanes whose ray has
-// finished test other lanes' triangles instead of idling, so a leaf of many triangles no longer
-// holds the warp in a loop that few lanes execute.  The result of every ray is the one trav_step
-// gives: the winner is the smallest t below the ray's best, ties to the first triangle in the
-// leaf's order, and its owner re-runs that one test for t and barycentrics.
-// All 32 lanes of every warp must call this (rays are taken in warp-aligned rounds).
-// With wray / wk (per-warp shared memory: 64 float4, 32 words) each lane's ray constants for the
-// tests are written there once per ray and read by the testers, instead of living in registers
-// through the descent and travelling by shuffles.
-// SINGLE: every ray of the launch is in one scene, view(0), which the kernel passes from its
-// parameter space; the scene's pointers and bounds are then read as launch constants instead of
-// through a per-lane pointer into device memory.
-template <bool ANY, bool COUNT, bool SPH, bool SINGLE = false, class View, class Load, class Store>
-__device__ __forceinline__ void grid_trace_coop(View view, uint32_t n, Load load, Store store, TraceCounts *cnt,
-                                                uint32_t &rays_done, unsigned long long *wkey, float4 *wray = nullptr,
-                                                uint32_t *wk = nullptr) {
-  const unsigned kFull = 0xFFFFFFFFu;
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t stride = gridDim.x * blockDim.x;
-  TravState st{};
-  TravEntry stack[kMaxStack];
-  const bool smray = wray != nullptr;
-  const SceneView *svp = nullptr;
-  auto SV = [&]() -> const SceneView & {
-    if constexpr (SINGLE) return view(0u);
-    else return *svp;
-  };
-  for (uint32_t r0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); r0 < n; r0 += stride) {
-    const uint32_t i = r0 + lane;
-    bool active = false;
-    if (smray) __syncwarp(kFull);  // the previous round's readers are done with wray
-    if (i < n) {
-      if constexpr (!SINGLE) svp = &view(i);
-      Ray r;
-      load(i, r);
-      ++rays_done;
-      active = trav_init<SPH>(SV(), r, nullptr, 0, st, ANY);
-      if (!active) store(i, st.best_prim >= 0, st);
-      if (active && smray) {
-        wray[lane] = make_float4(st.pre.o.x, st.pre.o.y, st.pre.o.z, st.ray_tmin);
-        wray[32 + lane] = make_float4(st.pre.sx, st.pre.sy, st.pre.sz, st.best);
-        wk[lane] = (uint32_t)st.pre.kx | ((uint32_t)st.pre.ky << 2) | ((uint32_t)st.pre.kz << 4);
-      }
-    }
-    while (__any_sync(kFull, active)) {
-      uint32_t lw0 = kLeafTag, lw1 = 0;
-      float cell_tmax = 0.0f;
-      if (active) trav_descend<COUNT>(SV(), st, stack, nullptr, 0, cnt, lw0, lw1, cell_tmax);
-      const uint32_t count = active ? (lw0 >> 2) : 0u;
-      // inclusive prefix sum of the leaf sizes over the warp
-      uint32_t incl = count;
-      for (uint32_t d = 1; d < 32; d <<= 1) {
-        const uint32_t v = __shfl_up_sync(kFull, incl, d);
-        if (lane >= d) incl += v;
-      }
-      const uint32_t total = __shfl_sync(kFull, incl, 31);
-      const uint32_t excl = incl - count;
-      // the owner's ray, as the tests need it
-      const uint32_t kpack = smray ? 0u : ((uint32_t)st.pre.kx | ((uint32_t)st.pre.ky << 2) | ((uint32_t)st.pre.kz << 4));
-      const unsigned long long ltp = (!SINGLE && active) ? (unsigned long long)SV().ltris : 0ull;
-      if (!ANY) wkey[lane] = ~0ull;
-      if (!ANY && smray && active) wray[32 + lane].w = st.best;
-      __syncwarp(kFull);
-      uint32_t hit_owners = 0u;
-      for (uint32_t base = 0; base < total; base += 32) {
-        const uint32_t k = base + lane;
-        // owner = the first lane whose inclusive sum exceeds k
-        uint32_t o = 0;
-        for (uint32_t step = 16; step >= 1; step >>= 1) {
-          const uint32_t v = __shfl_sync(kFull, incl, o + step - 1);
-          if (v <= k) o += step;
-        }
-        RayPre p;
-        uint32_t kp;
-        float tmin_o, best_o;
-        if (smray) {
-          const float4 ra = wray[o], rb = wray[32 + o];
-          p.o.x = ra.x; p.o.y = ra.y; p.o.z = ra.z; tmin_o = ra.w;
-          p.sx = rb.x; p.sy = rb.y; p.sz = rb.z; best_o = rb.w;
-          kp = wk[o];
-        } else {
-          p.o.x = __shfl_sync(kFull, st.pre.o.x, o);
-          p.o.y = __shfl_sync(kFull, st.pre.o.y, o);
-          p.o.z = __shfl_sync(kFull, st.pre.o.z, o);
-          p.sx = __shfl_sync(kFull, st.pre.sx, o);
-          p.sy = __shfl_sync(kFull, st.pre.sy, o);
-          p.sz = __shfl_sync(kFull, st.pre.sz, o);
-          kp = __shfl_sync(kFull, kpack, o);
-          tmin_o = __shfl_sync(kFull, st.ray_tmin, o);
-          best_o = __shfl_sync(kFull, st.best, o);
-        }
-        p.kx = (int)(kp & 3u); p.ky = (int)((kp >> 2) & 3u); p.kz = (int)((kp >> 4) & 3u);
-        const uint32_t first_o = __shfl_sync(kFull, lw1, o);
-        const uint32_t excl_o = __shfl_sync(kFull, excl, o);
-        const F4 *lt = SINGLE ? view(0u).ltris : reinterpret_cast<const F4 *>(__shfl_sync(kFull, ltp, o));
-        if (k < total) {
-          if (COUNT) cnt->tris++;
-          const uint32_t idx = k - excl_o;
-          const int64_t r = 3 * ((int64_t)first_o + idx);
-          F4 a = load_f4(lt, r + 0);
-          F4 b = load_f4(lt, r + 1);
-          F4 c = load_f4(lt, r + 2);
-          const bool culled = (f_bits(b.w) & 1u) != 0u;
-          float t, b1, b2;
-          if (intersect_tri(p, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), culled, tmin_o, best_o, t,
-                            b1, b2)) {
-            if (ANY) hit_owners |= 1u << o;
-            else atomicMin(&wkey[o], ((unsigned long long)f_bits(t) << 32) | idx);
-          }
-        }
-      }
-      bool found = false;
-      if (ANY) {
-        found = ((__reduce_or_sync(kFull, hit_owners) >> lane) & 1u) != 0u;
-      } else {
-        __syncwarp(kFull);
-        const unsigned long long key = wkey[lane];
-        __syncwarp(kFull);
-        if (active && key != ~0ull) {
-          // the winner: redo its test for t and the barycentrics (the same inputs, the same result)
-          const uint32_t idx = (uint32_t)(key & 0xFFFFFFFFull);
-          const int64_t r = 3 * ((int64_t)lw1 + idx);
-          F4 a = load_f4(SV().ltris, r + 0);
-          F4 b = load_f4(SV().ltris, r + 1);
-          F4 c = load_f4(SV().ltris, r + 2);
-          float t, b1, b2;
-          RayPre q = st.pre;
-          if (smray) {  // the constants as the testers read them, not held in registers
-            const float4 ra = wray[lane], rb = wray[32 + lane];
-            const uint32_t kq = wk[lane];
-            q.o = v3(ra.x, ra.y, ra.z);
-            q.sx = rb.x; q.sy = rb.y; q.sz = rb.z;
-            q.kx = (int)(kq & 3u); q.ky = (int)((kq >> 2) & 3u); q.kz = (int)((kq >> 4) & 3u);
-          }
-          if (intersect_tri(q, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z),
-                            (f_bits(b.w) & 1u) != 0u, st.ray_tmin, st.best, t, b1, b2)) {
-            st.best = t; st.best_prim = (int32_t)f_bits(a.w); st.bb1 = b1; st.bb2 = b2;
-          }
-        }
-      }
-      if (active) {
-        bool done;
-        if (ANY && found) {
-          st.best_prim = 0;  // occluded: any non-negative value
-          done = true;
-        } else {
-          done = trav_after_leaf<ANY>(st, stack, cell_tmax);
-        }
-        if (done) {
-          store(i, st.best_prim >= 0, st);
-          active = false;
-        }
-      }
-    }
   }
 }
 #endif

@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "hd_wide.h"
 
 namespace mgpu {
 
@@ -36,21 +37,14 @@ constexpr int kBlock = 128;
 constexpr int kHardCap = 1024;          // vertex cap when max_depth = 0 (Milton has none)
 constexpr int kCtrRay = 0;              // counters[kCtrRay + b]  live paths at bounce b
 constexpr int kCtrNee = kHardCap + 8;   // counters[kCtrNee + b]  shadow rays at bounce b
-constexpr int kCtrFetchExt = 2 * (kHardCap + 8);   // work counters of the persistent extend kernel
-constexpr int kCtrFetchSh = 3 * (kHardCap + 8);    // ... and of the persistent shadow kernel
-constexpr int kCtrTrunc = 4 * (kHardCap + 8);
+constexpr int kCtrTrunc = 2 * (kHardCap + 8);
 constexpr int kNumCounters = kCtrTrunc + 8;
 constexpr int kBinBits = 14;           // queue binning keys: 2^14 bins
 constexpr int kBins = 1 << kBinBits;
 constexpr int kBinSmem = kBins * 4;    // dynamic shared memory of a sorting block
 constexpr double kAutoWaveBytes = 40e9;  // workspace budget of an automatic wave
-#ifndef MGPU_TRAV_MIN_BLOCKS
-#define MGPU_TRAV_MIN_BLOCKS 12
-#endif
-// Resident 128-thread blocks per SM the traversal kernels are compiled for: 12 caps them at 40
-// registers (a few bytes of spills to L1) for 48 warps per SM instead of 36-40, which hides more
-// of the node-load latency (mid frame: 215 -> 226 Mpaths/s; 10 and 16 blocks measured 221).
-constexpr int kTravMinBlocks = MGPU_TRAV_MIN_BLOCKS;
+// Resident 128-thread blocks per SM that the kd-tree kernels are compiled for: 40 registers
+constexpr int kTravMinBlocks = 12;
 #ifndef MGPU_SHADE_MIN_BLOCKS
 #define MGPU_SHADE_MIN_BLOCKS 8
 #endif
@@ -301,38 +295,30 @@ __global__ void __launch_bounds__(kBlock) k_generate(RenderArgs a) {
 }
 
 // extend: closest hit for the live queue of bounce b
-// traversal kernel shapes (mgpu_tune_set "persistent" / "coop_leaf")
-constexpr int kShapeGrid = 0;     // grid-stride, one ray per lane to completion
-constexpr int kShapePersist = 1;  // persistent warps with per-lane refill
-constexpr int kShapeCoop = 2;     // grid-stride, leaf triangles shared by the warp
-#ifndef MGPU_COOP_MIN_BLOCKS
-#define MGPU_COOP_MIN_BLOCKS 12
-#endif
-#ifndef MGPU_COOP_EXT_MIN_BLOCKS
-#define MGPU_COOP_EXT_MIN_BLOCKS 10
-#endif
-// resident 128-thread blocks per SM (their register budget) of the warp-cooperative traversal
-// shape: any hit 12 (40 registers), closest hit 10 (48 registers: its shared-memory reduction and
-// winner re-test hold more state; mid frame 90.7 ms at 10 against 95.7 at 12 and 97.7 at 14, the
-// any-hit kernel 116.0 at 10 against 113.2 at 12)
-constexpr int kCoopMinBlocks = MGPU_COOP_MIN_BLOCKS;
-constexpr int kCoopExtMinBlocks = MGPU_COOP_EXT_MIN_BLOCKS;
+// Traversal: the 8-wide hierarchy (hd_wide.h), or the kd-tree, one ray per lane, for a scene that has
+// none and with mgpu_tune_set("wide", 0).
+constexpr int kWideSmem = kWideBlock / 32 * (int)sizeof(WideShared);
 
-// BLK: threads per block of a traversal kernel (mgpu_tune_set "trav_block"); the resident
-// blocks per SM scale with it, so every block size gets the same register budget per thread
-template <bool COUNT, int SHAPE, bool SPH = false, int BLK = kBlock>
-__global__ void __launch_bounds__(BLK, (SHAPE == kShapeCoop ? kCoopExtMinBlocks : kTravMinBlocks) * kBlock / BLK)
-    k_extend(RenderArgs a, int b) {
+__device__ __forceinline__ WideShared &wide_shared(uint32_t *&next) {
+  extern __shared__ __align__(16) unsigned char wide_smem[];
+  __shared__ uint32_t counter;
+  if (threadIdx.x == 0) counter = 0u;
+  __syncthreads();
+  next = &counter;
+  return reinterpret_cast<WideShared *>(wide_smem)[threadIdx.x >> 5];
+}
+
+template <bool COUNT, bool WIDE, bool SPH>
+__global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMinBlocks)
+    k_extend(const __grid_constant__ RenderArgs a, int b) {
   const uint32_t n = a.counters[kCtrRay + b];
   const float4 *qo = a.qo[b & 1], *qd = a.qd[b & 1];
   float4 *qhit = a.qhit;
   TraceCounts c = {0, 0, 0, 0};
   uint32_t rays = 0;
   const bool single = a.njobs == 1;
-  const SceneView *view0 = &a.jobs[0].view;
-  auto view_of = [&](uint32_t i) -> const SceneView & {
-    return single ? *view0 : a.jobs[__float_as_int(qd[i].w)].view;
-  };
+  auto view_of = [&](uint32_t i) -> const SceneView & { return a.jobs[__float_as_int(qd[i].w)].view; };
+  auto view0 = [&](uint32_t) -> const SceneView & { return a.view0; };
   auto load = [&](uint32_t i, Ray &r) {
     float4 o = qo[i], d = qd[i];
     r.o = v3(o.x, o.y, o.z);
@@ -340,28 +326,22 @@ __global__ void __launch_bounds__(BLK, (SHAPE == kShapeCoop ? kCoopExtMinBlocks 
     r.d = v3(d.x, d.y, d.z);
     r.tmax = INFINITY;
   };
-  auto store = [&](uint32_t i, bool hit, const TravState &st) {
-    qhit[i] = make_float4(hit ? st.best : INFINITY, __int_as_float(hit ? st.best_prim : -1), hit ? st.bb1 : 0.0f,
-                          hit ? st.bb2 : 0.0f);
-  };
-  if (SHAPE == kShapePersist) {
-    persistent_trace<false, COUNT, SPH>(view_of, nullptr, 0, n, &a.counters[kCtrFetchExt + b], load, store, &c, rays);
-  } else if (SHAPE == kShapeCoop) {
-    // per warp: the closest-hit keys of the shared leaf tests and the lanes' ray constants
-    __shared__ unsigned long long wkey[BLK];
-    __shared__ float4 wray[2 * BLK];
-    __shared__ uint32_t wk[BLK];
-    if (single)
-      grid_trace_coop<false, COUNT, SPH, true>([&](uint32_t) -> const SceneView & { return a.view0; }, n, load, store,
-                                               &c, rays, wkey + (threadIdx.x & ~31u), wray + 2 * (threadIdx.x & ~31u),
-                                               wk + (threadIdx.x & ~31u));
-    else
-      grid_trace_coop<false, COUNT, SPH>(view_of, n, load, store, &c, rays, wkey + (threadIdx.x & ~31u),
-                                         wray + 2 * (threadIdx.x & ~31u), wk + (threadIdx.x & ~31u));
+  if constexpr (WIDE) {
+    auto store = [&](uint32_t i, bool hit, const Hit &h) {
+      qhit[i] = make_float4(hit ? h.t : INFINITY, __int_as_float(hit ? h.prim : -1), hit ? h.b1 : 0.0f, hit ? h.b2 : 0.0f);
+    };
+    uint32_t *next;
+    WideShared &sh = wide_shared(next);
+    if (single) wide_trace<false, SPH, COUNT, SPH, true>(view0, n, load, store, sh, next, &c, rays);
+    else wide_trace<false, SPH, COUNT, SPH, false>(view_of, n, load, store, sh, next, &c, rays);
   } else {
+    auto store = [&](uint32_t i, bool hit, const TravState &st) {
+      qhit[i] = make_float4(hit ? st.best : INFINITY, __int_as_float(hit ? st.best_prim : -1), hit ? st.bb1 : 0.0f,
+                            hit ? st.bb2 : 0.0f);
+    };
     grid_trace<false, COUNT, SPH>(view_of, nullptr, 0, n, load, store, &c, rays);
   }
-  if (COUNT && rays) {
+  if (COUNT && rays + c.nodes + c.tris) {
     atomicAdd(&a.tcount[0], (unsigned long long)c.nodes);
     atomicAdd(&a.tcount[1], (unsigned long long)c.refs);
     atomicAdd(&a.tcount[2], (unsigned long long)c.tris);
@@ -577,21 +557,20 @@ __global__ void __launch_bounds__(kBlock, kShadeMinBlocks) k_shade(RenderArgs a,
 }
 
 // shadow: any-hit query per queued light sample; an occluded sample's slot is zeroed
-template <bool COUNT, int SHAPE, bool SPH = false, int BLK = kBlock>
-__global__ void __launch_bounds__(BLK, (SHAPE == kShapeCoop ? kCoopMinBlocks : kTravMinBlocks) * kBlock / BLK)
-    k_shadow(RenderArgs a, int b) {
+template <bool COUNT, bool WIDE, bool SPH>
+__global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMinBlocks)
+    k_shadow(const __grid_constant__ RenderArgs a, int b) {
   const uint32_t n = a.counters[kCtrNee + b];
   const float4 *so = a.so, *sd = a.sd;
   float4 *slots = a.slots;
   TraceCounts c = {0, 0, 0, 0};
   uint32_t rays = 0;
   const bool single = a.njobs == 1;
-  const SceneView *view0 = &a.jobs[0].view;
   auto view_of = [&](uint32_t i) -> const SceneView & {
-    if (single) return *view0;
     const uint32_t slot = __float_as_uint(so[i].w);
     return a.jobs[a.path_job[slot / (uint32_t)a.nl_stride]].view;
   };
+  auto view0 = [&](uint32_t) -> const SceneView & { return a.view0; };
   auto load = [&](uint32_t i, Ray &r) {
     float4 o = so[i], d = sd[i];
     r.o = v3(o.x, o.y, o.z);
@@ -599,26 +578,18 @@ __global__ void __launch_bounds__(BLK, (SHAPE == kShapeCoop ? kCoopMinBlocks : k
     r.d = v3(d.x, d.y, d.z);
     r.tmax = d.w;
   };
-  auto store = [&](uint32_t i, bool hit, const TravState &) {
+  auto store = [&](uint32_t i, bool hit, const auto &) {
     if (hit) slots[__float_as_uint(so[i].w)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   };
-  if (SHAPE == kShapePersist) {
-    persistent_trace<true, COUNT, SPH>(view_of, nullptr, 0, n, &a.counters[kCtrFetchSh + b], load, store, &c, rays);
-  } else if (SHAPE == kShapeCoop) {
-    // per warp: the lanes' ray constants for the shared leaf tests
-    __shared__ float4 wray[2 * BLK];
-    __shared__ uint32_t wk[BLK];
-    if (single)
-      grid_trace_coop<true, COUNT, SPH, true>([&](uint32_t) -> const SceneView & { return a.view0; }, n, load, store,
-                                              &c, rays, nullptr, wray + 2 * (threadIdx.x & ~31u),
-                                              wk + (threadIdx.x & ~31u));
-    else
-      grid_trace_coop<true, COUNT, SPH>(view_of, n, load, store, &c, rays, nullptr, wray + 2 * (threadIdx.x & ~31u),
-                                        wk + (threadIdx.x & ~31u));
+  if constexpr (WIDE) {
+    uint32_t *next;
+    WideShared &sh = wide_shared(next);
+    if (single) wide_trace<true, SPH, COUNT, SPH, true>(view0, n, load, store, sh, next, &c, rays);
+    else wide_trace<true, SPH, COUNT, SPH, false>(view_of, n, load, store, sh, next, &c, rays);
   } else {
     grid_trace<true, COUNT, SPH>(view_of, nullptr, 0, n, load, store, &c, rays);
   }
-  if (COUNT && rays) {
+  if (COUNT && rays + c.nodes + c.tris) {
     atomicAdd(&a.tcount[4], (unsigned long long)c.nodes);
     atomicAdd(&a.tcount[5], (unsigned long long)c.refs);
     atomicAdd(&a.tcount[6], (unsigned long long)c.tris);
@@ -808,13 +779,10 @@ constexpr int kCarveoutAuto = -2;
 
 // process-wide tuning knobs (mgpu_tune_set)
 struct Tuning {
-  std::atomic<int> persistent{0};     // persistent warp-level traversal with ray refill
-  // grid-stride traversal with the leaf triangles shared by the warp: bit 0 for the shadow
-  // (any-hit) kernel, bit 1 for the extension (closest-hit) kernel
-  std::atomic<int> coop_leaf{3};
-  // threads per block of the grid-stride and warp-shared traversal kernels: 64, 128 or 256 (mid
-  // frame: 256 is 0.6 % faster than 128, 64 equal to 128)
-  std::atomic<int> trav_block{256};
+  // the 8-wide hierarchy where every scene of a render has one; 0: the kd-tree
+  std::atomic<int> wide{1};
+  // shapes of kd-tree kernels that are no more: kept for callers that set and read them back
+  std::atomic<int> persistent{0}, coop_leaf{3}, trav_block{256};
   std::atomic<int> bin_shadow{1};     // counting-sort shadow rays by (light, origin cell)
   std::atomic<int> bin_extension{1};  // counting-sort extension rays by (octant, origin cell)
   // waves of fewer paths skip binning: sorting a few hundred thousand rays costs more (four
@@ -986,35 +954,32 @@ static int64_t noalloc_paths(int64_t nl_slots) {
 // Function attributes belong to a device's context: they are set on the current device before
 // its first render and again after the carveout knob changes.
 //   the sorting blocks: kBins counters of dynamic shared memory, above the 48 KB default;
+//   the wide traversal kernels: their warps' records, above the 48 KB default too;
 //   the traversal and shade kernels: the L1 / shared-memory split ("carveout").  These kernels
-//   chase pointers through L1 and their block needs little shared memory (none, or the shared
-//   leaf tests' per-warp records); the driver's own choice for the shared-leaf shadow kernel is a
-//   132 KB shared-memory configuration where 64 KB keeps all its blocks resident, and the L1 it
-//   gives up makes that kernel 4 % slower on the mid frame.  The automatic carveout asks for the
-//   least shared memory that keeps the kernel's register-limited number of resident blocks.
+//   chase pointers through L1 and need little shared memory, so the automatic carveout asks for
+//   the least shared memory that keeps the kernel's register-limited number of resident blocks and
+//   leaves the rest of the SM's 256 KB to L1.
 struct CarveoutKernel {
   const void *f;
   int block;
+  int dyn;  // dynamic shared memory of a block
 };
 
 static std::vector<CarveoutKernel> carveout_kernels() {
-  return {{(const void *)k_extend<false, kShapeGrid>, kBlock},      {(const void *)k_extend<false, kShapePersist>, kBlock},
-          {(const void *)k_extend<false, kShapeCoop>, kBlock},      {(const void *)k_extend<true, kShapeGrid>, kBlock},
-          {(const void *)k_extend<true, kShapePersist>, kBlock},    {(const void *)k_extend<true, kShapeCoop>, kBlock},
-          {(const void *)k_extend<false, kShapeGrid, true>, kBlock}, {(const void *)k_extend<true, kShapeGrid, true>, kBlock},
-          {(const void *)k_shadow<false, kShapeGrid>, kBlock},      {(const void *)k_shadow<false, kShapePersist>, kBlock},
-          {(const void *)k_shadow<false, kShapeCoop>, kBlock},      {(const void *)k_shadow<true, kShapeGrid>, kBlock},
-          {(const void *)k_shadow<true, kShapePersist>, kBlock},    {(const void *)k_shadow<true, kShapeCoop>, kBlock},
-          {(const void *)k_shadow<false, kShapeGrid, true>, kBlock}, {(const void *)k_shadow<true, kShapeGrid, true>, kBlock},
-          {(const void *)k_extend<false, kShapeGrid, false, 64>, 64},
-          {(const void *)k_extend<false, kShapeGrid, false, 256>, 256},
-          {(const void *)k_extend<false, kShapeCoop, false, 64>, 64},
-          {(const void *)k_extend<false, kShapeCoop, false, 256>, 256},
-          {(const void *)k_shadow<false, kShapeGrid, false, 64>, 64},
-          {(const void *)k_shadow<false, kShapeGrid, false, 256>, 256},
-          {(const void *)k_shadow<false, kShapeCoop, false, 64>, 64},
-          {(const void *)k_shadow<false, kShapeCoop, false, 256>, 256},
-          {(const void *)k_shade<false>, kBlock},                    {(const void *)k_shade<true>, kBlock}};
+  return {{(const void *)k_extend<false, true, false>, kWideBlock, kWideSmem},
+          {(const void *)k_extend<false, true, true>, kWideBlock, kWideSmem},
+          {(const void *)k_extend<true, true, false>, kWideBlock, kWideSmem},
+          {(const void *)k_extend<true, true, true>, kWideBlock, kWideSmem},
+          {(const void *)k_shadow<false, true, false>, kWideBlock, kWideSmem},
+          {(const void *)k_shadow<false, true, true>, kWideBlock, kWideSmem},
+          {(const void *)k_shadow<true, true, false>, kWideBlock, kWideSmem},
+          {(const void *)k_shadow<true, true, true>, kWideBlock, kWideSmem},
+          {(const void *)k_extend<false, false, true>, kBlock, 0},
+          {(const void *)k_extend<true, false, true>, kBlock, 0},
+          {(const void *)k_shadow<false, false, true>, kBlock, 0},
+          {(const void *)k_shadow<true, false, true>, kBlock, 0},
+          {(const void *)k_shade<false>, kBlock, 0},
+          {(const void *)k_shade<true>, kBlock, 0}};
 }
 
 // percent of the SM's shared memory that holds the kernel's resident blocks (registers and
@@ -1026,9 +991,9 @@ static cudaError_t auto_carveout(const CarveoutKernel &k, int smem_sm, int reser
   e = cudaFuncSetAttribute(k.f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e != cudaSuccess) return e;
   int blocks = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k.f, k.block, 0);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k.f, k.block, (size_t)k.dyn);
   if (e != cudaSuccess) return e;
-  const int64_t need = (int64_t)blocks * (int64_t)(fa.sharedSizeBytes + (size_t)reserved);
+  const int64_t need = (int64_t)blocks * (int64_t)(fa.sharedSizeBytes + (size_t)k.dyn + (size_t)reserved);
   pct = (int)std::min<int64_t>(100, (need * 100 + smem_sm - 1) / smem_sm);
   return cudaSuccess;
 }
@@ -1047,6 +1012,9 @@ static cudaError_t kernel_attributes() {
     const void *bins[] = {(const void *)k_bin_hist, (const void *)k_bin_scatter<2>, (const void *)k_bin_scatter<3>};
     for (const void *kf : bins)
       if ((e = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, kBinSmem)) != cudaSuccess) return e;
+    for (const CarveoutKernel &k : carveout_kernels())
+      if (k.dyn && (e = cudaFuncSetAttribute(k.f, cudaFuncAttributeMaxDynamicSharedMemorySize, k.dyn)) != cudaSuccess)
+        return e;
   }
   int smem_sm = 0, reserved = 0;
   if ((e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev)) != cudaSuccess) return e;
@@ -1314,31 +1282,21 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
     MGPU_CUDA(cudaMemcpyAsync(w->jobs, all.data(), all.size() * sizeof(JobArgs), cudaMemcpyHostToDevice, st));
   }
 
-  const bool persist = g_tune.persistent.load() != 0;
-  const bool coop_sh = (g_tune.coop_leaf.load() & 1) != 0, coop_ext = (g_tune.coop_leaf.load() & 2) != 0;
   bool sph = false;  // a job's scene has analytic spheres: the traversal kernels that test them
-  for (const Job &j : jobs) sph = sph || j.scene->view.nsphere > 0;
-  // threads per traversal block: 128 for the persistent, sphere and counted kernels; the
-  // grid-stride and warp-shared shapes of the plain render also come in 64 and 256
-  const int tb = (sph || persist || COUNT) ? kBlock : g_tune.trav_block.load();
-  auto kext = sph        ? k_extend<COUNT, kShapeGrid, true>
-              : persist  ? k_extend<COUNT, kShapePersist>
-              : coop_ext ? (tb == 64 ? k_extend<COUNT, kShapeCoop, false, 64>
-                            : tb == 256 ? k_extend<COUNT, kShapeCoop, false, 256> : k_extend<COUNT, kShapeCoop>)
-                         : (tb == 64 ? k_extend<COUNT, kShapeGrid, false, 64>
-                            : tb == 256 ? k_extend<COUNT, kShapeGrid, false, 256> : k_extend<COUNT, kShapeGrid>);
-  auto kshw = sph        ? k_shadow<COUNT, kShapeGrid, true>
-              : persist  ? k_shadow<COUNT, kShapePersist>
-              : coop_sh  ? (tb == 64 ? k_shadow<COUNT, kShapeCoop, false, 64>
-                            : tb == 256 ? k_shadow<COUNT, kShapeCoop, false, 256> : k_shadow<COUNT, kShapeCoop>)
-                         : (tb == 64 ? k_shadow<COUNT, kShapeGrid, false, 64>
-                            : tb == 256 ? k_shadow<COUNT, kShapeGrid, false, 256> : k_shadow<COUNT, kShapeGrid>);
-  const int tb_ext = (sph || persist || COUNT) ? kBlock : tb, tb_sh = tb_ext;
+  bool wide = g_tune.wide.load() != 0;  // every scene has the 8-wide hierarchy
+  for (const Job &j : jobs) {
+    sph = sph || j.scene->view.nsphere > 0;
+    wide = wide && (j.scene->view.wnodes != nullptr || j.scene->view.ntri == 0);
+  }
+  auto kext = !wide ? k_extend<COUNT, false, true> : sph ? k_extend<COUNT, true, true> : k_extend<COUNT, true, false>;
+  auto kshw = !wide ? k_shadow<COUNT, false, true> : sph ? k_shadow<COUNT, true, true> : k_shadow<COUNT, true, false>;
+  const int tb = wide ? kWideBlock : kBlock;
+  const size_t tsm = wide ? (size_t)kWideSmem : 0;
   MGPU_CUDA(kernel_attributes());
   const int g_gen = grid_for((const void *)k_generate, 0);
-  const int g_ext = grid_for((const void *)kext, 0, tb_ext);
+  const int g_ext = grid_for((const void *)kext, tsm, tb);
   const int g_sha = grid_for((const void *)k_shade<true>, 0);
-  const int g_shw = grid_for((const void *)kshw, 0, tb_sh);
+  const int g_shw = grid_for((const void *)kshw, tsm, tb);
   const int g_acc = grid_for((const void *)k_accumulate, 0);
   const int g_bin = device_sm_count() * 4;
   const int bin_ext = g_tune.bin_extension.load(), bin_sh = g_tune.bin_shadow.load();
@@ -1407,7 +1365,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
       int chunk = wv.unlimited ? std::min(4, max_b - b) : max_b;
       for (int k = 0; k < chunk; ++k, ++b) {
         m = pf.begin(kProfExtend, st);
-        kext<<<g_ext, tb_ext, 0, st>>>(a, b);
+        kext<<<g_ext, tb, tsm, st>>>(a, b);
         pf.end(m, st);
         m = pf.begin(kProfShade, st);
         if (surf) k_shade<true><<<g_sha, kBlock, 0, st>>>(a, b);
@@ -1435,7 +1393,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
           pf.end(m, st);
         }
         m = pf.begin(kProfShadow, st);
-        kshw<<<g_shw, tb_sh, 0, st>>>(a, b);
+        kshw<<<g_shw, tb, tsm, st>>>(a, b);
         pf.end(m, st);
         launches += 3;
       }
@@ -1623,6 +1581,7 @@ int mgpu_tune_set(const char *key, int64_t value) {
   if (k == "persistent") g_tune.persistent.store(value != 0);
   else if (k == "coop_leaf" && value >= 0 && value <= 3) g_tune.coop_leaf.store((int)value);
   else if (k == "trav_block" && (value == 64 || value == 128 || value == 256)) g_tune.trav_block.store((int)value);
+  else if (k == "wide") g_tune.wide.store(value != 0);
   else if (k == "bin_shadow") g_tune.bin_shadow.store(value != 0);
   else if (k == "bin_extension") g_tune.bin_extension.store(value != 0);
   else if (k == "bin_min_paths" && value >= 0) g_tune.bin_min_paths.store(value);
@@ -1639,6 +1598,7 @@ int mgpu_tune_get(const char *key, int64_t *value) {
   if (k == "persistent") *value = g_tune.persistent.load();
   else if (k == "coop_leaf") *value = g_tune.coop_leaf.load();
   else if (k == "trav_block") *value = g_tune.trav_block.load();
+  else if (k == "wide") *value = g_tune.wide.load();
   else if (k == "bin_shadow") *value = g_tune.bin_shadow.load();
   else if (k == "bin_extension") *value = g_tune.bin_extension.load();
   else if (k == "bin_min_paths") *value = g_tune.bin_min_paths.load();

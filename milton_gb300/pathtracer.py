@@ -71,8 +71,7 @@ def _desc(scene: Scene) -> N.SceneDesc:
 @dataclass
 class KdSettings:
     """kdTreeAccel build parameters: Milton's defaults (kdTreeAccel.h:97-104) except the traversal
-    cost, MGPU_KD_COST_TRAVERSAL = 3 (include/mgpu.h: a node step costs the GPU's traversal
-    kernels about three triangle tests); ``KdSettings.milton()`` is Milton's set exactly."""
+    cost, MGPU_KD_COST_TRAVERSAL = 3 (include/mgpu.h); ``KdSettings.milton()`` is Milton's set exactly."""
     min_prims: int = 3
     max_depth: int = 24
     cost_traversal: float = 3.0
@@ -352,7 +351,7 @@ def profile_enable(enable: bool = True) -> None:
 
 
 def tune(key: str, value: int) -> None:
-    """Process-wide tuning knob (persistent, bin_shadow, bin_extension); results are unchanged."""
+    """Process-wide tuning knob (wide, bin_shadow, bin_extension, ...); results are unchanged."""
     N.check(N.load().mgpu_tune_set(key.encode(), int(value)))
 
 

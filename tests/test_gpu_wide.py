@@ -1,0 +1,161 @@
+"""The 8-wide hierarchy that rays traverse against the kd-tree, bit for bit: the counted ray query and
+mgpu_tune_set("wide", 0) go through the kd-tree, everything else through the hierarchy."""
+import numpy as np
+import pytest
+
+from gpu_util import gpu_any, gpu_trace
+from milton_gb300 import pathtracer as pt
+from milton_gb300 import scenegen
+from milton_gb300.scene import SceneBuilder, camera, dielectric, diffuse
+from raygen import camera_rays, sphere_rays
+
+pytestmark = pytest.mark.gpu
+
+
+def _soup(tris, culled=False):
+    b = SceneBuilder()
+    m = b.material(diffuse(0.5))
+    b.add("t", np.asarray(tris, np.float32), np.broadcast_to(np.float32([0, 1, 0]), (len(tris), 3, 3)), m, culled=culled)
+    return b.build(camera(eye=(0, 1, 3), look=(0, 0, -1), up=(0, 1, 0), height_angle=40.0, aspect=1.0))
+
+
+def _random_tris(n, seed, size=0.2, scale=1.0, offset=(0, 0, 0)):
+    rng = np.random.default_rng(seed)
+    c = rng.uniform(-1, 1, (n, 1, 3))
+    return (c + rng.normal(size=(n, 3, 3)) * size) * scale + np.asarray(offset)
+
+
+def _scene(kind):
+    if kind.startswith("n"):  # sizes around the leaf, node and builder block limits
+        return _soup(_random_tris(int(kind[1:]), 7, size=0.5 if int(kind[1:]) < 100 else 0.05))
+    if kind == "culled":
+        return _soup(_random_tris(500, 3), culled=True)
+    if kind == "coincident":  # every triangle twice, and a stack of copies of one
+        t = _random_tris(300, 5)
+        return _soup(np.concatenate([t, t[::-1], np.repeat(t[:1], 40, 0)]))
+    if kind == "flat":        # one plane, a grid of axis-aligned quads
+        g = np.arange(40) / 20.0 - 1.0
+        q = [scenegen.quad_tris((x, 0, z + .05), (x + .05, 0, z + .05), (x + .05, 0, z), (x, 0, z)) for x in g for z in g]
+        return _soup(np.concatenate(q))
+    if kind == "points":      # degenerate triangles among proper ones
+        t = _random_tris(200, 6)
+        t[::3] = t[::3, :1]
+        t[1::6, 2] = t[1::6, 1]
+        return _soup(t)
+    if kind == "line":        # clusters each nearest to the one before (linearly growing gaps)
+        x = np.cumsum(np.arange(5000) * 1e-6)[:, None, None]
+        return _soup(np.concatenate([x + np.zeros((1, 3, 1)), np.zeros((5000, 3, 2))], -1) +
+                     np.float32([[0, 0, 0], [0, 1e-2, 0], [0, 0, 1e-2]]))
+    if kind == "far":         # small geometry far from the origin
+        return _soup(_random_tris(2000, 8, size=0.05, scale=1.0, offset=(3000, -2000, 5000)))
+    if kind == "scales":      # one huge quad and tiny detail
+        return _soup(np.concatenate([scenegen.quad_tris((-1e4, -1, 1e4), (1e4, -1, 1e4), (1e4, -1, -1e4), (-1e4, -1, -1e4)),
+                                     _random_tris(3000, 9, size=1e-3)]))
+    if kind == "balls":       # analytic spheres beside triangles
+        s = scenegen.plain(2)
+        s.spheres = np.float32([[0.3, 0.9, 0.5, 0.2, 0, 0, 0, 1], [-0.5, 1.5, 0.0, 0.3, 0, 0, 0, 1]])
+        s.sphere_mat = np.int32([0, 0])
+        s.sphere_light = np.int32([-1, -1])
+        return s
+    return scenegen.plain(1) if kind == "plain" else scenegen.random_scene(9, 60_000)
+
+
+def _rays(s, n, seed):
+    v = s.tri_v.reshape(-1, 3)
+    lo, hi = v.min(0) - 0.3, v.max(0) + 0.3
+    if np.ptp(v, axis=0).max() > 1e3:  # the detail, not the huge quad
+        lo, hi = np.full(3, -1.2), np.full(3, 1.2)
+    r = np.concatenate([camera_rays(s.camera, n, seed), sphere_rays(lo, hi, n, seed + 1)])
+    rng = np.random.default_rng(seed + 2)
+    ax = sphere_rays(lo, hi, n, seed + 3)  # axis-parallel, -0 among the zeros, origins on vertex planes
+    k = rng.integers(0, 3, n)
+    ax[:, 4:7] = np.where(rng.random((n, 3)) < 0.5, -0.0, 0.0)
+    ax[np.arange(n), 4 + k] = np.where(rng.random(n) < 0.5, -1.0, 1.0)
+    p = v[rng.integers(0, len(v), n)]
+    on = rng.random((n, 3)) < 0.3
+    ax[:, 0:3] = np.where(on, p, ax[:, 0:3])
+    aimed = sphere_rays(lo, hi, n, seed + 4)  # at points of triangles: edges, vertices, interiors
+    t = s.tri_v[rng.integers(0, s.ntri, n)].astype(np.float64)
+    w = rng.dirichlet((1, 1, 1), n) * np.where(rng.random((n, 1)) < 0.5, 1.0, rng.integers(0, 2, (n, 3)))
+    w /= np.maximum(w.sum(1, keepdims=True), 1e-9)
+    d = (t * w[..., None]).sum(1) - aimed[:, 0:3]
+    aimed[:, 4:7] = d / np.maximum(np.linalg.norm(d, axis=1, keepdims=True), 1e-9)
+    short = sphere_rays(lo, hi, n, seed + 5)
+    short[:, 3] = rng.uniform(0, 0.5, n)
+    short[:, 7] = short[:, 3] + rng.uniform(0, 1.5, n)
+    short[::2, 4:7] *= 3.7  # directions need not be unit
+    return np.concatenate([r, ax, aimed, short]).astype(np.float32)
+
+
+KINDS = ["n1", "n2", "n3", "n4", "n7", "n25", "n2047", "n2048", "n2049", "n4097", "culled", "coincident", "flat", "points",
+         "line", "far", "scales", "balls", "plain", "random"]
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_ray_queries_equal_the_kd_trees(cuda, kind):
+    s = _scene(kind)
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    for n in (20_000, 33):
+        rays = _rays(s, n, 11)
+        kd, _ = gpu_trace(cuda, ds, rays, counts=True)
+        wide, _ = gpu_trace(cuda, ds, rays)
+        same = np.all(kd.view(np.uint32) == wide.view(np.uint32), axis=1)
+        assert same.all(), (kind, n, int((~same).sum()), rays[~same][:2], kd[~same][:2], wide[~same][:2])
+        assert np.array_equal(gpu_any(cuda, ds, rays) != 0, kd[:, 1].view(np.int32) >= 0)
+
+
+@pytest.mark.parametrize("kind", ["plain", "random", "textured", "balls", "deep", "batch"])
+def test_films_equal_the_kd_trees(cuda, kind):
+    if kind == "textured":
+        s = scenegen.textured(3)
+    elif kind in ("balls", "deep"):
+        s = _scene("balls" if kind == "balls" else "random")
+        s.materials[s.tri_mat[0]] = dielectric(1.5)
+    else:
+        s = _scene("random" if kind == "batch" else kind)
+    scenes = [pt.DeviceScene(s, pt.Accel(s))]
+    if kind == "batch":
+        p = scenegen.plain(5)
+        scenes += [pt.DeviceScene(p, pt.Accel(p)), scenes[0]]
+    depth = 0 if kind == "deep" else 6
+    sizes = [(61, 43), (40, 24), (16, 9)]
+    out = []
+    assert pt.tune_get("wide") == 1
+    try:
+        for wide in (0, 1):
+            pt.tune("wide", wide)
+            films = [pt.Film(*wh) for wh in sizes[:len(scenes)]]
+            b = pt.Batch()
+            for k, (ds, f, wh) in enumerate(zip(scenes, films, sizes)):
+                b.add(ds, pt.RenderSettings(*wh, 9, max_depth=depth, rr_start_depth=3, seed=31 + k), f)
+            b.render()
+            out.append([f.raw() for f in films])
+    finally:
+        pt.tune("wide", 1)
+    for a, c in zip(*out):
+        assert np.array_equal(a.view(np.uint32), c.view(np.uint32))
+
+
+def test_negative_tmin_and_lines(cuda):
+    # the hierarchy's box tests move the planes by an absolute amount, so t < 0 needs no special case:
+    # lines (tmin = -inf) and rays that start behind the origin against a brute force in 64 bits
+    s = scenegen.plain(1)
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    r = sphere_rays((-1, 0, -1), (1, 2, 1), 3000, 5)
+    r[::2, 3] = -np.inf
+    r[1::2, 3] = -0.75
+    h, _ = gpu_trace(cuda, ds, r)
+    o, d = r[:, None, 0:3].astype(np.float64), r[:, None, 4:7].astype(np.float64)
+    v = s.tri_v.astype(np.float64)
+    e1, e2 = v[:, 1] - v[:, 0], v[:, 2] - v[:, 0]
+    with np.errstate(divide="ignore", invalid="ignore"):
+        p = np.cross(d, e2)
+        det = (e1 * p).sum(-1)
+        q = np.cross(o - v[:, 0], e1)
+        b1, b2 = ((o - v[:, 0]) * p).sum(-1) / det, (d * q).sum(-1) / det
+        t = (e2 * q).sum(-1) / det
+        t = np.where((b1 >= 0) & (b2 >= 0) & (b1 + b2 <= 1) & (t > r[:, 3:4]), t, np.inf)
+    best = t.min(1)
+    # FP32 against FP64: a ray within rounding of an edge (about 1e-6 of the box) may decide otherwise
+    ok = np.isclose(h[:, 0], best, rtol=1e-4, atol=1e-5) | (np.isinf(h[:, 0]) & np.isinf(best))
+    assert ok.mean() >= 0.999, ok.mean()
