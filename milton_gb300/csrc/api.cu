@@ -493,13 +493,19 @@ int mgpu_scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void
   s->nlight = desc->nlight;
   bool wide = false;
   uint32_t wide_nodes = 0;
-  if (int rc = wide_build(s->view.tris, T, base + L.off_wnodes, (F4 *)(base + L.off_wtris), base + L.off_wscratch, st,
+  s->view.wextent = 0.0f;
+  for (int k = 0; k < 3; ++k) {
+    const float c = 0.5f * s->view.bmin[k] + 0.5f * s->view.bmax[k];
+    s->view.wcentre[k] = std::isfinite(c) ? c : 0.0f;
+    s->view.wextent = std::max(s->view.wextent, std::max(s->view.bmax[k] - s->view.wcentre[k], s->view.wcentre[k] - s->view.bmin[k]));
+  }
+  if (int rc = wide_build(s->view.tris, T, s->view.wcentre, base + L.off_wnodes, (F4 *)(base + L.off_wtris), base + L.off_wscratch, st,
                           &wide_nodes, &wide)) {
     cudaFree(s->d_block);
     delete s;
     return rc;
   }
-  s->view.wnodes = wide ? (const uint4 *)(base + L.off_wnodes) : nullptr;
+  s->view.wnodes = wide ? (const uint32_t *)(base + L.off_wnodes) : nullptr;
   s->view.wtris = wide ? (const F4 *)(base + L.off_wtris) : nullptr;
   // staging the top of the tree in shared memory costs more occupancy than it saves on GB300
   // (the L1 keeps those pairs anyway); mgpu_scene_set_top_pairs turns it on

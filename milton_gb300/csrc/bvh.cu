@@ -89,9 +89,10 @@ struct Build {
   uint2 *bsum;            // per block: survivors, merges
   uint32_t *ctr;          // counters (kC*)
   int32_t *wroot;         // binary root of every wide node
-  uint4 *wnodes;
+  uint32_t *wnodes;
   F4 *wtris;
   uint32_t cap_nodes;
+  float centre[3];        // node coordinates are relative to it
 };
 
 // counters
@@ -715,25 +716,24 @@ __device__ void emit_node(const Build &B, uint32_t w, bool valid, int32_t *xn, i
     if ((at >> 4) == lane) slot = (int)(at & 7u);
     free_slots &= ~(1u << (at & 7u));
   }
-  // the grid: a step of a power of two, its origin a thirty-second step below the box, so that every
-  // child keeps at least a sixty-fourth step of slack after rounding outward
-  float org[3], inv[3];
-  uint32_t expo[3];
+  // the grid: a step of a power of two, its origin (stored less 2^15 steps, so that the traversal can
+  // take a plane's byte as the float 1 + byte / 2^15) at least a thirty-second step below the
+  // box, so that every child keeps at least a sixty-fourth step of slack after rounding outward
+  float org[3], inv[3], step[3];
   bool fits = true;
   for (int k = 0; k < 3; ++k) {
-    const float s0 = fmaxf(fmaxf((box.hi[k] - box.lo[k]) * (1.0f / 254.0f), 6.0e-8f * fmaxf(fabsf(box.lo[k]), fabsf(box.hi[k]))),
-                           1.0e-30f);
+    const float lo = __fsub_rd(box.lo[k], B.centre[k]), hi = __fsub_ru(box.hi[k], B.centre[k]);
+    const float s0 = fmaxf(fmaxf((hi - lo) * (1.0f / 254.0f), 6.0e-8f * fmaxf(fabsf(lo), fabsf(hi))), 1.0e-30f);
     int e = (int)(__float_as_uint(s0) >> 23) - 127;
     if (__float_as_uint(s0) & 0x7FFFFFu) ++e;
     for (;; ++e) {
       fits = fits && e <= 112;  // 2^15 s is a finite float
       if (!fits) break;
-      const float st = __uint_as_float((uint32_t)(e + 127) << 23);
+      step[k] = __uint_as_float((uint32_t)(e + 127) << 23);
       inv[k] = __uint_as_float((uint32_t)(127 - e) << 23);
-      org[k] = __fsub_rd(box.lo[k], st * (1.0f / 32.0f));
-      if ((box.hi[k] - org[k]) * inv[k] + 1.0f / 60.0f <= 255.0f) break;
+      org[k] = __fsub_rd(__fsub_rd(lo, step[k] * (1.0f / 32.0f)), step[k] * 32768.0f);
+      if (((hi - org[k]) - step[k] * 32768.0f) * inv[k] + 1.0f / 32.0f <= 255.0f) break;
     }
-    expo[k] = (uint32_t)(e + 15 + 127);
   }
   const int cnt = x < 0 || !leaf ? 0 : (x < B.n ? 1 : (int)B.cut[x - B.n].prims);
   const uint32_t imask = __reduce_or_sync(group, x >= 0 && !leaf ? 1u << slot : 0u);
@@ -750,8 +750,8 @@ __device__ void emit_node(const Build &B, uint32_t w, bool valid, int32_t *xn, i
     if (lane == 0u) B.ctr[kCFail] = 1u;
     return;
   }
-  uint4 *o = B.wnodes + (size_t)w * (kWideWords / 4);
-  uint8_t *q = reinterpret_cast<uint8_t *>(o + 2);
+  uint32_t *o = B.wnodes + (size_t)w * kWideWords;
+  uint8_t *q = reinterpret_cast<uint8_t *>(o + 8);
   if (x < 0) {  // an empty slot: a box turned inside out, and neither mask names it
     int skip = (int)lane - nk;
     uint32_t f = free_slots;
@@ -760,8 +760,9 @@ __device__ void emit_node(const Build &B, uint32_t w, bool valid, int32_t *xn, i
     for (int k = 0; k < 3; ++k) { q[8 * k + e] = 255; q[24 + 8 * k + e] = 0; }
   } else {
     for (int k = 0; k < 3; ++k) {
-      const float lo = floorf((kb.lo[k] - org[k]) * inv[k] - 1.0f / 60.0f);
-      const float hi = ceilf((kb.hi[k] - org[k]) * inv[k] + 1.0f / 60.0f);
+      const double g = (double)org[k] + 32768.0 * (double)step[k];  // exact: the grid's origin
+      const float lo = floorf((float)((double)kb.lo[k] - B.centre[k] - g) * inv[k] - 1.0f / 60.0f);
+      const float hi = ceilf((float)((double)kb.hi[k] - B.centre[k] - g) * inv[k] + 1.0f / 60.0f);
       q[8 * k + slot] = (uint8_t)fminf(fmaxf(lo, 0.0f), 255.0f);
       q[24 + 8 * k + slot] = (uint8_t)fminf(fmaxf(hi, 0.0f), 255.0f);
     }
@@ -792,9 +793,14 @@ __device__ void emit_node(const Build &B, uint32_t w, bool valid, int32_t *xn, i
     }
   }
   if (lane == 0u) {
-    o[0] = make_uint4(__float_as_uint(org[0]), __float_as_uint(org[1]), __float_as_uint(org[2]),
-                      expo[0] | (expo[1] << 8) | (expo[2] << 16) | (imask << 24));
-    o[1] = make_uint4(cb, tb, tvalid, 0u);
+    for (int k = 0; k < 3; ++k) {
+      o[k] = __float_as_uint(org[k]);
+      o[4 + k] = __float_as_uint(step[k] * 32768.0f);
+    }
+    o[3] = cb;
+    o[7] = tb;
+    o[20] = imask;
+    o[21] = tvalid;
   }
 }
 
@@ -921,8 +927,8 @@ size_t wide_scratch(int64_t n) {
   return n > 0 && n <= kSmall ? place_scratch(B, n, nullptr) : 0;
 }
 
-int wide_build(const F4 *tris, int64_t n, void *wnodes, F4 *wtris, void *scratch, cudaStream_t st, uint32_t *nodes_out,
-               bool *ok) {
+int wide_build(const F4 *tris, int64_t n, const float *centre, void *wnodes, F4 *wtris, void *scratch, cudaStream_t st,
+               uint32_t *nodes_out, bool *ok) {
   *ok = false;
   *nodes_out = 0;
   if (n <= 0) return MGPU_OK;
@@ -930,8 +936,9 @@ int wide_build(const F4 *tris, int64_t n, void *wnodes, F4 *wtris, void *scratch
   memset(&B, 0, sizeof(B));
   B.n = (int32_t)n;
   B.tris = tris;
-  B.wnodes = (uint4 *)wnodes;
+  B.wnodes = (uint32_t *)wnodes;
   B.wtris = wtris;
+  for (int k = 0; k < 3; ++k) B.centre[k] = centre[k];
   B.cap_nodes = (uint32_t)wide_node_cap(n);
   const int radix_blocks = (int)((n + kRadixTile - 1) / kRadixTile);
   const size_t bytes = place_scratch(B, n, nullptr);

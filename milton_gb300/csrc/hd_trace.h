@@ -52,8 +52,10 @@ struct SceneView {
   const F4 *spheres;       // 2 per analytic sphere: (center, radius), world-to-object quaternion
   int32_t nsphere;         // spheres are primitives ntri .. ntri + nsphere - 1
 #if defined(__CUDACC__)
-  const uint4 *wnodes;     // 8-wide hierarchy (hd_wide.h), nullptr: none
+  const uint32_t *wnodes;  // 8-wide hierarchy (hd_wide.h), nullptr: none
   const F4 *wtris;         // its triangle records, 3 per triangle
+  float wcentre[3];        // what its node coordinates are relative to
+  float wextent;           // the largest coordinate of its box from there
 #endif
 };
 

@@ -297,15 +297,20 @@ __global__ void __launch_bounds__(kBlock) k_generate(RenderArgs a) {
 // extend: closest hit for the live queue of bounce b
 // Traversal: the 8-wide hierarchy (hd_wide.h), or the kd-tree, one ray per lane, for a scene that has
 // none and with mgpu_tune_set("wide", 0).
-constexpr int kWideSmem = kWideBlock / 32 * (int)sizeof(WideShared);
+struct WideBlockShared {
+  WideShared warp[kWideBlock / 32];
+  WideTables tables;
+  uint32_t next;
+};
+constexpr int kWideSmem = (int)sizeof(WideBlockShared);
 
-__device__ __forceinline__ WideShared &wide_shared(uint32_t *&next) {
+__device__ __forceinline__ WideBlockShared &wide_shared() {
   extern __shared__ __align__(16) unsigned char wide_smem[];
-  __shared__ uint32_t counter;
-  if (threadIdx.x == 0) counter = 0u;
+  WideBlockShared &s = *reinterpret_cast<WideBlockShared *>(wide_smem);
+  wide_tables(s.tables);
+  if (threadIdx.x == 0) s.next = 0u;
   __syncthreads();
-  next = &counter;
-  return reinterpret_cast<WideShared *>(wide_smem)[threadIdx.x >> 5];
+  return s;
 }
 
 template <bool COUNT, bool WIDE, bool SPH>
@@ -330,10 +335,10 @@ __global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMi
     auto store = [&](uint32_t i, bool hit, const Hit &h) {
       qhit[i] = make_float4(hit ? h.t : INFINITY, __int_as_float(hit ? h.prim : -1), hit ? h.b1 : 0.0f, hit ? h.b2 : 0.0f);
     };
-    uint32_t *next;
-    WideShared &sh = wide_shared(next);
-    if (single) wide_trace<false, SPH, COUNT, SPH, true>(view0, n, load, store, sh, next, &c, rays);
-    else wide_trace<false, SPH, COUNT, SPH, false>(view_of, n, load, store, sh, next, &c, rays);
+    WideBlockShared &ws = wide_shared();
+    WideShared &sh = ws.warp[threadIdx.x >> 5];
+    if (single) wide_trace<false, SPH, COUNT, SPH, true, true>(view0, n, load, store, sh, ws.tables, &ws.next, &c, rays);
+    else wide_trace<false, SPH, COUNT, SPH, false, true>(view_of, n, load, store, sh, ws.tables, &ws.next, &c, rays);
   } else {
     auto store = [&](uint32_t i, bool hit, const TravState &st) {
       qhit[i] = make_float4(hit ? st.best : INFINITY, __int_as_float(hit ? st.best_prim : -1), hit ? st.bb1 : 0.0f,
@@ -582,10 +587,10 @@ __global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMi
     if (hit) slots[__float_as_uint(so[i].w)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   };
   if constexpr (WIDE) {
-    uint32_t *next;
-    WideShared &sh = wide_shared(next);
-    if (single) wide_trace<true, SPH, COUNT, SPH, true>(view0, n, load, store, sh, next, &c, rays);
-    else wide_trace<true, SPH, COUNT, SPH, false>(view_of, n, load, store, sh, next, &c, rays);
+    WideBlockShared &ws = wide_shared();
+    WideShared &sh = ws.warp[threadIdx.x >> 5];
+    if (single) wide_trace<true, SPH, COUNT, SPH, true, true>(view0, n, load, store, sh, ws.tables, &ws.next, &c, rays);
+    else wide_trace<true, SPH, COUNT, SPH, false, true>(view_of, n, load, store, sh, ws.tables, &ws.next, &c, rays);
   } else {
     grid_trace<true, COUNT, SPH>(view_of, nullptr, 0, n, load, store, &c, rays);
   }

@@ -52,10 +52,11 @@ __global__ void __launch_bounds__(kTraceWideBlock, 4)
     k_trace_wide(const __grid_constant__ SceneView s, const float4 *__restrict__ rays, float4 *__restrict__ hits,
                  uint8_t *__restrict__ occ, uint32_t n) {
   __shared__ WideShared wsh[kTraceWideBlock / 32];
+  __shared__ WideTables tables;
   __shared__ uint32_t next;
+  wide_tables(tables);
   if (threadIdx.x == 0) next = 0u;
   __syncthreads();
-  uint32_t done = 0;
   auto load = [&](uint32_t i, Ray &r) {
     float4 a = __ldg(rays + 2 * (size_t)i), b = __ldg(rays + 2 * (size_t)i + 1);
     r.o = v3(a.x, a.y, a.z);
@@ -67,8 +68,8 @@ __global__ void __launch_bounds__(kTraceWideBlock, 4)
     if (ANY) occ[i] = hit ? 1 : 0;
     else hits[i] = make_float4(hit ? h.t : INFINITY, __int_as_float(hit ? h.prim : -1), hit ? h.b1 : 0.0f, hit ? h.b2 : 0.0f);
   };
-  wide_trace<ANY, true, false, true, true>([&](uint32_t) -> const SceneView & { return s; }, n, load, store,
-                                           wsh[threadIdx.x >> 5], &next, nullptr, done);
+  wide_trace_refill<ANY, true, true>([&](uint32_t) -> const SceneView & { return s; }, n, load, store,
+                                     wsh[threadIdx.x >> 5], tables, &next);
 }
 
 template <bool ANY, bool COUNT>
