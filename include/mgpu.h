@@ -312,9 +312,9 @@ int mgpu_render(const mgpu_scene *scene, const mgpu_render_params *params, mgpu_
  * 32 MiB device array compiled into libmgpu.so; every GPU that loads the library's rendering
  * module holds it until the process exits.  The caller still provides the inputs and outputs: a
  * scene from mgpu_scene_create and a film from mgpu_film_create, made beforehand.
- *   - The scratch bounds the wave: with 4 light samples per vertex it holds about 65 000
- *     paths in flight (wave_paths 0 picks the most that fit), so large frames render slower
- *     than with mgpu_render.  A wave_paths above that capacity is rejected with
+ *   - The scratch bounds the wave: with 4 light samples per vertex wave_paths may be up to about
+ *     65 000 paths in flight (wave_paths 0 picks the most that fit, about 89 000), so large frames
+ *     render slower than with mgpu_render.  A wave_paths above the limit is rejected with
  *     MGPU_E_INVALID and a message naming the capacity; nothing is rendered.
  *   - The array comes into existence when the rendering module is loaded on a device.  Under
  *     CUDA's lazy module loading (the default) that is the first render call of any kind on
@@ -369,9 +369,11 @@ int mgpu_profile_read(double *ms6, uint64_t *launches6);
  *                    device (default 1); 0 = the kd-tree, one ray per lane
  *   "persistent" 0/1, "coop_leaf" 0..3, "trav_block" 64 / 128 / 256: shapes of earlier kd-tree
  *                    kernels; accepted and read back, they select nothing
- *   "bin_shadow"     0/1  counting-sort shadow rays by (light, origin cell) (default 1)
  *   "bin_extension"  0/1  counting-sort extension rays by (direction octant, origin cell) (default 1)
- *   "bin_min_paths"  n    waves of fewer paths are not binned (default 2^22)
+ *   "bin_min_paths"  n    waves of fewer paths are not sorted (default 2^25), nor are waves of scenes
+ *                    below 300,000 triangles; 0 = every wave is
+ *   "bin_shadow"     0/1  a sort of the shadow rays that is no more; accepted and read back, selects
+ *                    nothing
  *   "carveout"       -2..100  shared-memory carveout (percent) preferred for the traversal and
  *                    shade kernels: -2 = per kernel, the least shared memory that keeps all its
  *                    register-limited resident blocks, the rest of the SM's memory as L1

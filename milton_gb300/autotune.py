@@ -2,8 +2,8 @@
 capacity) and queue binning by timing a short calibration render of the actual requests, and caches
 the choice per workload size class.  Results never depend on these knobs (every path draws its
 own counter-based random numbers and each film sums its samples in sample order), only speed does.
-The "persistent" and "trav_block" entries select nothing any more (include/mgpu.h); they are kept at
-one value so that a configuration still names them."""
+The "persistent", "bin_shadow" and "trav_block" entries select nothing any more (include/mgpu.h); they
+are kept at one value so that a configuration still names them."""
 from __future__ import annotations
 
 import itertools
@@ -12,7 +12,7 @@ import math
 from . import pathtracer as pt
 
 WAVES = (1 << 21, 1 << 22, 1 << 23, 1 << 24, 1 << 25, 1 << 26)
-SHAPES = ((0, 1, 1), (0, 1, 0), (0, 0, 1), (0, 0, 0))  # (persistent, bin_shadow, bin_extension)
+SHAPES = ((0, 1, 1), (0, 1, 0))  # (persistent, bin_shadow, bin_extension)
 BLOCKS = (256,)
 
 _cache: dict = {}

@@ -490,6 +490,7 @@ int mgpu_scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void
   s->d_mats = (float *)(base + off_mats);
   s->d_lights = (float *)(base + off_lights);
   s->nmat = desc->nmat;
+  for (int i = 1; i < desc->nmat; ++i) s->mixed = s->mixed || desc->materials[16 * i] != desc->materials[0];
   s->nlight = desc->nlight;
   bool wide = false;
   uint32_t wide_nodes = 0;

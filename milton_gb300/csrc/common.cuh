@@ -73,6 +73,7 @@ struct mgpu_scene {
   mgpu::SceneView view{};       // device pointers
   float4 *d_shade = nullptr;    // 3 per triangle: (n0, mat), (n1, light), (n2, 0)
   float *d_mats = nullptr;
+  bool mixed = false;           // its materials have more than one kind of BSDF
   float *d_lights = nullptr;
   float2 *d_uv = nullptr;       // 3 per triangle by id (nullptr: every uv is (0, 0))
   float4 *d_texrec = nullptr;   // 2 per texture: (texel offset, width, height, kind), (repeat u, v, bump intensity, 0)

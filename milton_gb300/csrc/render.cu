@@ -42,15 +42,10 @@ constexpr int kNumCounters = kCtrTrunc + 8;
 constexpr int kBinBits = 14;           // queue binning keys: 2^14 bins
 constexpr int kBins = 1 << kBinBits;
 constexpr int kBinSmem = kBins * 4;    // dynamic shared memory of a sorting block
+constexpr int64_t kBinMinTris = 300000;   // smallest scene whose extension rays are sorted
 constexpr double kAutoWaveBytes = 40e9;  // workspace budget of an automatic wave
 // Resident 128-thread blocks per SM that the kd-tree kernels are compiled for: 40 registers
 constexpr int kTravMinBlocks = 12;
-#ifndef MGPU_SHADE_MIN_BLOCKS
-#define MGPU_SHADE_MIN_BLOCKS 8
-#endif
-// the shade kernel at 8 blocks per SM (64 registers, spilling ~0.8 KB to L1) against its natural
-// 125 registers: 211 -> 184 ms per 5 mid frames
-constexpr int kShadeMinBlocks = MGPU_SHADE_MIN_BLOCKS;
 
 // One job chunk of a wave (device memory).
 struct JobArgs {
@@ -63,7 +58,7 @@ struct JobArgs {
   const float4 *texels;
   int32_t bg_tex;          // background environment map (1 + texture index) or 0
   float bg_le[3];          // constant background radiance (bg_tex == 0)
-  int32_t nlight, nl_slots, sh_cell_bits;
+  int32_t nlight, nl_slots;
   float cell_scale[3];     // queue-bin cells: 32 / the scene's extent per axis (0: a flat axis)
   Camera cam;
   Rng rng;
@@ -92,9 +87,9 @@ struct RenderArgs {
   float4 *so, *sd;               // shadow ray queue: origin + slot index, direction + tmax
   float4 *slots;                 // nl_stride per path: direct-light contribution per light sample
   float4 *qo_u, *qd_u, *qt_u;    // unsorted next-ray queue (binning on)
-  float4 *so_u, *sd_u;           // unsorted shadow queue (binning on)
-  uint32_t *qkey, *skey;         // bin keys of the unsorted queues
-  int32_t bin_ext, bin_sh;       // counting-sort the queues by (direction octant | light, origin cell)
+  uint32_t *qkey;                // bin keys of the unsorted queue
+  int32_t bin_ext;               // counting-sort the queue by (direction octant, origin cell)
+  int32_t sort_hits;             // a scene of the wave has more than one kind of BSDF
   uint32_t *counters;
   unsigned long long *stats;     // [0] extension rays, [1] shadow rays, [2] truncated paths, [3] bounces
   unsigned long long *tcount;    // counted mode: ext nodes, refs, tris, rays; shadow nodes, refs, tris, rays
@@ -217,8 +212,8 @@ __device__ __forceinline__ Light load_light(const JobArgs &J, int i) {
 
 // Binning keys (kBins = 16384).  Ray coherence: rays of one warp should start close together
 // and head the same way, so that they visit the same nodes.  Keys combine the direction
-// octant (extension rays) or the light index (shadow rays) with the Morton code of the
-// origin's cell in a 32x32x32 grid over the scene bounds (the top bits of it that fit).
+// octant with the Morton code of the origin's cell in a 32x32x32 grid over the scene bounds (the
+// top bits of it that fit).
 __device__ __forceinline__ uint32_t spread4(uint32_t v) {  // 4 bits -> every third bit
   return (v & 1u) | ((v & 2u) << 2) | ((v & 4u) << 4) | ((v & 8u) << 6);
 }
@@ -243,11 +238,6 @@ __device__ __forceinline__ uint32_t morton15(const JobArgs &J, V3 p) {
 __device__ __forceinline__ uint32_t ext_key(const JobArgs &J, V3 o, V3 d) {
   uint32_t oct = (d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u);
   return (oct << (kBinBits - 3)) | (morton15(J, o) >> (18 - kBinBits));
-}
-
-__device__ __forceinline__ uint32_t sh_key(const JobArgs &J, int light, V3 o) {
-  uint32_t cell = morton15(J, o) >> (15 - J.sh_cell_bits);
-  return (((uint32_t)light << J.sh_cell_bits) | cell) & (kBins - 1);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -365,17 +355,116 @@ __device__ __forceinline__ V3 fold_slots(const RenderArgs &a, int nl, int64_t p,
   return L;
 }
 
+// Threads of a shading block, and the rays that it takes at a time; four blocks per SM (64 registers; the
+// kernel's natural 125 and the spills of 48 both measure slower).
+constexpr int kShadeTile = 256;
+constexpr int kShadeMinBlocks = 4;
+
+// What a shading block keeps in shared memory: per warp the shadow rays that wait for a full 32, and the
+// counts and the order of the tile's rays.
+struct ShadeShared {
+  float4 so[kShadeTile / 32][64], sd[kShadeTile / 32][64];
+  uint32_t cnt[kShadeTile / 4];
+  uint8_t perm[kShadeTile];
+};
+
+// Position of the thread among the block's threads ordered by key (0..7).  cnt: 64 words that no thread
+// still reads.
+__device__ __forceinline__ uint32_t tile_rank(uint32_t *cnt, uint32_t key) {
+  constexpr unsigned kFull = 0xFFFFFFFFu;
+  static_assert(kShadeTile == 256, "eight warps");
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t mine = 0u, peers = 0u;
+#pragma unroll
+  for (uint32_t k = 0; k < 8u; ++k) {
+    const uint32_t m = __ballot_sync(kFull, key == k);
+    if (key == k) peers = m;
+    if (lane == k) mine = __popc(m);
+  }
+  if (lane < 8u) cnt[8u * lane + warp] = mine;
+  __syncthreads();
+  // exclusive prefix sums of the 64 counts, two per lane, by every warp for itself
+  const uint32_t x = cnt[2u * lane], y = cnt[2u * lane + 1u];
+  uint32_t inc = x + y;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t v = __shfl_up_sync(kFull, inc, d);
+    if (lane >= (uint32_t)d) inc += v;
+  }
+  const uint32_t at = 8u * key + warp;
+  const uint32_t ex = __shfl_sync(kFull, inc - x - y, at >> 1), x0 = __shfl_sync(kFull, x, at >> 1);
+  return ex + ((at & 1u) ? x0 : 0u) + __popc(peers & ((1u << lane) - 1u));
+}
+
+// A warp's shadow rays on their way to the queue: 32 at a time, one atomic and two coalesced stores (one
+// atomic per warp and light sample was 20 M to one address on the mid frame).
+struct ShadowStage {
+  float4 *o, *d;       // ring of 64
+  uint32_t *counter;
+  float4 *so, *sd;
+  uint32_t head, count;  // uniform over the warp
+  __device__ __forceinline__ void write(uint32_t m) {
+    const uint32_t lane = threadIdx.x & 31u;
+    __syncwarp();
+    uint32_t at = 0u;
+    if (lane == 0u) at = atomicAdd(counter, m);
+    at = __shfl_sync(0xFFFFFFFFu, at, 0);
+    if (lane < m) {
+      so[at + lane] = o[(head + lane) & 63u];
+      sd[at + lane] = d[(head + lane) & 63u];
+    }
+    __syncwarp();
+    head = (head + m) & 63u;
+    count -= m;
+  }
+  __device__ __forceinline__ void append(bool want, float4 o4, float4 d4) {
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, want);
+    if (want) {
+      const uint32_t e = (head + count + __popc(m & ((1u << (threadIdx.x & 31u)) - 1u))) & 63u;
+      o[e] = o4;
+      d[e] = d4;
+    }
+    count += __popc(m);
+    if (count >= 32u) write(32u);
+  }
+  __device__ __forceinline__ void flush() {
+    if (count) write(count);
+  }
+};
+
 // SURF: the wave has a scene with image maps, a background or analytic spheres.  Scenes without
 // them run the variant that has none of those branches, whose register allocation (and spilling)
 // is the lighter.
 template <bool SURF>
-__global__ void __launch_bounds__(kBlock, kShadeMinBlocks) k_shade(RenderArgs a, int b) {
+__global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(RenderArgs a, int b) {
+  __shared__ ShadeShared sh;
   const uint32_t n = a.counters[kCtrRay + b];
   const int cur = b & 1, nxt = (b + 1) & 1;
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
+  const uint32_t stride = gridDim.x * kShadeTile;
+  ShadowStage stage{sh.so[threadIdx.x >> 5], sh.sd[threadIdx.x >> 5], &a.counters[kCtrNee + b], a.so, a.sd, 0u, 0u};
+  for (uint32_t base = blockIdx.x * kShadeTile; base < n; base += stride) {
+    // the tile's rays in the order of what they hit: with the BSDFs of a tile side by side a warp runs one of
+    // them, and the barriers keep the block's warps in the same part of a kernel that exceeds the
+    // instruction cache (ncu, mid scene, second bounce: lanes per instruction 13.7 -> 24.9, warps waiting
+    // for instructions 9.6 -> 0.7 per issue; 30.7 -> 24.5 ms of the mid frame.  Sorted by warps of 128 rays,
+    // without barriers: 28.7)
     uint32_t i = base + threadIdx.x;
-    bool valid = i < n;
+    if (a.sort_hits) {
+      uint32_t cls = 4u;
+      if (i < n) {
+        const int prim = __float_as_int(a.qhit[i].y);
+        cls = 3u;
+        if (prim >= 0) {
+          const JobArgs &J = a.jobs[__float_as_int(a.qd[cur][i].w)];
+          const int mi = __float_as_int(__ldg(J.shade + 3 * (int64_t)prim).w);
+          cls = min((uint32_t)__ldg(J.mats + 4 * mi).x, 2u);
+        }
+      }
+      sh.perm[tile_rank(sh.cnt, cls)] = (uint8_t)threadIdx.x;
+      __syncthreads();
+      i = base + sh.perm[threadIdx.x];
+    }
+    const bool valid = i < n;
     bool want_next = false, do_nee = false;
     float4 no_o, no_d, no_t;
     int64_t p = 0;
@@ -467,7 +556,7 @@ __global__ void __launch_bounds__(kBlock, kShadeMinBlocks) k_shade(RenderArgs a,
       a.path_L[p] = make_float4(L.x, L.y, L.z, __uint_as_float(flags));
     }
     const JobArgs &J = a.jobs[j];
-    uint32_t q = warp_append(&a.counters[kCtrRay + b + 1], want_next);
+    const uint32_t q = warp_append(&a.counters[kCtrRay + b + 1], want_next);
     if (want_next) {
       if (a.bin_ext) {
         a.qo_u[q] = no_o;
@@ -546,20 +635,12 @@ __global__ void __launch_bounds__(kBlock, kShadeMinBlocks) k_shade(RenderArgs a,
         }
         a.slots[p * a.nl_stride + k] = make_float4(c.x, c.y, c.z, 0.0f);
       }
-      uint32_t e = warp_append(&a.counters[kCtrNee + b], want);
-      if (want) {
-        if (a.bin_sh) {
-          a.so_u[e] = so4;
-          a.sd_u[e] = sd4;
-          a.skey[e] = sh_key(J, k / s2n, P);
-        } else {
-          a.so[e] = so4;
-          a.sd[e] = sd4;
-        }
-      }
+      stage.append(want, so4, sd4);
     }
   }
+  stage.flush();
 }
+
 
 // shadow: any-hit query per queued light sample; an occluded sample's slot is zeroed
 template <bool COUNT, bool WIDE, bool SPH>
@@ -640,7 +721,6 @@ __global__ void __launch_bounds__(1024) k_bin_scan(const uint32_t *__restrict__ 
   for (int k = 0; k < per; ++k) cursor[threadIdx.x * per + k] = base + loc[k];
 }
 
-template <int NF4>
 __global__ void __launch_bounds__(256) k_bin_scatter(const uint32_t *__restrict__ keys, const uint32_t *count,
                                                     uint32_t *__restrict__ cursor, const float4 *__restrict__ in0,
                                                     const float4 *__restrict__ in1, const float4 *__restrict__ in2,
@@ -670,8 +750,8 @@ __global__ void __launch_bounds__(256) k_bin_scatter(const uint32_t *__restrict_
       if (i < n) {
         uint32_t pos = h[key[k]] + rank[k];
         out0[pos] = in0[i];
-        if (NF4 > 1) out1[pos] = in1[i];
-        if (NF4 > 2) out2[pos] = in2[i];
+        out1[pos] = in1[i];
+        out2[pos] = in2[i];
       }
     }
     __syncthreads();
@@ -764,8 +844,8 @@ struct Workspace {
   void *block = nullptr;
   float4 *path_L = nullptr, *qo[2] = {}, *qd[2] = {}, *qt[2] = {}, *qhit = nullptr;
   float4 *so = nullptr, *sd = nullptr, *slots = nullptr;
-  float4 *qo_u = nullptr, *qd_u = nullptr, *qt_u = nullptr, *so_u = nullptr, *sd_u = nullptr;
-  uint32_t *qkey = nullptr, *skey = nullptr, *hist = nullptr, *cursor = nullptr;  // hist/cursor: kBins each
+  float4 *qo_u = nullptr, *qd_u = nullptr, *qt_u = nullptr;
+  uint32_t *qkey = nullptr, *hist = nullptr, *cursor = nullptr;  // hist/cursor: kBins each
   uint32_t *path_job = nullptr;
   JobArgs *jobs = nullptr;
   uint32_t *counters = nullptr;
@@ -788,11 +868,15 @@ struct Tuning {
   std::atomic<int> wide{1};
   // shapes of kd-tree kernels that are no more: kept for callers that set and read them back
   std::atomic<int> persistent{0}, coop_leaf{3}, trav_block{256};
-  std::atomic<int> bin_shadow{1};     // counting-sort shadow rays by (light, origin cell)
   std::atomic<int> bin_extension{1};  // counting-sort extension rays by (octant, origin cell)
-  // waves of fewer paths skip binning: sorting a few hundred thousand rays costs more (four
-  // latency-bound launches per bounce) than the coherence it buys
-  std::atomic<int64_t> bin_min_paths{(int64_t)1 << 22};
+  // waves of fewer paths, and scenes of fewer than kBinMinTris triangles, skip the sort: it pays where
+  // tree and triangles are well beyond the L1s (64 M paths, sorted against not: 1 M triangles 117.5 / 120.5 ms,
+  // 300 k 81.8 / 82.3, 150 k 60.2 / 60.1, 50 k 31.8 / 30.8, 36 triangles 68.9 / 57.3; 16 M paths of 1 M
+  // triangles 30.95 / 31.02).  0: sort every wave.
+  std::atomic<int64_t> bin_min_paths{(int64_t)1 << 25};
+  // a sort of the shadow rays cost more than it saved and is no more (1 M triangles, 64 M paths: 6.1 ms of sorting
+  // and key writes for 3.5 of traversal); kept for callers that set and read it back
+  std::atomic<int> bin_shadow{1};
   // shared-memory carveout (%) of the traversal / shade kernels: -2 = per kernel, the least that
   // keeps its resident blocks (the rest of the SM's 256 KB is L1); -1 = the driver's choice
   std::atomic<int> carveout{kCarveoutAuto};
@@ -854,11 +938,10 @@ struct Profiler {
 static thread_local Profiler t_prof;
 
 // float4 arrays: path_L, 2 x (qo, qd, qt), qhit, unsorted (qo, qd, qt) = 11 per path;
-// so, sd, slots, unsorted (so, sd) = 5 per light sample; uint32 keys per path and per sample,
-// path_job per path; JobArgs entries
+// so, sd, slots = 3 per light sample; a uint32 key and path_job per path; JobArgs entries
 static size_t workspace_bytes(int64_t paths, int64_t slots, int64_t jobs) {
-  size_t f4 = (size_t)paths * 11 + (size_t)slots * 5;
-  size_t u32 = (size_t)paths * 2 + (size_t)slots + 2 * kBins + kNumCounters;
+  size_t f4 = (size_t)paths * 11 + (size_t)slots * 3;
+  size_t u32 = (size_t)paths * 2 + 2 * kBins + kNumCounters;
   return f4 * sizeof(float4) + (size_t)jobs * sizeof(JobArgs) + 12 * sizeof(unsigned long long) +
          u32 * sizeof(uint32_t) + 1024;
 }
@@ -874,14 +957,12 @@ static void workspace_layout(Workspace *w, void *block, int64_t paths, int64_t s
   w->qhit = f; f += paths;
   w->qo_u = f; f += paths; w->qd_u = f; f += paths; w->qt_u = f; f += paths;
   w->so = f; f += slots; w->sd = f; f += slots; w->slots = f; f += slots;
-  w->so_u = f; f += slots; w->sd_u = f; f += slots;
   w->jobs = (JobArgs *)f;  // JobArgs is a multiple of 8 bytes; float4 alignment holds
   w->stats = (unsigned long long *)(w->jobs + jobs);
   w->tcount = w->stats + 4;
   uint32_t *u = (uint32_t *)(w->tcount + 8);
   w->qkey = u; u += paths;
   w->path_job = u; u += paths;
-  w->skey = u; u += slots;
   w->hist = u; u += kBins;
   w->cursor = u; u += kBins;
   w->counters = u;
@@ -946,11 +1027,11 @@ static int noalloc_scratch(void **out) {
   return MGPU_OK;
 }
 
-// paths per wave that fit the fixed scratch for nl_slots light samples per path
-static int64_t noalloc_paths(int64_t nl_slots) {
+// paths per wave that fit the fixed scratch for nl_slots light samples per path; asked: the limit of an
+// explicit wave_paths, which stays what it was when a light sample took 84 bytes (now 48)
+static int64_t noalloc_paths(int64_t nl_slots, bool asked) {
   const size_t fixed = workspace_bytes(0, 0, kNoAllocJobs);
-  const size_t per = 11 * sizeof(float4) + 2 * sizeof(uint32_t) +
-                     (size_t)nl_slots * (5 * sizeof(float4) + sizeof(uint32_t));
+  const size_t per = 11 * sizeof(float4) + 2 * sizeof(uint32_t) + (size_t)nl_slots * (asked ? 84 : 3 * sizeof(float4));
   if (kNoAllocBytes <= fixed) return 0;
   int64_t p = (int64_t)((kNoAllocBytes - fixed) / per);
   return p / 64 * 64;
@@ -983,8 +1064,8 @@ static std::vector<CarveoutKernel> carveout_kernels() {
           {(const void *)k_extend<true, false, true>, kBlock, 0},
           {(const void *)k_shadow<false, false, true>, kBlock, 0},
           {(const void *)k_shadow<true, false, true>, kBlock, 0},
-          {(const void *)k_shade<false>, kBlock, 0},
-          {(const void *)k_shade<true>, kBlock, 0}};
+          {(const void *)k_shade<false>, kShadeTile, 0},
+          {(const void *)k_shade<true>, kShadeTile, 0}};
 }
 
 // percent of the SM's shared memory that holds the kernel's resident blocks (registers and
@@ -1014,7 +1095,7 @@ static cudaError_t kernel_attributes() {
   if ((int)applied.size() <= dev) applied.resize((size_t)dev + 1, INT_MIN);
   if (applied[(size_t)dev] == want) return cudaSuccess;
   if (applied[(size_t)dev] == INT_MIN) {
-    const void *bins[] = {(const void *)k_bin_hist, (const void *)k_bin_scatter<2>, (const void *)k_bin_scatter<3>};
+    const void *bins[] = {(const void *)k_bin_hist, (const void *)k_bin_scatter};
     for (const void *kf : bins)
       if ((e = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, kBinSmem)) != cudaSuccess) return e;
     for (const CarveoutKernel &k : carveout_kernels())
@@ -1130,11 +1211,6 @@ static JobArgs job_args(const Job &j) {
   J.filt = j.film->filter;
   J.film_fx = j.film->d_fx;
   J.path_out = (float4 *)j.path_out;
-  int nlp = 1;
-  while (nlp < std::min(sc->nlight, 16)) nlp <<= 1;
-  int lb = 0;
-  while ((1 << lb) < nlp) ++lb;
-  J.sh_cell_bits = std::min(15, kBinBits - lb);  // light index in the top bits, origin cell below
   for (int k = 0; k < 3; ++k) {
     const float ext = J.view.bmax[k] - J.view.bmin[k];
     J.cell_scale[k] = ext > 0.0f ? 32.0f / ext : 0.0f;
@@ -1225,7 +1301,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
     while (wave > ((int64_t)1 << 20) && (double)wave * per_path > kAutoWaveBytes) wave >>= 1;
   }
   if (noalloc) {
-    const int64_t pmax = noalloc_paths(nl_max);
+    const int64_t pmax = noalloc_paths(nl_max, true);
     if (pmax < 64)
       return fail(MGPU_E_INVALID, "mgpu_render_noalloc: " + std::to_string(nl_max) +
                                       " light samples per vertex do not fit the 32 MiB fixed scratch");
@@ -1233,7 +1309,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
       return fail(MGPU_E_INVALID, "mgpu_render_noalloc: wave_paths " + std::to_string(wave_req) +
                                       " exceeds the fixed scratch (32 MiB holds " + std::to_string(pmax) +
                                       " paths at " + std::to_string(nl_max) + " light samples per vertex)");
-    wave = wave_req > 0 ? wave_req : pmax;
+    wave = wave_req > 0 ? wave_req : noalloc_paths(nl_max, false);
   }
   std::vector<Wave> waves;
   bool use_graph = false;
@@ -1288,8 +1364,10 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
   }
 
   bool sph = false;  // a job's scene has analytic spheres: the traversal kernels that test them
+  bool sort_hits = false;
   bool wide = g_tune.wide.load() != 0;  // every scene has the 8-wide hierarchy
   for (const Job &j : jobs) {
+    sort_hits = sort_hits || j.scene->mixed;
     sph = sph || j.scene->view.nsphere > 0;
     wide = wide && (j.scene->view.wnodes != nullptr || j.scene->view.ntri == 0);
   }
@@ -1300,11 +1378,11 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
   MGPU_CUDA(kernel_attributes());
   const int g_gen = grid_for((const void *)k_generate, 0);
   const int g_ext = grid_for((const void *)kext, tsm, tb);
-  const int g_sha = grid_for((const void *)k_shade<true>, 0);
+  const int g_sha = grid_for((const void *)k_shade<true>, 0, kShadeTile);
   const int g_shw = grid_for((const void *)kshw, tsm, tb);
   const int g_acc = grid_for((const void *)k_accumulate, 0);
   const int g_bin = device_sm_count() * 4;
-  const int bin_ext = g_tune.bin_extension.load(), bin_sh = g_tune.bin_shadow.load();
+  const int bin_ext = g_tune.bin_extension.load();
   const int64_t bin_min = g_tune.bin_min_paths.load();
 
   // The launches are captured on a private stream (the caller's may be the legacy default
@@ -1345,10 +1423,12 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
     for (int k = 0; k < 2; ++k) { a.qo[k] = w->qo[k]; a.qd[k] = w->qd[k]; a.qt[k] = w->qt[k]; }
     a.qhit = w->qhit;
     a.so = w->so; a.sd = w->sd; a.slots = w->slots;
-    a.qo_u = w->qo_u; a.qd_u = w->qd_u; a.qt_u = w->qt_u; a.so_u = w->so_u; a.sd_u = w->sd_u;
-    a.qkey = w->qkey; a.skey = w->skey;
-    a.bin_ext = wv.npaths >= bin_min ? bin_ext : 0;
-    a.bin_sh = wv.npaths >= bin_min ? bin_sh : 0;
+    a.qo_u = w->qo_u; a.qd_u = w->qd_u; a.qt_u = w->qt_u;
+    a.qkey = w->qkey;
+    int64_t wave_tris = 0;
+    for (const JobArgs &c : wv.chunks) wave_tris = std::max(wave_tris, c.view.ntri);
+    a.bin_ext = wv.npaths >= bin_min && (wave_tris >= kBinMinTris || bin_min == 0) ? bin_ext : 0;
+    a.sort_hits = sort_hits;
     a.counters = w->counters;
     a.stats = w->stats;
     a.tcount = w->tcount;
@@ -1373,29 +1453,19 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
         kext<<<g_ext, tb, tsm, st>>>(a, b);
         pf.end(m, st);
         m = pf.begin(kProfShade, st);
-        if (surf) k_shade<true><<<g_sha, kBlock, 0, st>>>(a, b);
-        else k_shade<false><<<g_sha, kBlock, 0, st>>>(a, b);
+        if (surf) k_shade<true><<<g_sha, kShadeTile, 0, st>>>(a, b);
+        else k_shade<false><<<g_sha, kShadeTile, 0, st>>>(a, b);
         pf.end(m, st);
-        if (a.bin_sh || a.bin_ext) {
+        if (a.bin_ext && b + 1 < max_b) {
+          const int nx = (b + 1) & 1;
           m = pf.begin(kProfBin, st);
-          if (a.bin_sh) {
-            cudaMemsetAsync(w->hist, 0, kBins * sizeof(uint32_t), st);
-            k_bin_hist<<<g_bin, 256, kBinSmem, st>>>(w->skey, a.counters + kCtrNee + b, w->hist);
-            k_bin_scan<<<1, 1024, 0, st>>>(w->hist, w->cursor);
-            k_bin_scatter<2><<<g_bin, 256, kBinSmem, st>>>(w->skey, a.counters + kCtrNee + b, w->cursor, w->so_u, w->sd_u,
-                                                    nullptr, w->so, w->sd, nullptr);
-            launches += 3;
-          }
-          if (a.bin_ext && b + 1 < max_b) {
-            const int nx = (b + 1) & 1;
-            cudaMemsetAsync(w->hist, 0, kBins * sizeof(uint32_t), st);
-            k_bin_hist<<<g_bin, 256, kBinSmem, st>>>(w->qkey, a.counters + kCtrRay + b + 1, w->hist);
-            k_bin_scan<<<1, 1024, 0, st>>>(w->hist, w->cursor);
-            k_bin_scatter<3><<<g_bin, 256, kBinSmem, st>>>(w->qkey, a.counters + kCtrRay + b + 1, w->cursor, w->qo_u,
-                                                    w->qd_u, w->qt_u, w->qo[nx], w->qd[nx], w->qt[nx]);
-            launches += 3;
-          }
+          cudaMemsetAsync(w->hist, 0, kBins * sizeof(uint32_t), st);
+          k_bin_hist<<<g_bin, 256, kBinSmem, st>>>(w->qkey, a.counters + kCtrRay + b + 1, w->hist);
+          k_bin_scan<<<1, 1024, 0, st>>>(w->hist, w->cursor);
+          k_bin_scatter<<<g_bin, 256, kBinSmem, st>>>(w->qkey, a.counters + kCtrRay + b + 1, w->cursor, w->qo_u, w->qd_u,
+                                                      w->qt_u, w->qo[nx], w->qd[nx], w->qt[nx]);
           pf.end(m, st);
+          launches += 3;
         }
         m = pf.begin(kProfShadow, st);
         kshw<<<g_shw, tb, tsm, st>>>(a, b);
