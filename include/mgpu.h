@@ -270,9 +270,9 @@ int mgpu_film_clear(mgpu_film *film, void *stream);
 int mgpu_film_destroy(mgpu_film *film);
 /* The film's output in FP64: out = host array of width*height*3 doubles (synchronises): the
  * per-pixel mean, or with a reconstruction filter set, sum(w L) / sum(w) over the samples
- * splatted onto each pixel.  The mean is taken on the device in a scratch buffer of 24 bytes
- * per pixel that the calling thread keeps for its later reads (grown to the largest film it
- * has read, released when the thread exits).                                                */
+ * splatted onto each pixel.  Taken on the device, which writes page-locked arrays (mgpu_host_alloc)
+ * itself; a pageable one is filled through at most 12 MB of page-locked staging that the calling
+ * thread keeps for its later reads (released when the thread exits).                          */
 int mgpu_film_read(mgpu_film *film, double *out_mean, void *stream);
 /* Reconstruction filter of ReconstructionRenderOutput (ReconstructionRenderOutput.cpp:30-83):
  * every sample is splatted onto the pixels within (ceil(support) | 1) / 2 of its own with
@@ -381,6 +381,11 @@ int mgpu_profile_read(double *ms6, uint64_t *launches6);
  *                    render                                                                     */
 int mgpu_tune_set(const char *key, int64_t value);
 int mgpu_tune_get(const char *key, int64_t *value);
+
+/* Page-locked host memory for results (film reads, tone maps): the device writes it without a
+ * staging copy.  No counterpart in the reference. */
+int mgpu_host_alloc(uint64_t bytes, void **out);
+int mgpu_host_free(void *p);
 
 /* Read bandwidth of this device (measurement only, no counterpart in the reference): one
  * launch reads a `bytes` buffer (cudaMalloc'd here; >= 4096, a multiple of 16) `reps` times

@@ -103,6 +103,8 @@ SIGNATURES = [
     ("mgpu_film_create", C.c_int, [C.c_int32, C.c_int32, C.c_void_p, C.POINTER(C.c_void_p)]),
     ("mgpu_film_clear", C.c_int, [C.c_void_p, C.c_void_p]),
     ("mgpu_film_destroy", C.c_int, [C.c_void_p]),
+    ("mgpu_host_alloc", C.c_int, [C.c_uint64, C.POINTER(C.c_void_p)]),
+    ("mgpu_host_free", C.c_int, [C.c_void_p]),
     ("mgpu_film_read", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),
     ("mgpu_film_read_raw", C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p]),
     ("mgpu_film_error", C.c_int, [C.POINTER(C.c_void_p), C.c_int32, C.c_void_p, C.c_void_p]),

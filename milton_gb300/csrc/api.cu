@@ -124,22 +124,20 @@ struct FilmRef {
 };
 constexpr int kErrBlocks = 64, kErrThreads = 256;
 
-__global__ void __launch_bounds__(kErrThreads) k_film_error_partial(const FilmRef *films, double2 *partial) {
-  const FilmRef f = films[blockIdx.y];
-  double acc = 0.0, cnt = 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * kErrThreads + threadIdx.x; i < f.npix; i += (int64_t)kErrBlocks * kErrThreads) {
-    const float4 S = f.sum[i], C = f.c[i];
-    const double n = S.w;
-    if (n > 1.0) {
-      const double mean = ((((double)S.x - C.x) + ((double)S.y - C.y)) + ((double)S.z - C.z)) / (3.0 * n);
-      const double var = fmax((double)C.w / n - mean * mean, 0.0) * n / (n - 1.0);
-      acc += var / n;
-      cnt += 1.0;
-    }
-  }
+// Blocks that reduce one film: one per 2,048 pixels within [64, 1024] (by the film alone, so that its value does
+// not depend on the films beside it).  64 for every film left the GPU idle on large ones (483,003
+// pixels: 212 -> 87 us a call, with two divisions a pixel instead of five).
+constexpr int kErrMaxBlocks = 1024;
+__host__ __device__ inline int err_blocks(int64_t npix) {
+  const int64_t b = (npix + 2047) / 2048;
+  return b < kErrBlocks ? kErrBlocks : (b > kErrMaxBlocks ? kErrMaxBlocks : (int)b);
+}
+
+// sum over the block in a fixed tree
+__device__ __forceinline__ void err_reduce(double &a, double &c) {
   __shared__ double sa[kErrThreads], sc[kErrThreads];
-  sa[threadIdx.x] = acc;
-  sc[threadIdx.x] = cnt;
+  sa[threadIdx.x] = a;
+  sc[threadIdx.x] = c;
   __syncthreads();
   for (int w = kErrThreads / 2; w > 0; w >>= 1) {
     if ((int)threadIdx.x < w) {
@@ -148,19 +146,42 @@ __global__ void __launch_bounds__(kErrThreads) k_film_error_partial(const FilmRe
     }
     __syncthreads();
   }
-  if (threadIdx.x == 0) partial[(int64_t)blockIdx.y * kErrBlocks + blockIdx.x] = make_double2(sa[0], sc[0]);
+  a = sa[0];
+  c = sc[0];
 }
 
-__global__ void k_film_error_final(const double2 *partial, int32_t n, double *out) {
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= n) return;
+__global__ void __launch_bounds__(kErrThreads) k_film_error_partial(const FilmRef *films, double2 *partial) {
+  const FilmRef f = films[blockIdx.y];
+  const int nb = err_blocks(f.npix);
+  if ((int)blockIdx.x >= nb) return;
+  double acc = 0.0, cnt = 0.0;
+  for (int64_t i = (int64_t)blockIdx.x * kErrThreads + threadIdx.x; i < f.npix; i += (int64_t)nb * kErrThreads) {
+    const float4 S = f.sum[i], C = f.c[i];
+    const double n = S.w;
+    if (n > 1.0) {
+      // two divisions (FP64 runs at two a clock and SM): 1 / n, and the variance of the mean,
+      // (m2 - mean^2) n / (n - 1) / n
+      const double inv = 1.0 / n;
+      const double mean = ((((double)S.x - C.x) + ((double)S.y - C.y)) + ((double)S.z - C.z)) * (inv * (1.0 / 3.0));
+      acc += fmax((double)C.w * inv - mean * mean, 0.0) / (n - 1.0);
+      cnt += 1.0;
+    }
+  }
+  err_reduce(acc, cnt);
+  if (threadIdx.x == 0) partial[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = make_double2(acc, cnt);
+}
+
+__global__ void __launch_bounds__(kErrThreads) k_film_error_final(const FilmRef *films, const double2 *partial,
+                                                                  int stride, double *out) {
+  const int nb = err_blocks(films[blockIdx.x].npix);
   double a = 0.0, c = 0.0;
-  for (int b = 0; b < kErrBlocks; ++b) {
-    const double2 p = partial[(int64_t)f * kErrBlocks + b];
+  for (int b = threadIdx.x; b < nb; b += kErrThreads) {
+    const double2 p = partial[(int64_t)blockIdx.x * stride + b];
     a += p.x;
     c += p.y;
   }
-  out[f] = c > 0.0 ? sqrt(a / c) : INFINITY;
+  err_reduce(a, c);
+  if (threadIdx.x == 0) out[blockIdx.x] = c > 0.0 ? sqrt(a / c) : INFINITY;
 }
 
 // Reinhard tone map (ReinhardToneMap::map, M/renderers/tonemaps/ReinhardToneMap.cpp:25-94) of the
@@ -261,16 +282,73 @@ __global__ void k_tonemap_map(ToneSrc t, const double2 *partial, uchar4 *out) {
   }
 }
 
-// per-thread device scratch of the error estimate (grown as needed, per device)
-struct ErrScratch {
+// Scratch of the film reads of one host thread, kept for its next read and released when the thread exits: a
+// device buffer and a page-locked host buffer, each grown to the largest need.  A film read is
+// synchronous, so the thread's next one finds them free.
+struct ReadScratch {
+  void *d = nullptr, *h = nullptr;
+  size_t d_bytes = 0, h_bytes = 0;
   int device = -1;
-  size_t bytes = 0;
-  void *d = nullptr;
-  ~ErrScratch() {
-    if (d) cudaFree(d);
+  void release_device() {
+    if (!d) return;
+    int cur = 0;
+    cudaGetDevice(&cur);
+    if (cur != device) cudaSetDevice(device);
+    cudaFree(d);
+    if (cur != device) cudaSetDevice(cur);
+    d = nullptr;
+    d_bytes = 0;
+  }
+  cudaError_t device_buffer(size_t need, void **out) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (d && (dev != device || need > d_bytes)) release_device();
+    if (!d) {
+      if ((e = cudaMalloc(&d, need)) != cudaSuccess) {
+        d = nullptr;
+        return e;
+      }
+      d_bytes = need;
+      device = dev;
+    }
+    *out = d;
+    return cudaSuccess;
+  }
+  // portable and mapped: a kernel of any device writes there
+  cudaError_t host_buffer(size_t need, void **out) {
+    if (h && need > h_bytes) {
+      cudaFreeHost(h);
+      h = nullptr;
+      h_bytes = 0;
+    }
+    if (!h) {
+      const cudaError_t e = cudaHostAlloc(&h, need, cudaHostAllocPortable | cudaHostAllocMapped);
+      if (e != cudaSuccess) {
+        h = nullptr;
+        return e;
+      }
+      h_bytes = need;
+    }
+    *out = h;
+    return cudaSuccess;
+  }
+  ~ReadScratch() {
+    release_device();
+    if (h) cudaFreeHost(h);
   }
 };
-static thread_local ErrScratch t_err;
+static thread_local ReadScratch t_read;
+
+// the device's view of a page-locked host buffer, or nullptr for pageable memory
+static void *device_view(const void *p) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+}
 
 }  // namespace mgpu
 
@@ -641,87 +719,92 @@ int mgpu_film_read_raw(mgpu_film *f, float *out8, void *stream) {
   return MGPU_OK;
 }
 
-// mean = (sum - compensation) / count in FP64 (ProgressiveFilterValue::getValue,
-// ProgressiveFilterValue.h:26-31; a pixel with no samples reads as black)
-// Device scratch and page-locked host staging of the film reads of one host thread: grown to the
-// largest read and kept for the next, released when the thread exits.  A film read is
-// synchronous, so the thread's next read finds them free.
-struct MeanScratch {
-  void *p = nullptr, *h = nullptr;  // device buffer, page-locked host staging of the same size
-  size_t bytes = 0;
-  int device = -1;
-  void release() {
-    if (p) cudaFree(p);
-    if (h) cudaFreeHost(h);
-    p = h = nullptr;
-    bytes = 0;
-  }
-  cudaError_t get(int dev, size_t need, void **out, void **host) {
-    if (p && (dev != device || need > bytes)) release();
-    if (!p) {
-      cudaError_t e = cudaMalloc(&p, need);
-      if (e == cudaSuccess) e = cudaMallocHost(&h, need);
-      if (e != cudaSuccess) {
-        release();
-        return e;
-      }
-      bytes = need;
-      device = dev;
-    }
-    *out = p;
-    *host = h;
-    return cudaSuccess;
-  }
-  ~MeanScratch() { release(); }
-};
-static thread_local MeanScratch t_mean_scratch;
-
-// Per pixel mean of the compensated film: (sum - compensation) / count in FP64, 0 for a pixel
-// without samples.
+// The film's output in FP64 for pixels first .. first + count - 1, written by the kernel where the host reads
+// it (page-locked memory): the per-pixel mean (sum - compensation) / count (ProgressiveFilterValue::
+// getValue, ProgressiveFilterValue.h:26-31; 0 for a pixel without samples), or with a reconstruction
+// filter sum(w L) / sum(w).  256 pixels at a time go through shared memory so that the stores to
+// the host are whole lines.
 __global__ void __launch_bounds__(256) k_film_mean(const float4 *__restrict__ sum, const float4 *__restrict__ comp,
-                                                   int64_t npix, double *__restrict__ out) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < npix; i += (int64_t)gridDim.x * blockDim.x) {
-    const float4 s = sum[i], c = comp[i];
-    const double cnt = s.w;
-    double r = 0.0, g = 0.0, b = 0.0;
-    if (cnt > 0) {
-      r = ((double)s.x - (double)c.x) / cnt;
-      g = ((double)s.y - (double)c.y) / cnt;
-      b = ((double)s.z - (double)c.z) / cnt;
+                                                   const unsigned long long *__restrict__ fx, int64_t first,
+                                                   int64_t count, double *__restrict__ out) {
+  __shared__ double rgb[768];
+  for (int64_t base = (int64_t)blockIdx.x * 256; base < count; base += (int64_t)gridDim.x * 256) {
+    const int64_t i = base + threadIdx.x;
+    if (i < count) {
+      double r = 0.0, g = 0.0, b = 0.0;
+      if (fx) {
+        const unsigned long long *q = fx + 4 * (first + i);
+        const double w = (double)q[3];
+        if (w > 0) {
+          r = (double)q[0] / w;
+          g = (double)q[1] / w;
+          b = (double)q[2] / w;
+        }
+      } else {
+        const float4 s = sum[first + i], c = comp[first + i];
+        const double cnt = s.w;
+        if (cnt > 0) {
+          r = ((double)s.x - (double)c.x) / cnt;
+          g = ((double)s.y - (double)c.y) / cnt;
+          b = ((double)s.z - (double)c.z) / cnt;
+        }
+      }
+      rgb[3 * threadIdx.x] = r;
+      rgb[3 * threadIdx.x + 1] = g;
+      rgb[3 * threadIdx.x + 2] = b;
     }
-    out[3 * i + 0] = r;
-    out[3 * i + 1] = g;
-    out[3 * i + 2] = b;
+    __syncthreads();
+    const int64_t n = 3 * (count - base < 256 ? count - base : 256);
+    for (int k = (int)threadIdx.x; k < n; k += 256) out[3 * base + k] = rgb[k];
+    __syncthreads();
   }
 }
 
 int mgpu_film_read(mgpu_film *f, double *out_mean, void *stream) {
   if (!f || !out_mean) return fail(MGPU_E_INVALID, "mgpu_film_read: null argument");
-  size_t n = (size_t)f->width * f->height;
-  if (f->d_fx) {
-    // reconstruction filter: per pixel sum(w L) / sum(w) (ProgressiveFilterValue, weights > 0)
-    std::vector<unsigned long long> fx(4 * n);
-    cudaStream_t st = as_stream(stream);
-    MGPU_CUDA(cudaMemcpyAsync(fx.data(), f->d_fx, fx.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+  const int64_t n = (int64_t)f->width * f->height;
+  cudaStream_t st = as_stream(stream);
+  auto launch = [&](int64_t first, int64_t count, double *dst) {
+    const unsigned grid = (unsigned)std::min<int64_t>((count + 255) / 256, (int64_t)device_sm_count() * 8);
+    k_film_mean<<<grid, 256, 0, st>>>(f->d_sum, f->d_c, f->d_fx, first, count, dst);
+    g_launches.fetch_add(1);
+    return cudaGetLastError();
+  };
+  // into the caller's array where the device can write it
+  if (double *dst = (double *)device_view(out_mean)) {
+    MGPU_CUDA(launch(0, n, dst));
     MGPU_CUDA(cudaStreamSynchronize(st));
-    for (size_t i = 0; i < n; ++i) {
-      const double w = (double)fx[4 * i + 3];
-      for (int k = 0; k < 3; ++k) out_mean[3 * i + k] = w > 0 ? (double)fx[4 * i + k] / w : 0.0;
-    }
     return MGPU_OK;
   }
-  // the FP64 means are taken on the device; only they cross to the host, through page-locked
-  // staging, and are copied from there into the caller's array
-  cudaStream_t st = as_stream(stream);
-  const size_t bytes = 3 * n * sizeof(double);
-  double *d_mean = nullptr, *h_mean = nullptr;
-  MGPU_CUDA(t_mean_scratch.get(f->device, bytes, (void **)&d_mean, (void **)&h_mean));
-  k_film_mean<<<device_sm_count() * 4, 256, 0, st>>>(f->d_sum, f->d_c, (int64_t)n, d_mean);
-  g_launches.fetch_add(1);
-  MGPU_CUDA(cudaGetLastError());
-  MGPU_CUDA(cudaMemcpyAsync(h_mean, d_mean, bytes, cudaMemcpyDeviceToHost, st));
-  MGPU_CUDA(cudaStreamSynchronize(st));
-  memcpy(out_mean, h_mean, bytes);
+  // pageable: through two page-locked pieces, the host copying one while the device writes the other
+  constexpr int64_t kPiece = 1 << 18;  // pixels
+  constexpr int64_t piece = kPiece;
+  double *h = nullptr;
+  if (n <= kPiece) {
+    MGPU_CUDA(t_read.host_buffer((size_t)n * 3 * sizeof(double), (void **)&h));
+    MGPU_CUDA(launch(0, n, h));
+    MGPU_CUDA(cudaStreamSynchronize(st));
+    memcpy(out_mean, h, (size_t)n * 3 * sizeof(double));
+    return MGPU_OK;
+  }
+  MGPU_CUDA(t_read.host_buffer((size_t)2 * piece * 3 * sizeof(double), (void **)&h));
+  cudaEvent_t done[2] = {nullptr, nullptr};
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < 2 && e == cudaSuccess; ++k) e = cudaEventCreateWithFlags(&done[k], cudaEventDisableTiming);
+  for (int64_t k = 0; k * piece < n + piece && e == cudaSuccess; ++k) {
+    if (k * piece < n) {
+      e = launch(k * piece, std::min(piece, n - k * piece), h + (k & 1) * 3 * piece);
+      if (e == cudaSuccess) e = cudaEventRecord(done[k & 1], st);
+    }
+    if (k > 0 && e == cudaSuccess) {
+      const int64_t q = k - 1, cnt = std::min(piece, n - q * piece);
+      e = cudaEventSynchronize(done[q & 1]);
+      if (e == cudaSuccess) memcpy(out_mean + 3 * q * piece, h + (q & 1) * 3 * piece, (size_t)cnt * 3 * sizeof(double));
+    }
+  }
+  for (int k = 0; k < 2; ++k)
+    if (done[k]) cudaEventDestroy(done[k]);
+  if (e != cudaSuccess) return cuda_fail(e, "mgpu_film_read");
   return MGPU_OK;
 }
 
@@ -729,20 +812,20 @@ int mgpu_film_tonemap(mgpu_film *f, uint8_t *out_rgba, void *stream) {
   if (!f || !out_rgba) return fail(MGPU_E_INVALID, "mgpu_film_tonemap: null argument");
   const int64_t npix = (int64_t)f->width * f->height;
   ToneSrc ref{FilmRef{f->d_sum, f->d_c, npix}, f->d_fx};
-  void *d = nullptr;
-  const size_t b_part = align_up(kErrBlocks * sizeof(double2), 256);
-  MGPU_CUDA(cudaMalloc(&d, b_part + (size_t)npix * sizeof(uchar4)));
-  double2 *part = (double2 *)d;
-  uchar4 *img = (uchar4 *)((char *)d + b_part);
+  double2 *part = nullptr;
+  uchar4 *img = nullptr;
+  MGPU_CUDA(t_read.device_buffer(kErrBlocks * sizeof(double2), (void **)&part));
+  const size_t bytes = (size_t)npix * sizeof(uchar4);
+  void *dst = device_view(out_rgba);
+  if ((uintptr_t)dst & 3) dst = nullptr;
+  if (!dst) MGPU_CUDA(t_read.host_buffer(bytes, (void **)&img));
   cudaStream_t st = as_stream(stream);
   k_tonemap_reduce<<<kErrBlocks, kErrThreads, 0, st>>>(ref, part);
-  k_tonemap_map<<<device_sm_count() * 4, 256, 0, st>>>(ref, part, img);
+  k_tonemap_map<<<device_sm_count() * 4, 256, 0, st>>>(ref, part, dst ? (uchar4 *)dst : img);
   g_launches.fetch_add(2);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(out_rgba, img, (size_t)npix * sizeof(uchar4), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFree(d);
-  if (e != cudaSuccess) return cuda_fail(e, "mgpu_film_tonemap");
+  MGPU_CUDA(cudaGetLastError());
+  MGPU_CUDA(cudaStreamSynchronize(st));
+  if (!dst) memcpy(out_rgba, img, bytes);
   return MGPU_OK;
 }
 
@@ -750,43 +833,41 @@ int mgpu_film_error(mgpu_film *const *films, int32_t n, double *out_rmse, void *
   if (n < 0 || n > 65535 || (n > 0 && (!films || !out_rmse)))
     return fail(MGPU_E_INVALID, "mgpu_film_error: bad argument");
   if (n == 0) return MGPU_OK;
-  std::vector<FilmRef> refs((size_t)n);
+  // the films' records and their estimates in page-locked memory that the kernels read and write
+  const size_t b_refs = align_up((size_t)n * sizeof(FilmRef), 256);
+  char *h = nullptr;
+  MGPU_CUDA(t_read.host_buffer(b_refs + (size_t)n * sizeof(double), (void **)&h));
+  FilmRef *refs = (FilmRef *)h;
+  double *est = (double *)(h + b_refs);
+  int blocks = kErrBlocks;
   for (int32_t i = 0; i < n; ++i) {
     if (!films[i]) return fail(MGPU_E_INVALID, "mgpu_film_error: null film");
     refs[i].sum = films[i]->d_sum;
     refs[i].c = films[i]->d_c;
     refs[i].npix = (int64_t)films[i]->width * films[i]->height;
+    blocks = std::max(blocks, err_blocks(refs[i].npix));
   }
-  const size_t b_refs = align_up((size_t)n * sizeof(FilmRef), 256);
-  const size_t b_part = align_up((size_t)n * kErrBlocks * sizeof(double2), 256);
-  const size_t need = b_refs + b_part + (size_t)n * sizeof(double);
-  int dev = 0;
-  MGPU_CUDA(cudaGetDevice(&dev));
-  if (t_err.device != dev || t_err.bytes < need) {
-    if (t_err.d) {
-      int cur = dev;
-      if (t_err.device != dev) cudaSetDevice(t_err.device);
-      cudaFree(t_err.d);
-      if (t_err.device != dev) cudaSetDevice(cur);
-      t_err.d = nullptr;
-    }
-    t_err.bytes = 0;
-    MGPU_CUDA(cudaMalloc(&t_err.d, need));
-    t_err.device = dev;
-    t_err.bytes = need;
-  }
-  char *base = (char *)t_err.d;
-  FilmRef *d_refs = (FilmRef *)base;
-  double2 *d_part = (double2 *)(base + b_refs);
-  double *d_out = (double *)(base + b_refs + b_part);
+  double2 *part = nullptr;
+  MGPU_CUDA(t_read.device_buffer((size_t)n * blocks * sizeof(double2), (void **)&part));
   cudaStream_t st = as_stream(stream);
-  MGPU_CUDA(cudaMemcpyAsync(d_refs, refs.data(), (size_t)n * sizeof(FilmRef), cudaMemcpyHostToDevice, st));
-  k_film_error_partial<<<dim3(kErrBlocks, n), kErrThreads, 0, st>>>(d_refs, d_part);
-  k_film_error_final<<<(n + 127) / 128, 128, 0, st>>>(d_part, n, d_out);
+  k_film_error_partial<<<dim3(blocks, n), kErrThreads, 0, st>>>(refs, part);
+  k_film_error_final<<<n, kErrThreads, 0, st>>>(refs, part, blocks, est);
   g_launches.fetch_add(2);
   MGPU_CUDA(cudaGetLastError());
-  MGPU_CUDA(cudaMemcpyAsync(out_rmse, d_out, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, st));
   MGPU_CUDA(cudaStreamSynchronize(st));
+  memcpy(out_rmse, est, (size_t)n * sizeof(double));
+  return MGPU_OK;
+}
+
+// Page-locked host memory that every device can write (results are then read without a staging copy).
+int mgpu_host_alloc(uint64_t bytes, void **out) {
+  if (!out || bytes == 0) return fail(MGPU_E_INVALID, "mgpu_host_alloc: bad argument");
+  MGPU_CUDA(cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable | cudaHostAllocMapped));
+  return MGPU_OK;
+}
+
+int mgpu_host_free(void *p) {
+  if (p) MGPU_CUDA(cudaFreeHost(p));
   return MGPU_OK;
 }
 

@@ -17,6 +17,7 @@ from dataclasses import dataclass, field
 import numpy as np
 
 from . import _native as N
+from . import hostmem
 from .scene import Scene
 
 
@@ -178,12 +179,12 @@ class Film:
     filter = ("none", 0.0, {})
 
     def mean(self, stream=None) -> np.ndarray:
-        out = np.zeros((self.height, self.width, 3), np.float64)
+        out = hostmem.empty((self.height, self.width, 3), np.float64)
         N.check(self._lib.mgpu_film_read(self.handle, N.ptr(out), _stream_handle(stream)))
         return out
 
     def raw(self, stream=None) -> np.ndarray:
-        out = np.zeros((2, self.height, self.width, 4), np.float32)
+        out = hostmem.empty((2, self.height, self.width, 4), np.float32)
         N.check(self._lib.mgpu_film_read_raw(self.handle, N.ptr(out), _stream_handle(stream)))
         return out
 
@@ -207,7 +208,7 @@ class Film:
 
     def tonemap(self, stream=None) -> np.ndarray:
         """mgpu_film_tonemap: Milton's Reinhard tone map of the per-pixel means, (H, W, 4) uint8."""
-        out = np.zeros((self.height, self.width, 4), np.uint8)
+        out = hostmem.empty((self.height, self.width, 4), np.uint8)
         N.check(self._lib.mgpu_film_tonemap(self.handle, N.ptr(out), _stream_handle(stream)))
         return out
 

@@ -1,0 +1,64 @@
+"""Film reads into page-locked and pageable arrays, at the sizes where the pieces end, and the pool of
+page-locked result arrays."""
+import ctypes as C
+import gc
+
+import numpy as np
+import pytest
+
+from milton_gb300 import _native as N
+from milton_gb300 import hostmem
+from milton_gb300 import pathtracer as pt
+from milton_gb300 import scenegen
+
+pytestmark = pytest.mark.gpu
+
+
+# 65,536 x 4 = one piece exactly, + 4 one more, 2 pieces and a remainder, one pixel, a tile of 256 and more
+@pytest.mark.parametrize("w,h", [(1, 1), (16, 16), (257, 1), (512, 512), (65537, 4), (1025, 770)])
+@pytest.mark.parametrize("kind", ["none", "mitchell"])
+def test_mean_is_the_same_in_any_memory(cuda, w, h, kind):
+    s = scenegen.plain(0)
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    f = pt.Film(w, h)
+    if kind != "none":
+        f.set_filter(kind, 3.0)
+    pt.render(ds, pt.RenderSettings(w, h, 2, max_depth=2, rr_start_depth=3, seed=3), f)
+    pinned = f.mean()
+    pageable = np.full((h, w, 3), np.nan)
+    N.check(N.load().mgpu_film_read(f.handle, N.ptr(pageable), None))
+    assert np.array_equal(pinned, pageable)
+    if kind == "none":
+        raw = f.raw().astype(np.float64)
+        n = raw[0, ..., 3:4]
+        assert np.array_equal(pageable, (raw[0, ..., :3] - raw[1, ..., :3]) / n)
+        # the estimate of the kernel against the same formula on the host (FP64 sums in another order)
+        assert pt.film_error([f])[0] == pytest.approx(pt.rmse_estimate(f.raw()), rel=1e-9, abs=1e-15)
+    rgba = np.zeros((h, w, 4), np.uint8)
+    N.check(N.load().mgpu_film_tonemap(f.handle, N.ptr(rgba), None))
+    assert np.array_equal(rgba, f.tonemap())
+
+
+def test_pool_gives_blocks_back_and_stays_bounded(cuda):
+    before = hostmem._total
+    a = hostmem.empty((1 << 17,), np.float64)
+    a[:] = 1.0
+    view = a[5:10]
+    addr = a.ctypes.data
+    del a
+    gc.collect()
+    b = hostmem.empty((1 << 17,), np.float64)  # the view still holds the first block
+    assert b.ctypes.data != addr and np.all(view == 1.0)
+    del view
+    gc.collect()
+    c = hostmem.empty((1 << 17,), np.float64)
+    assert c.ctypes.data == addr
+    del b, c
+    gc.collect()
+    keep = [hostmem.empty((48 << 20,), np.uint8) for _ in range(8)]  # beyond the limit: ordinary arrays
+    assert hostmem._total <= hostmem.LIMIT and all(k.nbytes == 48 << 20 for k in keep)
+    del keep
+    gc.collect()
+    assert hostmem._total <= max(before, hostmem.LIMIT)
+    p = C.c_void_p()
+    assert N.load().mgpu_host_alloc(0, C.byref(p)) != N.MGPU_OK
