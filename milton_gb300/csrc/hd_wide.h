@@ -190,11 +190,11 @@ __device__ __forceinline__ float wide_unorder(uint32_t u) {
 // side of it in the kd-tree.
 constexpr float kWideTie = 1.0f / 131072.0f;
 
-// The kd-tree's answer for one ray: closest hit, or any (h.prim >= 0).  SEQ: a leaf's triangles one after
+// The kd-tree's answer for one ray: closest hit, or any (h.prim >= 0).  seq: a leaf's triangles one after
 // another, each against the t before it; otherwise the smallest (t, leaf order) among those accepted
 // against the t before the leaf.
-template <bool ANY, bool SPH, bool SEQ>
-__device__ __noinline__ void kd_ray(const SceneView &s, const Ray &r, Hit &h) {
+template <bool ANY, bool SPH>
+__device__ __noinline__ void kd_ray(const SceneView &s, const Ray &r, bool seq, Hit &h) {
   TravState st;
   TravEntry stack[kMaxStack];
   if (trav_init<SPH>(s, r, nullptr, 0, st, ANY)) {
@@ -210,8 +210,8 @@ __device__ __noinline__ void kd_ray(const SceneView &s, const Ray &r, Hit &h) {
         const F4 a = load_f4(s.ltris, q), b = load_f4(s.ltris, q + 1), c = load_f4(s.ltris, q + 2);
         float t, b1, b2;
         if (intersect_tri(st.pre, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), (f_bits(b.w) & 1u) != 0u,
-                          st.ray_tmin, SEQ ? st.best : best0, t, b1, b2) &&
-            (SEQ || !took || t < st.best)) {
+                          st.ray_tmin, seq ? st.best : best0, t, b1, b2) &&
+            (seq || !took || t < st.best)) {
           took = true;
           st.best = t; st.best_prim = (int32_t)f_bits(a.w); st.bb1 = b1; st.bb2 = b2;
         }
@@ -237,11 +237,11 @@ __device__ __noinline__ void kd_ray(const SceneView &s, const Ray &r, Hit &h) {
 // queries): kd-tree 187.7 ms of traversal, nodes of 80 bytes with per-node slack and child order by mask
 // permutation 95.0, the node step as it is now 83.7.
 //   ANY     occlusion: the first hit ends the ray; otherwise the closest
-//   SEQ     which of the kd-tree's orders decides near ties (kd_ray)
+//   seq     which of the kd-tree's orders decides near ties (kd_ray)
 //   SINGLE  every ray is in the scene view(0), which the kernel passes from its parameter space
 //   TZERO   every ray starts at t = 0
 // All 32 lanes call round(), the other members are per lane or say so.
-template <bool ANY, bool SEQ, bool COUNT, bool SPH, bool SINGLE, bool TZERO, class View, class Load, class Store>
+template <bool ANY, bool COUNT, bool SPH, bool SINGLE, bool TZERO, class View, class Load, class Store>
 struct WideWarp {
   static constexpr unsigned kFull = 0xFFFFFFFFu;
   View view;
@@ -251,6 +251,7 @@ struct WideWarp {
   const WideTables &tab;
   TraceCounts *cnt;
   const uint32_t lane;
+  const bool seq;
   uint2 *stack;
   WideRay w{};
   WideGroup ng{0u, 0u}, tg{0u, 0u};
@@ -405,7 +406,7 @@ struct WideWarp {
       Ray r;
       load(i, r);
       if (kd) {
-        kd_ray<ANY, SPH, SEQ>(s, r, h);
+        kd_ray<ANY, SPH>(s, r, seq, h);
       } else {
         // the winner again, for its barycentrics: the same inputs, the same result
         const int64_t q = 3 * (int64_t)rec;
@@ -436,26 +437,30 @@ struct WideChunks {
   }
 };
 
-// Rays 0 .. n - 1, a warp's 32 to completion (next: a counter of the block, zero at the start).  For rays that
+// All of them, by one block.
+struct WideAll {
+  __device__ __forceinline__ unsigned long long ray(uint32_t pos) const { return pos; }
+};
+
+// Rays 0 .. n - 1 (those that `rays` gives the block), a warp's 32 to completion (next: a counter of the block, zero at the start).  For rays that
 // lie in a queue with their neighbours: a lane that ends early waits, which costs less than what the other
 // shape (below) adds to the node loop's registers (mid frame 83.7 against 92 ms).
 // All 32 lanes of every warp must call this.
-template <bool ANY, bool SEQ, bool COUNT, bool SPH, bool SINGLE, bool TZERO, class View, class Load, class Store>
-__device__ __forceinline__ void wide_trace(View view, uint32_t n, Load load, Store store, WideShared &sh,
-                                           const WideTables &tab, uint32_t *next, TraceCounts *cnt,
+template <bool ANY, bool COUNT, bool SPH, bool SINGLE, bool TZERO, class Rays, class View, class Load, class Store>
+__device__ __forceinline__ void wide_trace(const Rays &rays, View view, uint32_t n, Load load, Store store, bool seq,
+                                           WideShared &sh, const WideTables &tab, uint32_t *next, TraceCounts *cnt,
                                            uint32_t &rays_done) {
   constexpr unsigned kFull = 0xFFFFFFFFu;
   uint2 stack[kWideMaxDepth];
-  const WideChunks chunks(n);
   const uint32_t lane = threadIdx.x & 31u;
   for (;;) {
     uint32_t pos = 0u;
     if (lane == 0u) pos = atomicAdd(next, 32u);
-    const unsigned long long first = chunks.ray(__shfl_sync(kFull, pos, 0));
+    const unsigned long long first = rays.ray(__shfl_sync(kFull, pos, 0));
     if (first >= n) break;
     const uint32_t i = (uint32_t)first + lane;
     __syncwarp(kFull);  // the previous rays' readers are done with the shared records
-    WideWarp<ANY, SEQ, COUNT, SPH, SINGLE, TZERO, View, Load, Store> t{view, load, store, sh, tab, cnt, lane, stack};
+    WideWarp<ANY, COUNT, SPH, SINGLE, TZERO, View, Load, Store> t{view, load, store, sh, tab, cnt, lane, seq, stack};
     if (i < n) {
       t.start(i);
       ++rays_done;
@@ -480,13 +485,13 @@ __device__ __forceinline__ void wide_trace(View view, uint32_t n, Load load, Sto
 // All 32 lanes of every warp must call this.
 constexpr uint32_t kWideRefill = 16u;
 
-template <bool ANY, bool SEQ, bool SPH, class View, class Load, class Store>
-__device__ __forceinline__ void wide_trace_refill(View view, uint32_t n, Load load, Store store, WideShared &sh,
+template <bool ANY, bool SPH, class View, class Load, class Store>
+__device__ __forceinline__ void wide_trace_refill(View view, uint32_t n, Load load, Store store, bool seq, WideShared &sh,
                                                   const WideTables &tab, uint32_t *next) {
   constexpr unsigned kFull = 0xFFFFFFFFu;
   uint2 stack[kWideMaxDepth];
   const WideChunks chunks(n);
-  WideWarp<ANY, SEQ, false, SPH, true, false, View, Load, Store> t{view, load, store, sh, tab, nullptr, threadIdx.x & 31u, stack};
+  WideWarp<ANY, false, SPH, true, false, View, Load, Store> t{view, load, store, sh, tab, nullptr, threadIdx.x & 31u, seq, stack};
   uint32_t i = 0u;
   bool have = false;  // the lane holds ray i
   bool more = true;   // the block has rays left (uniform over the warp)

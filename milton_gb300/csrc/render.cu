@@ -94,6 +94,7 @@ struct RenderArgs {
   unsigned long long *stats;     // [0] extension rays, [1] shadow rays, [2] truncated paths, [3] bounces
   unsigned long long *tcount;    // counted mode: ext nodes, refs, tris, rays; shadow nodes, refs, tris, rays
   int32_t max_b;
+  int32_t seq;                   // near ties are decided as the one-ray-per-lane kd-tree kernels do
   SceneView view0;               // the scene of a wave of one scene (njobs == 1)
 };
 
@@ -327,8 +328,8 @@ __global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMi
     };
     WideBlockShared &ws = wide_shared();
     WideShared &sh = ws.warp[threadIdx.x >> 5];
-    if (single) wide_trace<false, SPH, COUNT, SPH, true, true>(view0, n, load, store, sh, ws.tables, &ws.next, &c, rays);
-    else wide_trace<false, SPH, COUNT, SPH, false, true>(view_of, n, load, store, sh, ws.tables, &ws.next, &c, rays);
+    if (single) wide_trace<false, COUNT, SPH, true, true>(WideChunks(n), view0, n, load, store, SPH, sh, ws.tables, &ws.next, &c, rays);
+    else wide_trace<false, COUNT, SPH, false, true>(WideChunks(n), view_of, n, load, store, SPH, sh, ws.tables, &ws.next, &c, rays);
   } else {
     auto store = [&](uint32_t i, bool hit, const TravState &st) {
       qhit[i] = make_float4(hit ? st.best : INFINITY, __int_as_float(hit ? st.best_prim : -1), hit ? st.bb1 : 0.0f,
@@ -360,11 +361,19 @@ __device__ __forceinline__ V3 fold_slots(const RenderArgs &a, int nl, int64_t p,
 constexpr int kShadeTile = 256;
 constexpr int kShadeMinBlocks = 4;
 
-// What a shading block keeps in shared memory: per warp the shadow rays that wait for a full 32, and the
-// counts and the order of the tile's rays.
+// What a shading block keeps in shared memory: per warp the shadow rays that wait for a full 32 (or, while
+// the block traces its own rays, the traversal's records), the counts and the order of the tile's
+// rays, and the block's own queue counts.
 struct ShadeShared {
-  float4 so[kShadeTile / 32][64], sd[kShadeTile / 32][64];
+  union {
+    struct {
+      float4 so[kShadeTile / 32][64], sd[kShadeTile / 32][64];
+    } stage;
+    WideShared wide[kShadeTile / 32];
+  };
+  WideTables tables;
   uint32_t cnt[kShadeTile / 4];
+  uint32_t next, rays, shadow;
   uint8_t perm[kShadeTile];
 };
 
@@ -432,17 +441,92 @@ struct ShadowStage {
   }
 };
 
+// One block's closest hits of rays base .. n - 1 of bounce b, and its shadow rays (whole paths, k_shade).
+template <bool SPH>
+__device__ __noinline__ void block_extend(const RenderArgs &a, ShadeShared &sh, int b, uint32_t base, uint32_t n) {
+  const float4 *qo = a.qo[b & 1] + base, *qd = a.qd[b & 1] + base;
+  uint32_t done = 0u;
+  wide_trace<false, false, SPH, false, true>(
+      WideAll(), [&](uint32_t i) -> const SceneView & { return a.jobs[__float_as_int(qd[i].w)].view; }, n - base,
+      [&](uint32_t i, Ray &r) {
+        const float4 o = qo[i], d = qd[i];
+        r.o = v3(o.x, o.y, o.z);
+        r.tmin = 0.0f;
+        r.d = v3(d.x, d.y, d.z);
+        r.tmax = INFINITY;
+      },
+      [&](uint32_t i, bool hit, const Hit &h) {
+        a.qhit[base + i] = make_float4(hit ? h.t : INFINITY, __int_as_float(hit ? h.prim : -1), hit ? h.b1 : 0.0f,
+                                       hit ? h.b2 : 0.0f);
+      },
+      a.seq != 0, sh.wide[threadIdx.x >> 5], sh.tables, &sh.next, nullptr, done);
+}
+
+template <bool SPH>
+__device__ __noinline__ void block_shadow(const RenderArgs &a, ShadeShared &sh, const float4 *so, const float4 *sd,
+                                          uint32_t n) {
+  uint32_t done = 0u;
+  wide_trace<true, false, SPH, false, true>(
+      WideAll(),
+      [&](uint32_t i) -> const SceneView & {
+        return a.jobs[a.path_job[__float_as_uint(so[i].w) / (uint32_t)a.nl_stride]].view;
+      },
+      n,
+      [&](uint32_t i, Ray &r) {
+        const float4 o = so[i], d = sd[i];
+        r.o = v3(o.x, o.y, o.z);
+        r.tmin = 0.0f;
+        r.d = v3(d.x, d.y, d.z);
+        r.tmax = d.w;
+      },
+      [&](uint32_t i, bool hit, const Hit &) {
+        if (hit) a.slots[__float_as_uint(so[i].w)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      },
+      a.seq != 0, sh.wide[threadIdx.x >> 5], sh.tables, &sh.next, nullptr, done);
+}
+
 // SURF: the wave has a scene with image maps, a background or analytic spheres.  Scenes without
 // them run the variant that has none of those branches, whose register allocation (and spilling)
 // is the lighter.
+//
+// whole: the launch takes whole paths instead of one bounce (waves of few paths).  Every block owns `whole` (at
+// most 256) rays of bounce b and runs their bounces to the end: it traces its rays, shades them, traces
+// their shadow rays, and keeps the queues in its own part of the arrays.  One launch instead of three per
+// bounce, and blocks whose paths have ended do not wait for others.  It is this kernel and not one of
+// its own so that the shading is the same machine code: compiled twice, its multiply-adds contract
+// differently and an image would depend on the wave size.
 template <bool SURF>
-__global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(RenderArgs a, int b) {
-  __shared__ ShadeShared sh;
-  const uint32_t n = a.counters[kCtrRay + b];
-  const int cur = b & 1, nxt = (b + 1) & 1;
-  const uint32_t stride = gridDim.x * kShadeTile;
-  ShadowStage stage{sh.so[threadIdx.x >> 5], sh.sd[threadIdx.x >> 5], &a.counters[kCtrNee + b], a.so, a.sd, 0u, 0u};
-  for (uint32_t base = blockIdx.x * kShadeTile; base < n; base += stride) {
+__global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(const __grid_constant__ RenderArgs a, int b,
+                                                                       uint32_t whole) {
+  extern __shared__ __align__(16) unsigned char shade_smem[];
+  ShadeShared &sh = *reinterpret_cast<ShadeShared *>(shade_smem);
+  uint32_t n = a.counters[kCtrRay + b], base = blockIdx.x * kShadeTile;
+  const uint32_t stride = gridDim.x * kShadeTile, total = n;
+  const int b0 = b;
+  const uint32_t warp = threadIdx.x >> 5;
+  uint32_t out = 0u;  // first entry of the queues that the block writes
+  uint32_t *next_ctr = &a.counters[kCtrRay + b + 1];
+  ShadowStage stage{sh.stage.so[warp], sh.stage.sd[warp], &a.counters[kCtrNee + b], a.so, a.sd, 0u, 0u};
+  if (whole) {
+    base = blockIdx.x * whole;
+    if (base >= total) return;
+    wide_tables(sh.tables);
+    out = base;
+    n = min(base + whole, total);
+    next_ctr = &sh.rays;
+    stage.counter = &sh.shadow;
+    stage.so = a.so + (size_t)base * a.nl_stride;
+    stage.sd = a.sd + (size_t)base * a.nl_stride;
+  }
+  for (;;) {
+    if (base >= n) break;
+    const int cur = b & 1, nxt = (b + 1) & 1;
+    if (whole) {
+      if (threadIdx.x == 0) sh.next = sh.rays = sh.shadow = 0u;
+      __syncthreads();
+      block_extend<SURF>(a, sh, b, base, n);
+      __syncthreads();
+    }
     // the tile's rays in the order of what they hit: with the BSDFs of a tile side by side a warp runs one of
     // them, and the barriers keep the block's warps in the same part of a kernel that exceeds the
     // instruction cache (ncu, mid scene, second bounce: lanes per instruction 13.7 -> 24.9, warps waiting
@@ -556,7 +640,7 @@ __global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(RenderArg
       a.path_L[p] = make_float4(L.x, L.y, L.z, __uint_as_float(flags));
     }
     const JobArgs &J = a.jobs[j];
-    const uint32_t q = warp_append(&a.counters[kCtrRay + b + 1], want_next);
+    const uint32_t q = out + warp_append(next_ctr, want_next);
     if (want_next) {
       if (a.bin_ext) {
         a.qo_u[q] = no_o;
@@ -637,8 +721,27 @@ __global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(RenderArg
       }
       stage.append(want, so4, sd4);
     }
+    if (!whole) {
+      base += stride;
+      continue;
+    }
+    stage.flush();
+    __syncthreads();
+    const uint32_t nshadow = sh.shadow, nrays = sh.rays;
+    __syncthreads();
+    if (threadIdx.x == 0) sh.next = 0u;
+    __syncthreads();
+    block_shadow<SURF>(a, sh, stage.so, stage.sd, nshadow);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      if (b > b0) atomicAdd(&a.counters[kCtrRay + b], n - base);
+      atomicAdd(&a.counters[kCtrNee + b], nshadow);
+    }
+    n = base + nrays;
+    ++b;
+    if (b >= a.max_b) n = base;
   }
-  stage.flush();
+  if (!whole) stage.flush();
 }
 
 
@@ -670,8 +773,8 @@ __global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMi
   if constexpr (WIDE) {
     WideBlockShared &ws = wide_shared();
     WideShared &sh = ws.warp[threadIdx.x >> 5];
-    if (single) wide_trace<true, SPH, COUNT, SPH, true, true>(view0, n, load, store, sh, ws.tables, &ws.next, &c, rays);
-    else wide_trace<true, SPH, COUNT, SPH, false, true>(view_of, n, load, store, sh, ws.tables, &ws.next, &c, rays);
+    if (single) wide_trace<true, COUNT, SPH, true, true>(WideChunks(n), view0, n, load, store, SPH, sh, ws.tables, &ws.next, &c, rays);
+    else wide_trace<true, COUNT, SPH, false, true>(WideChunks(n), view_of, n, load, store, SPH, sh, ws.tables, &ws.next, &c, rays);
   } else {
     grid_trace<true, COUNT, SPH>(view_of, nullptr, 0, n, load, store, &c, rays);
   }
@@ -866,6 +969,9 @@ constexpr int kCarveoutAuto = -2;
 struct Tuning {
   // the 8-wide hierarchy where every scene of a render has one; 0: the kd-tree
   std::atomic<int> wide{1};
+  // waves of at most this many paths run whole paths in one launch (0: none do; -1: three quarters of
+  // what is resident at once)
+  std::atomic<int64_t> whole_paths{-1};
   // shapes of kd-tree kernels that are no more: kept for callers that set and read them back
   std::atomic<int> persistent{0}, coop_leaf{3}, trav_block{256};
   std::atomic<int> bin_extension{1};  // counting-sort extension rays by (octant, origin cell)
@@ -1064,8 +1170,8 @@ static std::vector<CarveoutKernel> carveout_kernels() {
           {(const void *)k_extend<true, false, true>, kBlock, 0},
           {(const void *)k_shadow<false, false, true>, kBlock, 0},
           {(const void *)k_shadow<true, false, true>, kBlock, 0},
-          {(const void *)k_shade<false>, kShadeTile, 0},
-          {(const void *)k_shade<true>, kShadeTile, 0}};
+          {(const void *)k_shade<false>, kShadeTile, (int)sizeof(ShadeShared)},
+          {(const void *)k_shade<true>, kShadeTile, (int)sizeof(ShadeShared)}};
 }
 
 // percent of the SM's shared memory that holds the kernel's resident blocks (registers and
@@ -1378,7 +1484,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
   MGPU_CUDA(kernel_attributes());
   const int g_gen = grid_for((const void *)k_generate, 0);
   const int g_ext = grid_for((const void *)kext, tsm, tb);
-  const int g_sha = grid_for((const void *)k_shade<true>, 0, kShadeTile);
+  const int g_sha = grid_for((const void *)k_shade<true>, sizeof(ShadeShared), kShadeTile);
   const int g_shw = grid_for((const void *)kshw, tsm, tb);
   const int g_acc = grid_for((const void *)k_accumulate, 0);
   const int g_bin = device_sm_count() * 4;
@@ -1433,6 +1539,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
     a.stats = w->stats;
     a.tcount = w->tcount;
     a.max_b = wv.max_b;
+    a.seq = sph ? 1 : 0;
     const int max_b = wv.max_b;
     bool surf = false;  // a chunk's scene has image maps, a background or analytic spheres
     for (const JobArgs &c : wv.chunks)
@@ -1443,7 +1550,31 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
     k_generate<<<g_gen, kBlock, 0, st>>>(a);
     pf.end(m, st);
     ++launches;
+    auto kshd = surf ? k_shade<true> : k_shade<false>;
     int b = 0;
+    // Whole paths in one launch where the rays fit three quarters of the blocks that are resident at once: with
+    // more, the queues' compaction over the whole wave is worth its launches (waves against whole paths:
+    // 3,404 paths of a 2 k-triangle scene 154 / 77 us, 49,152 231 / 109; in the plain box 155,236 442 / 391,
+    // 262,144 527 / 640; textured 155,236 627 / 805; 131,072 without a depth cap 1,201 / 614).
+    const bool can_whole = wide && !COUNT && g_tune.whole_paths.load() != 0;
+    const int64_t whole_max = g_tune.whole_paths.load() > 0
+                                  ? g_tune.whole_paths.load()
+                                  : (int64_t)device_sm_count() * kShadeMinBlocks * kShadeTile * 3 / 4;
+    auto run_whole = [&](int64_t rays, int from) {
+      // a block per SM at least, then full tiles (textured, 49,152 paths: 398 us in tiles of 256, 557 of 96)
+      const int64_t sms = device_sm_count();
+      const uint32_t per = (uint32_t)std::min<int64_t>(kShadeTile, ((rays + sms - 1) / sms + 31) / 32 * 32);
+      RenderArgs w1 = a;
+      w1.bin_ext = 0;  // a block's next rays stay with the block
+      const int mk = pf.begin(kProfShade, st);
+      kshd<<<(unsigned)((rays + per - 1) / per), kShadeTile, sizeof(ShadeShared), st>>>(w1, from, per);
+      pf.end(mk, st);
+      ++launches;
+    };
+    if (can_whole && wv.npaths <= whole_max) {
+      run_whole(wv.npaths, 0);
+      b = max_b;
+    }
     while (b < max_b && err == cudaSuccess) {
       // with a fixed depth cap every bounce is launched blind; without one, check the live
       // count every 4 bounces and stop when the wave has drained
@@ -1453,8 +1584,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
         kext<<<g_ext, tb, tsm, st>>>(a, b);
         pf.end(m, st);
         m = pf.begin(kProfShade, st);
-        if (surf) k_shade<true><<<g_sha, kShadeTile, 0, st>>>(a, b);
-        else k_shade<false><<<g_sha, kShadeTile, 0, st>>>(a, b);
+        kshd<<<g_sha, kShadeTile, sizeof(ShadeShared), st>>>(a, b, 0);
         pf.end(m, st);
         if (a.bin_ext && b + 1 < max_b) {
           const int nx = (b + 1) & 1;
@@ -1476,6 +1606,10 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
       err = cudaMemcpyAsync(w->h_counters, w->counters + kCtrRay + b, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
       if (err == cudaSuccess) err = cudaStreamSynchronize(st);
       if (err != cudaSuccess || w->h_counters[0] == 0) break;
+      if (can_whole && (int64_t)w->h_counters[0] <= whole_max && b < max_b) {  // the long tail of few paths
+        run_whole(w->h_counters[0], b);
+        break;
+      }
     }
     m = pf.begin(kProfAccumulate, st);
     k_accumulate<<<g_acc, kBlock, 0, st>>>(a);
@@ -1657,6 +1791,7 @@ int mgpu_tune_set(const char *key, int64_t value) {
   else if (k == "coop_leaf" && value >= 0 && value <= 3) g_tune.coop_leaf.store((int)value);
   else if (k == "trav_block" && (value == 64 || value == 128 || value == 256)) g_tune.trav_block.store((int)value);
   else if (k == "wide") g_tune.wide.store(value != 0);
+  else if (k == "whole_paths" && value >= -1) g_tune.whole_paths.store(value);
   else if (k == "bin_shadow") g_tune.bin_shadow.store(value != 0);
   else if (k == "bin_extension") g_tune.bin_extension.store(value != 0);
   else if (k == "bin_min_paths" && value >= 0) g_tune.bin_min_paths.store(value);
@@ -1674,6 +1809,7 @@ int mgpu_tune_get(const char *key, int64_t *value) {
   else if (k == "coop_leaf") *value = g_tune.coop_leaf.load();
   else if (k == "trav_block") *value = g_tune.trav_block.load();
   else if (k == "wide") *value = g_tune.wide.load();
+  else if (k == "whole_paths") *value = g_tune.whole_paths.load();
   else if (k == "bin_shadow") *value = g_tune.bin_shadow.load();
   else if (k == "bin_extension") *value = g_tune.bin_extension.load();
   else if (k == "bin_min_paths") *value = g_tune.bin_min_paths.load();

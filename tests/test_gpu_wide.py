@@ -159,3 +159,29 @@ def test_negative_tmin_and_lines(cuda):
     # FP32 against FP64: a ray within rounding of an edge (about 1e-6 of the box) may decide otherwise
     ok = np.isclose(h[:, 0], best, rtol=1e-4, atol=1e-5) | (np.isinf(h[:, 0]) & np.isinf(best))
     assert ok.mean() >= 0.999, ok.mean()
+
+
+@pytest.mark.parametrize("w,h,spp,depth", [(1, 1, 1, 1), (5, 3, 7, 1), (16, 16, 1, 2), (33, 8, 1, 5), (37, 23, 4, 6),
+                                           (64, 64, 9, 0)])
+@pytest.mark.parametrize("kind", ["random", "textured", "balls"])
+def test_whole_paths_equal_the_waves(cuda, kind, w, h, spp, depth):
+    # one launch per wave (blocks of 32 to 256 rays, remainders, a long tail) against one launch per kernel and bounce
+    s = scenegen.textured(5) if kind == "textured" else _scene(kind)
+    if kind != "textured":
+        s.materials[s.tri_mat[0]] = dielectric(1.5)
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    st = pt.RenderSettings(w, h, spp, no_direct_samples=4, max_depth=depth, rr_start_depth=3, seed=8)
+    out, stats = [], []
+    assert pt.tune_get("whole_paths") == -1
+    try:
+        for whole in (0, -1, 1 << 20):
+            pt.tune("whole_paths", whole)
+            f = pt.Film(w, h)
+            pt.render(ds, st, f)
+            out.append(f.raw())
+            r = pt.render_stats()
+            stats.append((r["extension_rays"], r["shadow_rays"], r["bounces"], r["paths"]))
+    finally:
+        pt.tune("whole_paths", -1)
+    assert all(np.array_equal(out[0].view(np.uint32), o.view(np.uint32)) for o in out[1:])
+    assert stats[0] == stats[1] == stats[2] or depth == 0 and stats[0][:2] == stats[1][:2] == stats[2][:2]
