@@ -41,8 +41,9 @@ constexpr uint32_t kWideRootBits = 0x101u;  // pending slots and inner mask of t
 // 114 / 108 / 102 ms in blocks of 256 / 512 / 1024.
 constexpr int kWideBlock = 1024;
 // Rays that a block takes at a time; its warps take them 32 by 32 as they finish (mid frame: 97.0,
-// 96.3, 98.2, 101.1 ms at 1024, 512, 2048, 4096 against 102 in fixed grid-stride rounds).
-constexpr uint32_t kWideChunk = 512u;
+// 96.3, 98.2, 101.1 ms at 1024, 512, 2048, 4096 against 102 in fixed grid-stride rounds; on the
+// present kernels 86.4, 86.0, 85.6 at 1024, 512, 256).
+constexpr uint32_t kWideChunk = 256u;
 // Triangle tests waiting after a node step that are worth a round of their own: a full queue (32) keeps
 // every lane busy but lets the rays go on with a stale closest t (mid closest hits: 49.9 / 46.9 /
 // 46.5 ms at 32 / 16 / 8).
