@@ -89,6 +89,7 @@ struct RenderArgs {
   float4 *qo_u, *qd_u, *qt_u;    // unsorted next-ray queue (binning on)
   uint32_t *qkey;                // bin keys of the unsorted queue
   int32_t bin_ext;               // counting-sort the queue by (direction octant, origin cell)
+  int32_t dense;                 // every slot of the wave is a pixel
   int32_t sort_hits;             // a scene of the wave has more than one kind of BSDF
   uint32_t *counters;
   unsigned long long *stats;     // [0] extension rays, [1] shadow rays, [2] truncated paths, [3] bounces
@@ -244,9 +245,17 @@ __device__ __forceinline__ uint32_t ext_key(const JobArgs &J, V3 o, V3 d) {
 // ---------------------------------------------------------------------------------------
 // generate: camera rays for every path of the wave (RayTracer::sample, RayTracer.cpp:19-30;
 // SuperSampleGenerator strata, SuperSampleGenerator.cpp:60-90)
-__global__ void __launch_bounds__(kBlock) k_generate(RenderArgs a) {
+// A path's entry in the queue is its index in the wave where every slot is a pixel (a.dense: image sides that
+// are multiples of 8), else a block reserves its live paths with one atomic (one per warp was 2 M to
+// one address on the mid frame).  Throughput and state of a first vertex are constants that shading knows
+//.
+constexpr int kGenBlock = 256;
+
+__global__ void __launch_bounds__(kGenBlock) k_generate(const __grid_constant__ RenderArgs a) {
+  __shared__ uint32_t cnt[kGenBlock / 32], first;
   const int64_t n = a.npaths;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  if (a.dense && blockIdx.x == 0 && threadIdx.x == 0) a.counters[kCtrRay] = (uint32_t)n;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
     int64_t p = base + threadIdx.x;
     bool valid = p < n;
@@ -255,7 +264,7 @@ __global__ void __launch_bounds__(kBlock) k_generate(RenderArgs a) {
     if (valid) {
       const int j = job_of_path(a, p);
       const JobArgs &J = a.jobs[j];
-      a.path_job[p] = (uint32_t)j;
+      if (a.njobs > 1) a.path_job[p] = (uint32_t)j;
       int x, y, s;
       uint64_t pid = path_id(J, p, x, y, s);
       live = x < J.W && y < J.H;
@@ -276,11 +285,23 @@ __global__ void __launch_bounds__(kBlock) k_generate(RenderArgs a) {
       }
       a.path_L[p] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(flags));
     }
-    uint32_t q = warp_append(&a.counters[kCtrRay + 0], live);
+    uint32_t q = (uint32_t)p;
+    if (!a.dense) {
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, live), lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+      if (lane == 0u) cnt[warp] = __popc(m);
+      __syncthreads();
+      uint32_t at = __popc(m & ((1u << lane) - 1u)), all = 0u;
+      for (uint32_t w = 0; w < kGenBlock / 32; ++w) {
+        if (w < warp) at += cnt[w];
+        all += cnt[w];
+      }
+      if (threadIdx.x == 0) first = all ? atomicAdd(&a.counters[kCtrRay], all) : 0u;
+      __syncthreads();
+      q = first + at;
+    }
     if (live) {
       a.qo[0][q] = o4;
       a.qd[0][q] = d4;
-      a.qt[0][q] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(0u));
     }
   }
 }
@@ -470,7 +491,7 @@ __device__ __noinline__ void block_shadow(const RenderArgs &a, ShadeShared &sh, 
   wide_trace<true, false, SPH, false, true>(
       WideAll(),
       [&](uint32_t i) -> const SceneView & {
-        return a.jobs[a.path_job[__float_as_uint(so[i].w) / (uint32_t)a.nl_stride]].view;
+        return a.njobs == 1 ? a.jobs[0].view : a.jobs[a.path_job[__float_as_uint(so[i].w) / (uint32_t)a.nl_stride]].view;
       },
       n,
       [&](uint32_t i, Ray &r) {
@@ -559,7 +580,9 @@ __global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(const __g
     Material m;
     m.type = 0;
     if (valid) {
-      float4 o4 = a.qo[cur][i], d4 = a.qd[cur][i], t4 = a.qt[cur][i], h4 = a.qhit[i];
+      float4 o4 = a.qo[cur][i], d4 = a.qd[cur][i], h4 = a.qhit[i];
+      // a first vertex: throughput 1, depth 0 (k_generate writes none)
+      const float4 t4 = b == 0 ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : a.qt[cur][i];
       p = (int64_t)__float_as_int(o4.w);
       j = __float_as_int(d4.w);
       const JobArgs &J = a.jobs[j];
@@ -766,6 +789,7 @@ __global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMi
   uint32_t rays = 0;
   const bool single = a.njobs == 1;
   auto view_of = [&](uint32_t i) -> const SceneView & {
+    if (single) return a.jobs[0].view;
     const uint32_t slot = __float_as_uint(so[i].w);
     return a.jobs[a.path_job[slot / (uint32_t)a.nl_stride]].view;
   };
@@ -1492,7 +1516,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
   const int tb = wide ? kWideBlock : kBlock;
   const size_t tsm = wide ? (size_t)kWideSmem : 0;
   MGPU_CUDA(kernel_attributes());
-  const int g_gen = grid_for((const void *)k_generate, 0);
+  const int g_gen = grid_for((const void *)k_generate, 0, kGenBlock);
   const int g_ext = grid_for((const void *)kext, tsm, tb);
   const int g_sha = grid_for((const void *)k_shade<true>, sizeof(ShadeShared), kShadeTile);
   const int g_shw = grid_for((const void *)kshw, tsm, tb);
@@ -1545,6 +1569,8 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
     for (const JobArgs &c : wv.chunks) wave_tris = std::max(wave_tris, c.view.ntri);
     a.bin_ext = wv.npaths >= bin_min && (wave_tris >= kBinMinTris || bin_min == 0) ? bin_ext : 0;
     a.sort_hits = sort_hits;
+    a.dense = 1;
+    for (const JobArgs &c : wv.chunks) a.dense = a.dense && c.W % 8 == 0 && c.H % 8 == 0;
     a.counters = w->counters;
     a.stats = w->stats;
     a.tcount = w->tcount;
@@ -1557,7 +1583,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
              c.bg_le[2] != 0.0f || c.view.nsphere > 0;
     err = cudaMemsetAsync(w->counters, 0, kNumCounters * sizeof(uint32_t), st);
     int m = pf.begin(kProfGenerate, st);
-    k_generate<<<g_gen, kBlock, 0, st>>>(a);
+    k_generate<<<g_gen, kGenBlock, 0, st>>>(a);
     pf.end(m, st);
     ++launches;
     auto kshd = surf ? k_shade<true> : k_shade<false>;
