@@ -578,7 +578,7 @@ int mgpu_scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void
     s->view.wcentre[k] = std::isfinite(c) ? c : 0.0f;
     s->view.wextent = std::max(s->view.wextent, std::max(s->view.bmax[k] - s->view.wcentre[k], s->view.wcentre[k] - s->view.bmin[k]));
   }
-  if (int rc = wide_build(s->view.tris, T, s->view.wcentre, base + L.off_wnodes, (F4 *)(base + L.off_wtris), base + L.off_wscratch, st,
+  if (int rc = wide_build(s->view.tris, T, s->view, base + L.off_wnodes, (F4 *)(base + L.off_wtris), base + L.off_wscratch, st,
                           &wide_nodes, &wide)) {
     cudaFree(s->d_block);
     delete s;

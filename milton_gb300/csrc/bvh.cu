@@ -93,6 +93,7 @@ struct Build {
   F4 *wtris;
   uint32_t cap_nodes;
   float centre[3];        // node coordinates are relative to it
+  float bmin[3], bmax[3];  // the kd-tree's root box
 };
 
 // counters
@@ -735,6 +736,11 @@ __device__ void emit_node(const Build &B, uint32_t w, bool valid, int32_t *xn, i
       if (((hi - org[k]) - step[k] * 32768.0f) * inv[k] + 1.0f / 32.0f <= 255.0f) break;
     }
   }
+  // The kd-tree's root box leaves out triangles whose bounds compare equal under Milton's fuzzy comparison (flat
+  // ones from -1 to 1, kdbuild.cpp), and rays find such a triangle only inside that box.  A scene with one
+  // that sticks out keeps the kd-tree's answers, and its traversal.
+  if (w == 0u)
+    for (int k = 0; k < 3; ++k) fits = fits && box.lo[k] >= B.bmin[k] && box.hi[k] <= B.bmax[k];
   const int cnt = x < 0 || !leaf ? 0 : (x < B.n ? 1 : (int)B.cut[x - B.n].prims);
   const uint32_t imask = __reduce_or_sync(group, x >= 0 && !leaf ? 1u << slot : 0u);
   const uint32_t tvalid = __reduce_or_sync(group, cnt ? ((1u << cnt) - 1u) << (3 * slot) : 0u);
@@ -927,7 +933,7 @@ size_t wide_scratch(int64_t n) {
   return n > 0 && n <= kSmall ? place_scratch(B, n, nullptr) : 0;
 }
 
-int wide_build(const F4 *tris, int64_t n, const float *centre, void *wnodes, F4 *wtris, void *scratch, cudaStream_t st,
+int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F4 *wtris, void *scratch, cudaStream_t st,
                uint32_t *nodes_out, bool *ok) {
   *ok = false;
   *nodes_out = 0;
@@ -938,7 +944,11 @@ int wide_build(const F4 *tris, int64_t n, const float *centre, void *wnodes, F4 
   B.tris = tris;
   B.wnodes = (uint32_t *)wnodes;
   B.wtris = wtris;
-  for (int k = 0; k < 3; ++k) B.centre[k] = centre[k];
+  for (int k = 0; k < 3; ++k) {
+    B.centre[k] = view.wcentre[k];
+    B.bmin[k] = view.bmin[k];
+    B.bmax[k] = view.bmax[k];
+  }
   B.cap_nodes = (uint32_t)wide_node_cap(n);
   const int radix_blocks = (int)((n + kRadixTile - 1) / kRadixTile);
   const size_t bytes = place_scratch(B, n, nullptr);

@@ -50,7 +50,7 @@ int tex_upload(const mgpu_scene_desc *desc, const TexPlan &plan, float4 *d_texre
 // scratch memory, or a hierarchy beyond the traversal's limits) and the kd-tree is used.
 int64_t wide_node_cap(int64_t ntri);
 size_t wide_scratch(int64_t n);
-int wide_build(const F4 *tris, int64_t n, const float *centre, void *wnodes, F4 *wtris, void *scratch, cudaStream_t st,
+int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F4 *wtris, void *scratch, cudaStream_t st,
                uint32_t *nodes_out, bool *ok);
 
 }  // namespace mgpu

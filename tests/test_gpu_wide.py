@@ -185,3 +185,18 @@ def test_whole_paths_equal_the_waves(cuda, kind, w, h, spp, depth):
         pt.tune("whole_paths", -1)
     assert all(np.array_equal(out[0].view(np.uint32), o.view(np.uint32)) for o in out[1:])
     assert stats[0] == stats[1] == stats[2] or depth == 0 and stats[0][:2] == stats[1][:2] == stats[2][:2]
+
+
+def test_a_triangle_outside_the_kd_trees_root_box(cuda):
+    # flat quads from -1 to 1 do not widen the root box (Milton's fuzzy comparison), and are hit inside it only
+    t = _random_tris(400, 12, size=0.05) * 0.5
+    q = [scenegen.quad_tris((x, -1, 1), (x, 1, 1), (x, 1, -1), (x, -1, -1)) for x in (-0.9, 0.1, 0.9)]
+    s = _soup(np.concatenate(q + [t]))
+    a = pt.Accel(s)
+    ds = pt.DeviceScene(s, a)
+    rays = _rays(s, 5000, 13)
+    kd, _ = gpu_trace(cuda, ds, rays, counts=True)
+    wide, _ = gpu_trace(cuda, ds, rays)
+    assert (kd[:, 1].view(np.int32) >= 0).any()
+    assert np.array_equal(kd.view(np.uint32), wide.view(np.uint32))
+    assert np.array_equal(gpu_any(cuda, ds, rays) != 0, kd[:, 1].view(np.int32) >= 0)
