@@ -374,7 +374,7 @@ def run_ours(args):
     def per_ray(prefix, out_bytes):
         n = max(cnt[prefix + "_rays"], 1)
         nodes, refs, tris = cnt[prefix + "_nodes"] / n, cnt[prefix + "_refs"] / n, cnt[prefix + "_tris"] / n
-        return dict(nodes=nodes, refs=refs, tris=tris, bytes=32 + out_bytes + 96 * nodes + 4 * refs + 48 * tris)  # 8-wide nodes
+        return dict(nodes=nodes, refs=refs, tris=tris, bytes=32 + out_bytes + 128 * nodes + 4 * refs + 48 * tris)  # 8-wide nodes
 
     ext_ray = per_ray("ext", 16)
     sh_ray = per_ray("sh", 4)

@@ -639,6 +639,12 @@ __global__ void __launch_bounds__(128) k_bvh_cut(Build B) {
 // first wide node of the next level = the nodes there are now
 __global__ void k_bvh_level(Build B, int level) { B.ctr[kCLevel + level] = B.ctr[kCNodes]; }
 
+// The upper half of the smallest float no less than v whose lower half is zero.
+__device__ __forceinline__ uint32_t plane_above(float v) {
+  const uint32_t u = __float_as_uint(v);
+  return (u + ((u & 0x80000000u) ? 0u : 0xFFFFu)) >> 16;
+}
+
 // Eight lanes per wide node, one per child (called by whole warps; valid is uniform over the eight).
 // xn, xj: eight words of shared memory each per group.
 __device__ void emit_node(const Build &B, uint32_t w, bool valid, int32_t *xn, int32_t *xj) {
@@ -717,24 +723,13 @@ __device__ void emit_node(const Build &B, uint32_t w, bool valid, int32_t *xn, i
     if ((at >> 4) == lane) slot = (int)(at & 7u);
     free_slots &= ~(1u << (at & 7u));
   }
-  // the grid: a step of a power of two, its origin (stored less 2^15 steps, so that the traversal can
-  // take a plane's byte as the float 1 + byte / 2^15) at least a thirty-second step below the
-  // box, so that every child keeps at least a sixty-fourth step of slack after rounding outward
-  float org[3], inv[3], step[3];
+  // the node's centre, relative to the scene's
+  float mid[3];
   bool fits = true;
   for (int k = 0; k < 3; ++k) {
-    const float lo = __fsub_rd(box.lo[k], B.centre[k]), hi = __fsub_ru(box.hi[k], B.centre[k]);
-    const float s0 = fmaxf(fmaxf((hi - lo) * (1.0f / 254.0f), 6.0e-8f * fmaxf(fabsf(lo), fabsf(hi))), 1.0e-30f);
-    int e = (int)(__float_as_uint(s0) >> 23) - 127;
-    if (__float_as_uint(s0) & 0x7FFFFFu) ++e;
-    for (;; ++e) {
-      fits = fits && e <= 112;  // 2^15 s is a finite float
-      if (!fits) break;
-      step[k] = __uint_as_float((uint32_t)(e + 127) << 23);
-      inv[k] = __uint_as_float((uint32_t)(127 - e) << 23);
-      org[k] = __fsub_rd(__fsub_rd(lo, step[k] * (1.0f / 32.0f)), step[k] * 32768.0f);
-      if (((hi - org[k]) - step[k] * 32768.0f) * inv[k] + 1.0f / 32.0f <= 255.0f) break;
-    }
+    const float lo = box.lo[k] - B.centre[k], hi = box.hi[k] - B.centre[k];
+    mid[k] = 0.5f * lo + 0.5f * hi;
+    fits = fits && fmaxf(fabsf(lo), fabsf(hi)) <= 1.0e37f;  // the stored planes are finite
   }
   // The kd-tree's root box leaves out triangles whose bounds compare equal under Milton's fuzzy comparison (flat
   // ones from -1 to 1, kdbuild.cpp), and rays find such a triangle only inside that box.  A scene with one
@@ -757,20 +752,17 @@ __device__ void emit_node(const Build &B, uint32_t w, bool valid, int32_t *xn, i
     return;
   }
   uint32_t *o = B.wnodes + (size_t)w * kWideWords;
-  uint8_t *q = reinterpret_cast<uint8_t *>(o + 8);
-  if (x < 0) {  // an empty slot: a box turned inside out, and neither mask names it
+  if (x < 0) {  // an empty slot: neither mask names it
     int skip = (int)lane - nk;
     uint32_t f = free_slots;
     while (skip-- > 0) f &= f - 1u;
     const int e = __ffs(f) - 1;
-    for (int k = 0; k < 3; ++k) { q[8 * k + e] = 255; q[24 + 8 * k + e] = 0; }
+    for (int k = 0; k < 3; ++k) o[8 + 3 * e + k] = 0u;
   } else {
     for (int k = 0; k < 3; ++k) {
-      const double g = (double)org[k] + 32768.0 * (double)step[k];  // exact: the grid's origin
-      const float lo = floorf((float)((double)kb.lo[k] - B.centre[k] - g) * inv[k] - 1.0f / 60.0f);
-      const float hi = ceilf((float)((double)kb.hi[k] - B.centre[k] - g) * inv[k] + 1.0f / 60.0f);
-      q[8 * k + slot] = (uint8_t)fminf(fmaxf(lo, 0.0f), 255.0f);
-      q[24 + 8 * k + slot] = (uint8_t)fminf(fmaxf(hi, 0.0f), 255.0f);
+      const float lo = __double2float_rd((double)kb.lo[k] - B.centre[k] - mid[k]);
+      const float hi = __double2float_ru((double)kb.hi[k] - B.centre[k] - mid[k]);
+      o[8 + 3 * slot + k] = (plane_above(-lo) ^ 0x8000u) | (plane_above(hi) << 16);
     }
     if (leaf) {
       uint32_t at = tb + __popc(tvalid & ((1u << (3 * slot)) - 1u));
@@ -799,14 +791,12 @@ __device__ void emit_node(const Build &B, uint32_t w, bool valid, int32_t *xn, i
     }
   }
   if (lane == 0u) {
-    for (int k = 0; k < 3; ++k) {
-      o[k] = __float_as_uint(org[k]);
-      o[4 + k] = __float_as_uint(step[k] * 32768.0f);
-    }
+    for (int k = 0; k < 3; ++k) o[k] = __float_as_uint(mid[k]);
     o[3] = cb;
-    o[7] = tb;
-    o[20] = imask;
-    o[21] = tvalid;
+    o[4] = tb;
+    o[5] = imask;
+    o[6] = tvalid;
+    o[7] = 0u;
   }
 }
 

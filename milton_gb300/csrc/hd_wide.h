@@ -6,21 +6,25 @@
 // and barycentrics, bit for bit.
 //
 // Why a wide hierarchy: on the mid scene (1 M triangles) the kd-tree takes 50 dependent node steps
-// and 33 triangle tests per ray.  The node here holds eight child boxes on an 8-bit grid of the
-// parent's box in 96 bytes, as in Ylitie, Karras and Laine, "Efficient
-// Incoherent Ray Traversal on GPUs Through Compressed Wide BVHs", HPG 2017.
+// and 33 triangle tests per ray.  The node here holds eight child boxes as 16-bit floats around the
+// node's centre in 128 bytes, one cache line (8-bit grid coordinates in 96 bytes, as the paper has
+// them: more conversions per box, and flat boxes grow by a grid step, so that a ray met the wall it
+// starts on and the light it ends at; 24-triangle room: 4.5 -> 2.7 triangles per occlusion query, frame
+// 0.94 -> 0.87 ms; mid frame 111.4 -> 105.5 ms); the masks, the child order and the single stack entry per
+// level are those of Ylitie, Karras and Laine, "Efficient Incoherent Ray Traversal on GPUs Through
+// Compressed Wide BVHs", HPG 2017.
 //
-// Node (24 words, three 256-bit loads), coordinates relative to the scene's centre:
-//   0..2   origin of the child grid (below the node's box on every axis) minus 2^15 steps
+// Node (32 words, four 256-bit loads):
+//   0..2   centre of the node's box, relative to the scene's centre
 //   3      index of the first inner child (the inner children of a node are consecutive, in slot
 //          order)
-//   4..6   2^15 x the grid step per axis (a power of two)
-//   7      index of the node's first triangle record (the leaf children's triangles are
+//   4      index of the node's first triangle record (the leaf children's triangles are
 //          consecutive, in slot order)
-//   8..19  child planes: low x, y, z then high x, y, z, 8 bytes each (one per slot)
-//   20     mask of the slots that hold inner nodes
-//   21     triangles of the leaf children: bits 3 s .. 3 s + 2 hold slot s's count in unary
-//   22, 23 unused
+//   5      mask of the slots that hold inner nodes
+//   6      triangles of the leaf children: bits 3 s .. 3 s + 2 hold slot s's count in unary
+//   7      unused
+//   8 + 3 s + k   slot s's planes along axis k, relative to the centre: the upper halves of two floats, low
+//          plane in bits 0..15, high plane in bits 16..31
 // Triangle record: 3 x float4 as a kd leaf's (v0 + primitive id, v1 + flags, v2).
 //
 // A slot's number says where its child lies: bit k set = the upper side along axis k.  A ray visits
@@ -32,7 +36,7 @@
 
 namespace mgpu {
 
-constexpr int kWideWords = 24;       // 32-bit words per node
+constexpr int kWideWords = 32;       // 32-bit words per node
 constexpr int kWideLeafTris = 3;     // triangles per leaf child
 constexpr int kWideMaxDepth = 30;    // levels of node below the root that the traversal stack holds
 constexpr uint32_t kWideRootBits = 0x101u;  // pending slots and inner mask of the root's pseudo parent
@@ -49,19 +53,17 @@ constexpr uint32_t kWideChunk = 256u;
 // 46.5 ms at 32 / 16 / 8).
 constexpr uint32_t kWideFlush = 8u;
 
-// Box tests are conservative.  The builder leaves at least 1/64 step of slack around every child, which
-// covers what rounds relative to the node's own size (the offset by 2^15 steps: 1/512 step).  What
-// rounds relative to M, the largest coordinate of the scene box or the ray's origin from the
-// scene's centre -- the plane distances (4 x 2^-24 M) and the triangle test's sheared
-// coordinates (6 x 2^-24 of at most 2 M) -- is covered by moving every plane outward by
-// 1.25 x 2^-20 M, folded into the ray's constants.
-constexpr float kWideEps = 1.25f / 1048576.0f;
+// Box tests are conservative.  The planes are rounded outward when they are stored.  What rounds relative
+// to M, the largest coordinate of the scene box or the ray's origin from the scene's centre -- the
+// plane distances (6 x 2^-24 M) and the triangle test's sheared coordinates (6 x 2^-24 of at most
+// 2 M) -- is covered by moving every plane outward by 1.5 x 2^-20 M, folded into the ray's constants.
+constexpr float kWideEps = 1.5f / 1048576.0f;
 
 #if defined(__CUDACC__)
 
-// the byte `i` of w as the float 1 + byte / 2^15: one byte permute, no integer conversion
-__device__ __forceinline__ float wide_byte(uint32_t w, int i) {
-  return __uint_as_float(__byte_perm(w, 0x3F800000u, 0x7604u | ((uint32_t)i << 4)));
+// one half of w (which: the permute's selector) as the upper half of a float
+__device__ __forceinline__ float wide_half(uint32_t w, uint32_t which) {
+  return __uint_as_float(__byte_perm(w, 0u, which));
 }
 
 // Tables in shared memory, per block: first[oct][m] = the slot to visit first among those in m for a ray
@@ -120,7 +122,7 @@ struct WideRay {
   V3 inv;
   V3 kn, kf;            // -origin x inv moved outward: added to p x inv, near and far plane distances
   float tmin;
-  float best;           // closest t accepted so far (starts at the ray's tmax)
+  float best;           // t up to which boxes are visited: the ray's tmax, then just past the closest hit
   const uint8_t *first; // the table row of the ray's octant
 };
 
@@ -128,36 +130,39 @@ struct WideRay {
 __device__ __forceinline__ void wide_node(const uint32_t *__restrict__ nodes, uint32_t idx, const WideRay &w,
                                           float tmin, const WideTables &tab, WideGroup &ng, WideGroup &tg, uint32_t &tvalid) {
   const uint32_t *q = nodes + (size_t)idx * kWideWords;
-  const WideRow a = wide_load(q), b = wide_load(q + 8), c = wide_load(q + 16);
+  const WideRow a = wide_load(q);
+  uint32_t box[24];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const WideRow r = wide_load(q + 8 + 8 * k);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) box[8 * k + i] = r.w[i];
+  }
   const float px = __uint_as_float(a.w[0]), py = __uint_as_float(a.w[1]), pz = __uint_as_float(a.w[2]);
-  const float ax = __uint_as_float(a.w[4]) * w.inv.x, ay = __uint_as_float(a.w[5]) * w.inv.y,
-              az = __uint_as_float(a.w[6]) * w.inv.z;
   const float nx = fmaf(px, w.inv.x, w.kn.x), ny = fmaf(py, w.inv.y, w.kn.y), nz = fmaf(pz, w.inv.z, w.kn.z);
   const float fx = fmaf(px, w.inv.x, w.kf.x), fy = fmaf(py, w.inv.y, w.kf.y), fz = fmaf(pz, w.inv.z, w.kf.z);
-  const bool sx = w.inv.x < 0.0f, sy = w.inv.y < 0.0f, sz = w.inv.z < 0.0f;
+  // permutes that leave the near and the far half of a pair of planes on top of zeros
+  const uint32_t sx = w.inv.x < 0.0f ? 0x3244u : 0x1044u, sy = w.inv.y < 0.0f ? 0x3244u : 0x1044u,
+                 sz = w.inv.z < 0.0f ? 0x3244u : 0x1044u;
+  const uint32_t ux = sx ^ 0x2200u, uy = sy ^ 0x2200u, uz = sz ^ 0x2200u;
   uint32_t miss = 0u;
 #pragma unroll
-  for (int h = 1; h >= 0; --h) {
-    const uint32_t lox = b.w[h], loy = b.w[2 + h], loz = b.w[4 + h];
-    const uint32_t hix = b.w[6 + h], hiy = c.w[h], hiz = c.w[2 + h];
-    const uint32_t nearx = sx ? hix : lox, neary = sy ? hiy : loy, nearz = sz ? hiz : loz;
-    const uint32_t farx = sx ? lox : hix, fary = sy ? loy : hiy, farz = sz ? loz : hiz;
-#pragma unroll
-    for (int i = 3; i >= 0; --i) {
-      const float t0 = fmaxf(max3(fmaf(wide_byte(nearx, i), ax, nx), fmaf(wide_byte(neary, i), ay, ny),
-                                  fmaf(wide_byte(nearz, i), az, nz)), tmin);
-      const float t1 = fminf(min3(fmaf(wide_byte(farx, i), ax, fx), fmaf(wide_byte(fary, i), ay, fy),
-                                  fmaf(wide_byte(farz, i), az, fz)), w.best);
-      // the sign of t1 - t0 (t0 = t1 and NaN from two infinities give a plus: a hit) shifted in: one
-      // addition and one funnel shift instead of a comparison and a select
-      miss = __funnelshift_l(__float_as_uint(t1 - t0), miss, 1);
-    }
+  for (int i = 7; i >= 0; --i) {
+    const uint32_t bx = box[3 * i], by = box[3 * i + 1], bz = box[3 * i + 2];
+    const float t0 = max3(fmaf(wide_half(bx, sx), w.inv.x, nx), fmaf(wide_half(by, sy), w.inv.y, ny),
+                          fmaf(wide_half(bz, sz), w.inv.z, nz));
+    const float t1 = min3(fmaf(wide_half(bx, ux), w.inv.x, fx), fmaf(wide_half(by, uy), w.inv.y, fy),
+                          fmaf(wide_half(bz, uz), w.inv.z, fz));
+    // a miss if t1 < t0, best < t0 or t1 < tmin: the signs of the differences (NaN from two infinities has a
+    // plus: a hit), shifted in.  Additions instead of a maximum, a minimum and comparisons, because
+    // those share a pipe with the permutes (terrain 19.9 -> 19.6 ms a frame).
+    miss = __funnelshift_l(__float_as_uint(t1 - t0) | __float_as_uint(w.best - t0) | __float_as_uint(t1 - tmin), miss, 1);
   }
-  const uint32_t hits = ~miss & 0xFFu, imask = c.w[4];
+  const uint32_t hits = ~miss & 0xFFu, imask = a.w[5];
   ng.base = a.w[3];
   ng.bits = (hits & imask) | (imask << 8);
-  tg.base = a.w[7];
-  tvalid = c.w[5];
+  tg.base = a.w[4];
+  tvalid = a.w[6];
   tg.bits = tab.spread[hits & ~imask] & tvalid;
 }
 
@@ -236,7 +241,7 @@ __device__ __noinline__ void kd_ray(const SceneView &s, const Ray &r, bool seq, 
 // L2 below 8 % and DRAM below 3 % of their peaks.  The kd-tree's kernels were bound by the
 // latency of 50 dependent node loads per ray.  Mid frame (163 M closest hits, 226 M occlusion
 // queries): kd-tree 187.7 ms of traversal, nodes of 80 bytes with per-node slack and child order by mask
-// permutation 95.0, the node step as it is now 83.7.
+// permutation 95.0, nodes of 96 bytes on an 8-bit grid 83.7, as it is now 77.9.
 //   ANY     occlusion: the first hit ends the ray; otherwise the closest
 //   seq     which of the kd-tree's orders decides near ties (kd_ray)
 //   SINGLE  every ray is in the scene view(0), which the kernel passes from its parameter space
@@ -383,7 +388,9 @@ struct WideWarp {
       }
     } else {
       __syncwarp(kFull);
-      w.best = wide_unorder((uint32_t)(sh.key[lane] >> 32));
+      // hits within kWideTie behind the closest are looked at too: they make a near tie
+      const float t = wide_unorder((uint32_t)(sh.key[lane] >> 32));
+      w.best = fmaf(fabsf(t), 1.0625f * kWideTie, t);
     }
   }
 

@@ -200,3 +200,27 @@ def test_a_triangle_outside_the_kd_trees_root_box(cuda):
     assert (kd[:, 1].view(np.int32) >= 0).any()
     assert np.array_equal(kd.view(np.uint32), wide.view(np.uint32))
     assert np.array_equal(gpu_any(cuda, ds, rays) != 0, kd[:, 1].view(np.int32) >= 0)
+
+
+@pytest.mark.parametrize("scale,nudge", [(1.0, 0), (1.0, 1), (1.0, -1), (1e9, 1), (1e-9, -1)])
+def test_planes_at_the_roundings_of_16_bit_floats(cuda, scale, nudge):
+    # axis-aligned quads on, just above and just below values that the nodes store exactly (eight leading
+    # bits), on both sides of the centre: the rounding outward must not lose a quad, nor a sign
+    x = np.concatenate([np.arange(128, 256, 8) / 256, 2.0 ** -np.arange(1, 9), [0.0]])
+    x = np.unique(np.concatenate([x, -x])).astype(np.float32)
+    for _ in range(abs(nudge)):
+        x = np.nextafter(x, np.float32(np.inf * nudge))
+    q = np.concatenate([scenegen.quad_tris((v, -1, 1), (v, 1, 1), (v, 1, -1), (v, -1, -1)) for v in x[::5]] +
+                       [scenegen.quad_tris((-1, v, 1), (1, v, 1), (1, v, -1), (-1, v, -1)) for v in x[1::5]] +
+                       [scenegen.quad_tris((a, b, c), (a + .02, b, c), (a + .02, b + .02, c), (a, b + .02, c))
+                        for a in x[::4] for b in x[1::4] for c in x[2::4]])
+    s = _soup(q.astype(np.float64) * scale)
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    rays = _rays(_soup(q), 5000, 21)
+    rays[:, 0:4] *= np.float32(scale)
+    rays[:, 7] *= np.float32(scale)
+    kd, _ = gpu_trace(cuda, ds, rays, counts=True)
+    wide, _ = gpu_trace(cuda, ds, rays)
+    same = np.all(kd.view(np.uint32) == wide.view(np.uint32), axis=1)
+    assert same.all(), (int((~same).sum()), rays[~same][:2], kd[~same][:2], wide[~same][:2])
+    assert np.array_equal(gpu_any(cuda, ds, rays) != 0, kd[:, 1].view(np.int32) >= 0)
