@@ -368,7 +368,7 @@ int mgpu_profile_read(double *ms6, uint64_t *launches6);
  *   "wide"           0/1  traversal of the 8-wide hierarchy that mgpu_scene_create builds on the
  *                    device (default 1); 0 = the kd-tree, one ray per lane
  *   "whole_paths"    -1.. waves of at most n paths run every path to its end in one launch; 0 = none,
- *                    -1 = three quarters of what the GPU holds at once (default)
+ *                    -1 = what the GPU holds at once (default)
  *   "persistent" 0/1, "coop_leaf" 0..3, "trav_block" 64 / 128 / 256: shapes of earlier kd-tree
  *                    kernels; accepted and read back, they select nothing
  *   "bin_extension"  0/1  counting-sort extension rays by (direction octant, origin cell) (default 1)

@@ -380,7 +380,10 @@ __device__ __forceinline__ V3 fold_slots(const RenderArgs &a, int nl, int64_t p,
 // Threads of a shading block, and the rays that it takes at a time; four blocks per SM (64 registers; the
 // kernel's natural 125 and the spills of 48 both measure slower).
 constexpr int kShadeTile = 256;
-constexpr int kShadeMinBlocks = 4;
+// Blocks of the shade kernels per SM: three leave a thread 80 registers and half the spills of 64.  Shading per
+// frame at 3 / 4 / 2 blocks: mid scene 21.3 / 21.8 / 24.9 ms, plain box 0.302 / 0.332 / 0.327, terrain
+// 3.18 / 3.30 / 3.47, textured 0.99 / 1.00 / 1.12.
+constexpr int kShadeMinBlocks = 3;
 
 // What a shading block keeps in shared memory: per warp the shadow rays that wait for a full 32 (or, while
 // the block traces its own rays, the traversal's records), the counts and the order of the tile's
@@ -511,13 +514,13 @@ __device__ __noinline__ void block_shadow(const RenderArgs &a, ShadeShared &sh, 
 // them run the variant that has none of those branches, whose register allocation (and spilling)
 // is the lighter.
 //
-// whole: the launch takes whole paths instead of one bounce (waves of few paths).  Every block owns `whole` (at
+// WHOLE: the launch takes whole paths instead of one bounce (waves of few paths).  Every block owns `whole` (at
 // most 256) rays of bounce b and runs their bounces to the end: it traces its rays, shades them, traces
 // their shadow rays, and keeps the queues in its own part of the arrays.  One launch instead of three per
-// bounce, and blocks whose paths have ended do not wait for others.  It is this kernel and not one of
-// its own so that the shading is the same machine code: compiled twice, its multiply-adds contract
-// differently and an image would depend on the wave size.
-template <bool SURF>
+// bounce, and blocks whose paths have ended do not wait for others.  Both variants come from this one
+// text, with the traversal called and not inlined, so that the shading's multiply-adds contract alike in
+// them and an image does not depend on the wave size (tests/test_gpu_wide.py compares the bits).
+template <bool SURF, bool WHOLE>
 __global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(const __grid_constant__ RenderArgs a, int b,
                                                                        uint32_t whole) {
   extern __shared__ __align__(16) unsigned char shade_smem[];
@@ -529,7 +532,7 @@ __global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(const __g
   uint32_t out = 0u;  // first entry of the queues that the block writes
   uint32_t *next_ctr = &a.counters[kCtrRay + b + 1];
   ShadowStage stage{sh.stage.so[warp], sh.stage.sd[warp], &a.counters[kCtrNee + b], a.so, a.sd, 0u, 0u};
-  if (whole) {
+  if (WHOLE) {
     base = blockIdx.x * whole;
     if (base >= total) return;
     wide_tables(sh.tables);
@@ -543,7 +546,7 @@ __global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(const __g
   for (;;) {
     if (base >= n) break;
     const int cur = b & 1, nxt = (b + 1) & 1;
-    if (whole) {
+    if (WHOLE) {
       if (threadIdx.x == 0) sh.next = sh.rays = sh.shadow = 0u;
       __syncthreads();
       block_extend<SURF>(a, sh, b, base, n);
@@ -677,9 +680,9 @@ __global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(const __g
         a.qt[nxt][q] = no_t;
       }
     }
-    // What the light samples need now and then waits in shared memory, not in registers that spill (plain box:
-    // shading 0.340 -> 0.323 ms a frame, mid 24.0 -> 23.6).  Read back through `held`, which the compiler
-    // may not keep in registers.
+    // What the light samples need now and then waits in shared memory, not in registers that spill (textured
+    // frame, shading 1.007 -> 0.979 ms; plain box and mid scene within 1 %).  Read back through `held`, which
+    // the compiler may not keep in registers.
     volatile float(*held)[kShadeTile] = sh.held;
     held[0][threadIdx.x] = ng.x; held[1][threadIdx.x] = ng.y; held[2][threadIdx.x] = ng.z;
     held[3][threadIdx.x] = thr.x; held[4][threadIdx.x] = thr.y; held[5][threadIdx.x] = thr.z;
@@ -754,7 +757,7 @@ __global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(const __g
       }
       stage.append(want, so4, sd4);
     }
-    if (!whole) {
+    if (!WHOLE) {
       base += stride;
       continue;
     }
@@ -774,7 +777,7 @@ __global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(const __g
     ++b;
     if (b >= a.max_b) n = base;
   }
-  if (!whole) stage.flush();
+  if (!WHOLE) stage.flush();
 }
 
 
@@ -1003,8 +1006,7 @@ constexpr int kCarveoutAuto = -2;
 struct Tuning {
   // the 8-wide hierarchy where every scene of a render has one; 0: the kd-tree
   std::atomic<int> wide{1};
-  // waves of at most this many paths run whole paths in one launch (0: none do; -1: three quarters of
-  // what is resident at once)
+  // waves of at most this many paths run whole paths in one launch (0: none do; -1: what is resident at once)
   std::atomic<int64_t> whole_paths{-1};
   // shapes of kd-tree kernels that are no more: kept for callers that set and read them back
   std::atomic<int> persistent{0}, coop_leaf{3}, trav_block{256};
@@ -1204,8 +1206,10 @@ static std::vector<CarveoutKernel> carveout_kernels() {
           {(const void *)k_extend<true, false, true>, kBlock, 0},
           {(const void *)k_shadow<false, false, true>, kBlock, 0},
           {(const void *)k_shadow<true, false, true>, kBlock, 0},
-          {(const void *)k_shade<false>, kShadeTile, (int)sizeof(ShadeShared)},
-          {(const void *)k_shade<true>, kShadeTile, (int)sizeof(ShadeShared)}};
+          {(const void *)k_shade<false, false>, kShadeTile, (int)sizeof(ShadeShared)},
+          {(const void *)k_shade<true, false>, kShadeTile, (int)sizeof(ShadeShared)},
+          {(const void *)k_shade<false, true>, kShadeTile, (int)sizeof(ShadeShared)},
+          {(const void *)k_shade<true, true>, kShadeTile, (int)sizeof(ShadeShared)}};
 }
 
 // percent of the SM's shared memory that holds the kernel's resident blocks (registers and
@@ -1518,7 +1522,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
   MGPU_CUDA(kernel_attributes());
   const int g_gen = grid_for((const void *)k_generate, 0, kGenBlock);
   const int g_ext = grid_for((const void *)kext, tsm, tb);
-  const int g_sha = grid_for((const void *)k_shade<true>, sizeof(ShadeShared), kShadeTile);
+  const int g_sha = grid_for((const void *)k_shade<true, false>, sizeof(ShadeShared), kShadeTile);
   const int g_shw = grid_for((const void *)kshw, tsm, tb);
   const int g_acc = grid_for((const void *)k_accumulate, 0);
   const int g_bin = device_sm_count() * 4;
@@ -1586,16 +1590,17 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
     k_generate<<<g_gen, kGenBlock, 0, st>>>(a);
     pf.end(m, st);
     ++launches;
-    auto kshd = surf ? k_shade<true> : k_shade<false>;
+    auto kshd = surf ? k_shade<true, false> : k_shade<false, false>;
+    auto kshp = surf ? k_shade<true, true> : k_shade<false, true>;
     int b = 0;
-    // Whole paths in one launch where the rays fit three quarters of the blocks that are resident at once: with
-    // more, the queues' compaction over the whole wave is worth its launches (waves against whole paths:
-    // 3,404 paths of a 2 k-triangle scene 154 / 77 us, 49,152 231 / 109; in the plain box 155,236 442 / 391,
-    // 262,144 527 / 640; textured 155,236 627 / 805; 131,072 without a depth cap 1,201 / 614).
+    // Whole paths in one launch where the rays fit the blocks that are resident at once: with more, the queues'
+    // compaction over the whole wave is worth its launches (waves against whole paths: 3,404 paths of a 2 k-triangle
+    // scene 144 / 75 us, 49,152 212 / 94; in the plain box 115,600 379 / 269, 155,236 404 / 398; textured
+    // 115,600 561 / 521, 155,236 591 / 737; 105,800 without a depth cap 1,006 / 461).
     const bool can_whole = wide && !COUNT && g_tune.whole_paths.load() != 0;
     const int64_t whole_max = g_tune.whole_paths.load() > 0
                                   ? g_tune.whole_paths.load()
-                                  : (int64_t)device_sm_count() * kShadeMinBlocks * kShadeTile * 3 / 4;
+                                  : (int64_t)device_sm_count() * kShadeMinBlocks * kShadeTile;
     auto run_whole = [&](int64_t rays, int from) {
       // a block per SM at least, then full tiles (textured, 49,152 paths: 398 us in tiles of 256, 557 of 96)
       const int64_t sms = device_sm_count();
@@ -1603,7 +1608,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
       RenderArgs w1 = a;
       w1.bin_ext = 0;  // a block's next rays stay with the block
       const int mk = pf.begin(kProfShade, st);
-      kshd<<<(unsigned)((rays + per - 1) / per), kShadeTile, sizeof(ShadeShared), st>>>(w1, from, per);
+      kshp<<<(unsigned)((rays + per - 1) / per), kShadeTile, sizeof(ShadeShared), st>>>(w1, from, per);
       pf.end(mk, st);
       ++launches;
     };
