@@ -322,22 +322,25 @@ __global__ void __launch_bounds__(256) k_bvh_leaves(Build B, const int32_t *__re
 
 // ---- clustering ---------------------------------------------------------------------------
 
-// The neighbour of cluster i with the least union area; the order (area, smaller index, larger index)
-// is the same from both sides, so the least pair overall is mutual and every round merges.
-__device__ __forceinline__ int nearest(const Box *sb, int at, int i, int count) {
-  float best = INFINITY;
+// Whether cluster i prefers neighbour j, union area a, to bj, union area best (bj < 0: none yet): the least
+// area; the order (area, smaller index, larger index) is the same from both sides, so the least pair
+// overall is mutual and every round merges.
+__device__ __forceinline__ bool nearer(int i, float a, int j, float best, int bj) {
+  const int mn = min(i, j), mx = max(i, j), bn = min(i, bj), bx = max(i, bj);
+  return bj < 0 || a < best || (a == best && (mn < bn || (mn == bn && mx < bx)));
+}
+
+// The neighbour of cluster i (at sb[at]): of its 2 x kRadius candidates number q, q + lanes, ...
+__device__ __forceinline__ int nearest(const Box *sb, int at, int i, int count, int q, int lanes, float &best) {
   int bj = -1;
-  for (int d = 1; d <= kRadius; ++d) {
-#pragma unroll
-    for (int side = 0; side < 2; ++side) {
-      const int j = side ? i + d : i - d;
-      if (j < 0 || j >= count) continue;
-      const float a = half_area(join(sb[at], sb[at + (j - i)]));
-      const int mn = min(i, j), mx = max(i, j), bn = min(i, bj), bx = max(i, bj);
-      if (bj < 0 || a < best || (a == best && (mn < bn || (mn == bn && mx < bx)))) {
-        best = a;
-        bj = j;
-      }
+  best = INFINITY;
+  for (int o = q; o < 2 * kRadius; o += lanes) {
+    const int d = (o & 1) ? 1 + (o >> 1) : -1 - (o >> 1), j = i + d;
+    if (j < 0 || j >= count) continue;
+    const float a = half_area(join(sb[at], sb[at + d]));
+    if (nearer(i, a, j, best, bj)) {
+      best = a;
+      bj = j;
     }
   }
   return bj;
@@ -356,7 +359,9 @@ __global__ void __launch_bounds__(kPlocBlock) k_bvh_nearest(Build B) {
     }
     __syncthreads();
     const int i = base + (int)threadIdx.x;
-    if (i < count) B.nn[i] = force ? ((i ^ 1) < count ? (i ^ 1) : -1) : nearest(sb, (int)threadIdx.x + kRadius, i, count);
+    float best;
+    if (i < count)
+      B.nn[i] = force ? ((i ^ 1) < count ? (i ^ 1) : -1) : nearest(sb, (int)threadIdx.x + kRadius, i, count, 0, 1, best);
     __syncthreads();
   }
 }
@@ -489,22 +494,46 @@ __device__ void cluster_tail(const Build &B, TailShared &S, int count, uint32_t 
   __syncthreads();
   while (count > 1) {
     const bool force = S.force != 0;
-    for (int i = threadIdx.x; i < count; i += 1024)
-      S.nn[i] = force ? ((i ^ 1) < count ? (i ^ 1) : -1) : nearest(S.sb, i, i, count);
+    // up to 16 lanes share a cluster's candidates: the rounds of few clusters are many, and each waited for
+    // the 16 candidates one after another (36 clusters: 43 -> 24 us; 2,048: 148 -> 109)
+    int lanes = 1;
+    while (lanes < 2 * kRadius && 2 * lanes * count <= 1024) lanes *= 2;
+    for (int base = 0; base < count; base += 1024 / lanes) {
+      const int i = base + (int)threadIdx.x / lanes, q = (int)threadIdx.x & (lanes - 1);
+      float best = INFINITY;
+      int j = -1;
+      if (i < count) j = force ? ((i ^ 1) < count ? (i ^ 1) : -1) : nearest(S.sb, i, i, count, q, lanes, best);
+      for (int d = 1; d < lanes; d <<= 1) {
+        const float oa = __shfl_xor_sync(0xFFFFFFFFu, best, d);
+        const int oj = __shfl_xor_sync(0xFFFFFFFFu, j, d);
+        if (!force && oj >= 0 && nearer(i, oa, oj, best, j)) {
+          best = oa;
+          j = oj;
+        }
+      }
+      if (q == 0 && i < count) S.nn[i] = j;
+    }
     __syncthreads();
-    // two clusters per thread, in order
+    // two clusters per thread, in order; the warps beyond them only wait
+    const uint32_t warps = ((uint32_t)count + 63u) / 64u;
+    const bool busy = warp < warps;
     const int i0 = 2 * (int)threadIdx.x, i1 = i0 + 1;
     const int f0 = i0 < count ? fate(S.nn, i0) : 2, f1 = i1 < count ? fate(S.nn, i1) : 2;
-    const uint32_t k2 = (f0 != 2) + (f1 != 2), m2 = (f0 == 1) + (f1 == 1);
-    uint32_t ik = k2, im = m2;
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, ik, d), b = __shfl_up_sync(0xFFFFFFFFu, im, d);
-      if (lane >= (uint32_t)d) { ik += a; im += b; }
+    uint32_t k = 0u, m = 0u;
+    if (busy) {
+      const uint32_t k2 = (f0 != 2) + (f1 != 2), m2 = (f0 == 1) + (f1 == 1);
+      uint32_t ik = k2, im = m2;
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, ik, d), b = __shfl_up_sync(0xFFFFFFFFu, im, d);
+        if (lane >= (uint32_t)d) { ik += a; im += b; }
+      }
+      if (lane == 31u) { S.wk[warp] = ik; S.wm[warp] = im; }
+      k = ik - k2;
+      m = im - m2;
     }
-    if (lane == 31u) { S.wk[warp] = ik; S.wm[warp] = im; }
     __syncthreads();
-    uint32_t k = ik - k2, m = im - m2, tk = 0u, tm = 0u;
-    for (uint32_t w = 0; w < 32; ++w) {
+    uint32_t tk = 0u, tm = 0u;
+    for (uint32_t w = 0; w < warps; ++w) {
       if (w < warp) { k += S.wk[w]; m += S.wm[w]; }
       tk += S.wk[w];
       tm += S.wm[w];
@@ -571,6 +600,7 @@ struct Costs {
   int prims;
 };
 
+template <bool BLOCK>
 __device__ __forceinline__ Costs costs_of(const Build &B, int32_t id) {
   Costs r;
   if (id < B.n) {
@@ -579,21 +609,24 @@ __device__ __forceinline__ Costs costs_of(const Build &B, int32_t id) {
     r.prims = 1;
   } else {
     const Cut *q = B.cut + (id - B.n);
-    for (int k = 0; k < 7; ++k) r.c[k] = __ldcg(&q->c[k]);
-    r.prims = __ldcg(&q->prims);
+    for (int k = 0; k < 7; ++k) r.c[k] = BLOCK ? q->c[k] : __ldcg(&q->c[k]);
+    r.prims = BLOCK ? q->prims : __ldcg(&q->prims);
   }
   return r;
 }
 
-// Leaf i climbs; the second child to arrive at a node computes its cut.  Nothing waits.
-__device__ void climb(const Build &B, int64_t i) {
+// Leaf i climbs; the second child to arrive at a node computes its cut.  Nothing waits.  arrived: children of
+// inner node n + k whose cut is done.  BLOCK: all leaves climb in one block, which needs neither fences
+// nor loads beyond its SM.
+template <bool BLOCK>
+__device__ void climb(const Build &B, int64_t i, uint32_t *arrived) {
   int32_t at = B.n > 1 ? B.parent[i] : -1;
   while (at >= 0) {
-    __threadfence();
-    if (atomicAdd(&B.arrived[at - B.n], 1u) == 0u) break;
-    __threadfence();
+    if (BLOCK) __threadfence_block(); else __threadfence();
+    if (atomicAdd(&arrived[at - B.n], 1u) == 0u) break;
+    if (BLOCK) __threadfence_block(); else __threadfence();
     const BNode nd = B.node[at];
-    const Costs l = costs_of(B, nd.left), r = costs_of(B, nd.right);
+    const Costs l = costs_of<BLOCK>(B, nd.left), r = costs_of<BLOCK>(B, nd.right);
     const float area = half_area(nd.box);
     Cut c;
     c.pad = 0;
@@ -631,7 +664,7 @@ __device__ void climb(const Build &B, int64_t i) {
 
 __global__ void __launch_bounds__(128) k_bvh_cut(Build B) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < B.n; i += (int64_t)gridDim.x * blockDim.x)
-    climb(B, i);
+    climb<false>(B, i, B.arrived);
 }
 
 // ---- wide nodes ---------------------------------------------------------------------------
@@ -815,8 +848,10 @@ __global__ void __launch_bounds__(128) k_bvh_emit(Build B, int level) {
 // ---- small scenes -------------------------------------------------------------------------
 
 // Up to kSmall triangles: the whole build in one block, so that preparing a small scene costs one
-// launch (36 triangles: scene creation 0.33 -> 0.25 ms).  Same order, same clusters as the kernels
-// above.
+// launch (36 triangles: scene creation 0.33 -> 0.25 ms with the kernels above, warm 155 -> 118 us since
+// lanes share a cluster's candidates and the climb stays in the block).  It is a chain of short dependent
+// steps, bound by their latency: 36 triangles 55 us, 200 83, 2,048 239.  Same order, same clusters as
+// the kernels above.
 struct SmallShared {
   TailShared tail;
   uint64_t key[kSmall];
@@ -855,13 +890,15 @@ __global__ void __launch_bounds__(1024) k_bvh_small(Build B) {
       }
       __syncthreads();
     }
+  uint32_t *arrived = reinterpret_cast<uint32_t *>(S.key);  // the keys have been used
   for (uint32_t i = threadIdx.x; i < n; i += 1024) {
+    arrived[i] = 0u;
     S.tail.sb[i] = make_leaf(B, i, S.val[i]);
     S.tail.id[i] = (int32_t)i;
   }
   __syncthreads();
   cluster_tail(B, S.tail, (int)n, n);
-  for (uint32_t i = threadIdx.x; i < n; i += 1024) climb(B, i);
+  for (uint32_t i = threadIdx.x; i < n; i += 1024) climb<true>(B, i, arrived);
   __syncthreads();
   uint32_t w0 = 0u, w1 = 1u;
   int level = 0;
