@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(kGenBlock) k_generate(const __grid_constant__ 
 struct WideBlockShared {
   WideShared warp[kWideBlock / 32];
   WideTables tables;
-  uint32_t next;
+  uint32_t next, next_extend;
 };
 constexpr int kWideSmem = (int)sizeof(WideBlockShared);
 
@@ -320,20 +320,18 @@ __device__ __forceinline__ WideBlockShared &wide_shared() {
   extern __shared__ __align__(16) unsigned char wide_smem[];
   WideBlockShared &s = *reinterpret_cast<WideBlockShared *>(wide_smem);
   wide_tables(s.tables);
-  if (threadIdx.x == 0) s.next = 0u;
+  if (threadIdx.x == 0) s.next = s.next_extend = 0u;
   __syncthreads();
   return s;
 }
 
-template <bool COUNT, bool WIDE, bool SPH>
-__global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMinBlocks)
-    k_extend(const __grid_constant__ RenderArgs a, int b) {
+// closest hits of bounce b's rays, by the hierarchy
+template <bool COUNT, bool SPH>
+__device__ __forceinline__ void wide_extend(const RenderArgs &a, int b, WideBlockShared &ws, TraceCounts *c,
+                                            uint32_t &rays) {
   const uint32_t n = a.counters[kCtrRay + b];
   const float4 *qo = a.qo[b & 1], *qd = a.qd[b & 1];
   float4 *qhit = a.qhit;
-  TraceCounts c = {0, 0, 0, 0};
-  uint32_t rays = 0;
-  const bool single = a.njobs == 1;
   auto view_of = [&](uint32_t i) -> const SceneView & { return a.jobs[__float_as_int(qd[i].w)].view; };
   auto view0 = [&](uint32_t) -> const SceneView & { return a.view0; };
   auto load = [&](uint32_t i, Ray &r) {
@@ -343,20 +341,80 @@ __global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMi
     r.d = v3(d.x, d.y, d.z);
     r.tmax = INFINITY;
   };
+  auto store = [&](uint32_t i, bool hit, const Hit &h) {
+    qhit[i] = make_float4(hit ? h.t : INFINITY, __int_as_float(hit ? h.prim : -1), hit ? h.b1 : 0.0f, hit ? h.b2 : 0.0f);
+  };
+  WideShared &sh = ws.warp[threadIdx.x >> 5];
+  uint32_t *next = &ws.next_extend;
+  if (a.njobs == 1)
+    wide_trace<false, COUNT, SPH, true, true>(WideChunks(n), view0, n, load, store, SPH, sh, ws.tables, next, c, rays);
+  else
+    wide_trace<false, COUNT, SPH, false, true>(WideChunks(n), view_of, n, load, store, SPH, sh, ws.tables, next, c, rays);
+}
+
+// occlusion of bounce b's light samples, by the hierarchy; an occluded sample's slot is zeroed
+template <bool COUNT, bool SPH>
+__device__ __forceinline__ void wide_shadow(const RenderArgs &a, int b, WideBlockShared &ws, TraceCounts *c,
+                                            uint32_t &rays) {
+  const uint32_t n = a.counters[kCtrNee + b];
+  const float4 *so = a.so, *sd = a.sd;
+  float4 *slots = a.slots;
+  auto view_of = [&](uint32_t i) -> const SceneView & {
+    return a.jobs[a.path_job[__float_as_uint(so[i].w) / (uint32_t)a.nl_stride]].view;
+  };
+  auto view0 = [&](uint32_t) -> const SceneView & { return a.view0; };
+  auto load = [&](uint32_t i, Ray &r) {
+    float4 o = so[i], d = sd[i];
+    r.o = v3(o.x, o.y, o.z);
+    r.tmin = 0.0f;
+    r.d = v3(d.x, d.y, d.z);
+    r.tmax = d.w;
+  };
+  auto store = [&](uint32_t i, bool hit, const Hit &) {
+    if (hit) slots[__float_as_uint(so[i].w)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  };
+  WideShared &sh = ws.warp[threadIdx.x >> 5];
+  uint32_t *next = &ws.next;
+  if (a.njobs == 1)
+    wide_trace<true, COUNT, SPH, true, true>(WideChunks(n), view0, n, load, store, SPH, sh, ws.tables, next, c, rays);
+  else
+    wide_trace<true, COUNT, SPH, false, true>(WideChunks(n), view_of, n, load, store, SPH, sh, ws.tables, next, c, rays);
+}
+
+// Bounce b + 1's closest hits and bounce b's occlusion queries, which do not depend on each other: one launch,
+// and one end at which warps wait for the block's last rays, instead of two of each.
+template <bool SPH>
+__global__ void __launch_bounds__(kWideBlock, 1) k_traverse(const __grid_constant__ RenderArgs a, int b) {
+  TraceCounts c = {0, 0, 0, 0};
+  uint32_t rays = 0;
+  WideBlockShared &ws = wide_shared();
+  wide_extend<false, SPH>(a, b + 1, ws, &c, rays);
+  wide_shadow<false, SPH>(a, b, ws, &c, rays);
+}
+
+template <bool COUNT, bool WIDE, bool SPH>
+__global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMinBlocks)
+    k_extend(const __grid_constant__ RenderArgs a, int b) {
+  TraceCounts c = {0, 0, 0, 0};
+  uint32_t rays = 0;
   if constexpr (WIDE) {
-    auto store = [&](uint32_t i, bool hit, const Hit &h) {
-      qhit[i] = make_float4(hit ? h.t : INFINITY, __int_as_float(hit ? h.prim : -1), hit ? h.b1 : 0.0f, hit ? h.b2 : 0.0f);
-    };
-    WideBlockShared &ws = wide_shared();
-    WideShared &sh = ws.warp[threadIdx.x >> 5];
-    if (single) wide_trace<false, COUNT, SPH, true, true>(WideChunks(n), view0, n, load, store, SPH, sh, ws.tables, &ws.next, &c, rays);
-    else wide_trace<false, COUNT, SPH, false, true>(WideChunks(n), view_of, n, load, store, SPH, sh, ws.tables, &ws.next, &c, rays);
+    wide_extend<COUNT, SPH>(a, b, wide_shared(), &c, rays);
   } else {
+    const float4 *qo = a.qo[b & 1], *qd = a.qd[b & 1];
+    float4 *qhit = a.qhit;
+    auto view_of = [&](uint32_t i) -> const SceneView & { return a.jobs[__float_as_int(qd[i].w)].view; };
+    auto load = [&](uint32_t i, Ray &r) {
+      float4 o = qo[i], d = qd[i];
+      r.o = v3(o.x, o.y, o.z);
+      r.tmin = 0.0f;
+      r.d = v3(d.x, d.y, d.z);
+      r.tmax = INFINITY;
+    };
     auto store = [&](uint32_t i, bool hit, const TravState &st) {
       qhit[i] = make_float4(hit ? st.best : INFINITY, __int_as_float(hit ? st.best_prim : -1), hit ? st.bb1 : 0.0f,
                             hit ? st.bb2 : 0.0f);
     };
-    grid_trace<false, COUNT, SPH>(view_of, nullptr, 0, n, load, store, &c, rays);
+    grid_trace<false, COUNT, SPH>(view_of, nullptr, 0, a.counters[kCtrRay + b], load, store, &c, rays);
   }
   if (COUNT && rays + c.nodes + c.tris) {
     atomicAdd(&a.tcount[0], (unsigned long long)c.nodes);
@@ -377,13 +435,15 @@ __device__ __forceinline__ V3 fold_slots(const RenderArgs &a, int nl, int64_t p,
   return L;
 }
 
-// Threads of a shading block, and the rays that it takes at a time; four blocks per SM (64 registers; the
-// kernel's natural 125 and the spills of 48 both measure slower).
+// Threads of a shading block, and the rays that it takes at a time.
 constexpr int kShadeTile = 256;
 // Blocks of the shade kernels per SM: three leave a thread 80 registers and half the spills of 64.  Shading per
 // frame at 3 / 4 / 2 blocks: mid scene 21.3 / 21.8 / 24.9 ms, plain box 0.302 / 0.332 / 0.327, terrain
 // 3.18 / 3.30 / 3.47, textured 0.99 / 1.00 / 1.12.
 constexpr int kShadeMinBlocks = 3;
+
+// Light samples of a wave up to which traversals share launches (k_traverse)
+constexpr int64_t kMergeMaxSlots = (int64_t)1 << 22;
 
 // What a shading block keeps in shared memory: per warp the shadow rays that wait for a full 32 (or, while
 // the block traces its own rays, the traversal's records), the counts and the order of the tile's
@@ -785,35 +845,28 @@ __global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(const __g
 template <bool COUNT, bool WIDE, bool SPH>
 __global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMinBlocks)
     k_shadow(const __grid_constant__ RenderArgs a, int b) {
-  const uint32_t n = a.counters[kCtrNee + b];
-  const float4 *so = a.so, *sd = a.sd;
-  float4 *slots = a.slots;
   TraceCounts c = {0, 0, 0, 0};
   uint32_t rays = 0;
-  const bool single = a.njobs == 1;
-  auto view_of = [&](uint32_t i) -> const SceneView & {
-    if (single) return a.jobs[0].view;
-    const uint32_t slot = __float_as_uint(so[i].w);
-    return a.jobs[a.path_job[slot / (uint32_t)a.nl_stride]].view;
-  };
-  auto view0 = [&](uint32_t) -> const SceneView & { return a.view0; };
-  auto load = [&](uint32_t i, Ray &r) {
-    float4 o = so[i], d = sd[i];
-    r.o = v3(o.x, o.y, o.z);
-    r.tmin = 0.0f;
-    r.d = v3(d.x, d.y, d.z);
-    r.tmax = d.w;
-  };
-  auto store = [&](uint32_t i, bool hit, const auto &) {
-    if (hit) slots[__float_as_uint(so[i].w)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  };
   if constexpr (WIDE) {
-    WideBlockShared &ws = wide_shared();
-    WideShared &sh = ws.warp[threadIdx.x >> 5];
-    if (single) wide_trace<true, COUNT, SPH, true, true>(WideChunks(n), view0, n, load, store, SPH, sh, ws.tables, &ws.next, &c, rays);
-    else wide_trace<true, COUNT, SPH, false, true>(WideChunks(n), view_of, n, load, store, SPH, sh, ws.tables, &ws.next, &c, rays);
+    wide_shadow<COUNT, SPH>(a, b, wide_shared(), &c, rays);
   } else {
-    grid_trace<true, COUNT, SPH>(view_of, nullptr, 0, n, load, store, &c, rays);
+    const float4 *so = a.so, *sd = a.sd;
+    float4 *slots = a.slots;
+    auto view_of = [&](uint32_t i) -> const SceneView & {
+      if (a.njobs == 1) return a.jobs[0].view;
+      return a.jobs[a.path_job[__float_as_uint(so[i].w) / (uint32_t)a.nl_stride]].view;
+    };
+    auto load = [&](uint32_t i, Ray &r) {
+      float4 o = so[i], d = sd[i];
+      r.o = v3(o.x, o.y, o.z);
+      r.tmin = 0.0f;
+      r.d = v3(d.x, d.y, d.z);
+      r.tmax = d.w;
+    };
+    auto store = [&](uint32_t i, bool hit, const TravState &) {
+      if (hit) slots[__float_as_uint(so[i].w)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    };
+    grid_trace<true, COUNT, SPH>(view_of, nullptr, 0, a.counters[kCtrNee + b], load, store, &c, rays);
   }
   if (COUNT && rays + c.nodes + c.tris) {
     atomicAdd(&a.tcount[4], (unsigned long long)c.nodes);
@@ -1202,6 +1255,8 @@ static std::vector<CarveoutKernel> carveout_kernels() {
           {(const void *)k_shadow<false, true, true>, kWideBlock, kWideSmem},
           {(const void *)k_shadow<true, true, false>, kWideBlock, kWideSmem},
           {(const void *)k_shadow<true, true, true>, kWideBlock, kWideSmem},
+          {(const void *)k_traverse<false>, kWideBlock, kWideSmem},
+          {(const void *)k_traverse<true>, kWideBlock, kWideSmem},
           {(const void *)k_extend<false, false, true>, kBlock, 0},
           {(const void *)k_extend<true, false, true>, kBlock, 0},
           {(const void *)k_shadow<false, false, true>, kBlock, 0},
@@ -1517,6 +1572,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
   }
   auto kext = !wide ? k_extend<COUNT, false, true> : sph ? k_extend<COUNT, true, true> : k_extend<COUNT, true, false>;
   auto kshw = !wide ? k_shadow<COUNT, false, true> : sph ? k_shadow<COUNT, true, true> : k_shadow<COUNT, true, false>;
+  auto ktrv = sph ? k_traverse<true> : k_traverse<false>;
   const int tb = wide ? kWideBlock : kBlock;
   const size_t tsm = wide ? (size_t)kWideSmem : 0;
   MGPU_CUDA(kernel_attributes());
@@ -1616,14 +1672,24 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
       run_whole(wv.npaths, 0);
       b = max_b;
     }
+    // From the second bounce on, a bounce's occlusion queries and the next one's closest hits in one launch, where
+    // they are few enough that the ends of the launches count (per frame, apart against together, by the
+    // wave's light samples: 2.9 M, 300,000 triangles to depth 8, 2 passes 2.93 / 2.66 ms; 1.0 M in the
+    // plain box 0.866 / 0.840; 2.2 M, spheres without a depth cap 1.62 / 1.58; but 5.3 M textured 2.93 / 2.97 and
+    // 64 M paths of the mid scene 109.2 / 112.0: two traversals in one kernel leave each fewer
+    // registers, and the first bounce is the largest).  Per-kernel timing keeps them apart.
+    const bool merge = wide && !COUNT && !pf.enabled && wv.npaths * wv.nl_stride <= kMergeMaxSlots;
     while (b < max_b && err == cudaSuccess) {
       // with a fixed depth cap every bounce is launched blind; without one, check the live
       // count every 4 bounces and stop when the wave has drained
       int chunk = wv.unlimited ? std::min(4, max_b - b) : max_b;
       for (int k = 0; k < chunk; ++k, ++b) {
-        m = pf.begin(kProfExtend, st);
-        kext<<<g_ext, tb, tsm, st>>>(a, b);
-        pf.end(m, st);
+        if (k == 0 || b < 2 || !merge) {
+          m = pf.begin(kProfExtend, st);
+          kext<<<g_ext, tb, tsm, st>>>(a, b);
+          pf.end(m, st);
+          ++launches;
+        }
         m = pf.begin(kProfShade, st);
         kshd<<<g_sha, kShadeTile, sizeof(ShadeShared), st>>>(a, b, 0);
         pf.end(m, st);
@@ -1639,9 +1705,10 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
           launches += 3;
         }
         m = pf.begin(kProfShadow, st);
-        kshw<<<g_shw, tb, tsm, st>>>(a, b);
+        if (merge && b > 0 && k + 1 < chunk) ktrv<<<g_ext, tb, tsm, st>>>(a, b);
+        else kshw<<<g_shw, tb, tsm, st>>>(a, b);
         pf.end(m, st);
-        launches += 3;
+        launches += 2;
       }
       if (!wv.unlimited) break;
       err = cudaMemcpyAsync(w->h_counters, w->counters + kCtrRay + b, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);

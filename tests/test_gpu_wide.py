@@ -224,3 +224,37 @@ def test_planes_at_the_roundings_of_16_bit_floats(cuda, scale, nudge):
     same = np.all(kd.view(np.uint32) == wide.view(np.uint32), axis=1)
     assert same.all(), (int((~same).sum()), rays[~same][:2], kd[~same][:2], wide[~same][:2])
     assert np.array_equal(gpu_any(cuda, ds, rays) != 0, kd[:, 1].view(np.int32) >= 0)
+
+
+@pytest.mark.parametrize("depth,bins,nds", [(2, False, 1), (3, False, 4), (0, False, 1), (7, True, 1)])
+@pytest.mark.parametrize("kind", ["random", "balls", "batch"])
+def test_traversals_that_share_a_launch_equal_separate_ones(cuda, kind, depth, bins, nds):
+    # small waves trace a bounce's closest hits with the occlusion queries of the one before; per-kernel timing
+    # keeps the launches apart
+    scenes = [_scene("random"), scenegen.plain(4), _scene("n300")] if kind == "batch" else [_scene(kind)]
+    ds = [pt.DeviceScene(s, pt.Accel(s)) for s in scenes]
+    st = pt.RenderSettings(83, 61, 3, no_direct_samples=nds, max_depth=depth, rr_start_depth=2, seed=3)
+    out, stats = [], []
+    try:
+        pt.tune("whole_paths", 0)
+        if bins:
+            pt.tune("bin_min_paths", 0)
+        for timed in (False, True):
+            films = [pt.Film(83, 61) for _ in ds]
+            pt.profile_enable(timed)
+            if kind == "batch":
+                b = pt.Batch()
+                for d, f in zip(ds, films):
+                    b.add(d, st, f)
+                b.render()
+            else:
+                pt.render(ds[0], st, films[0])
+            r = pt.render_stats()
+            out.append([f.raw() for f in films])
+            stats.append((r["extension_rays"], r["shadow_rays"], r["bounces"], r["paths"]))
+    finally:
+        pt.profile_enable(False)
+        pt.tune("whole_paths", -1)
+        pt.tune("bin_min_paths", 1 << 25)
+    assert all(np.array_equal(x.view(np.uint32), y.view(np.uint32)) for x, y in zip(*out))
+    assert stats[0] == stats[1]
