@@ -242,6 +242,15 @@ __device__ __forceinline__ uint32_t ext_key(const JobArgs &J, V3 o, V3 d) {
   return (oct << (kBinBits - 3)) | (morton15(J, o) >> (18 - kBinBits));
 }
 
+// The kernels of a small wave are launched so that each may start while the one before it drains (programmatic
+// stream serialization): every thread of every kernel calls chain() before it touches memory that another
+// kernel writes; it waits there until the kernel before has ended and its writes are visible.  Without
+// that launch attribute it returns at once.
+__device__ __forceinline__ void chain() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ---------------------------------------------------------------------------------------
 // generate: camera rays for every path of the wave (RayTracer::sample, RayTracer.cpp:19-30;
 // SuperSampleGenerator strata, SuperSampleGenerator.cpp:60-90)
@@ -253,6 +262,7 @@ constexpr int kGenBlock = 256;
 
 __global__ void __launch_bounds__(kGenBlock) k_generate(const __grid_constant__ RenderArgs a) {
   __shared__ uint32_t cnt[kGenBlock / 32], first;
+  chain();
   const int64_t n = a.npaths;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   if (a.dense && blockIdx.x == 0 && threadIdx.x == 0) a.counters[kCtrRay] = (uint32_t)n;
@@ -321,6 +331,7 @@ __device__ __forceinline__ WideBlockShared &wide_shared() {
   WideBlockShared &s = *reinterpret_cast<WideBlockShared *>(wide_smem);
   wide_tables(s.tables);
   if (threadIdx.x == 0) s.next = s.next_extend = 0u;
+  chain();
   __syncthreads();
   return s;
 }
@@ -400,6 +411,7 @@ __global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMi
   if constexpr (WIDE) {
     wide_extend<COUNT, SPH>(a, b, wide_shared(), &c, rays);
   } else {
+    chain();
     const float4 *qo = a.qo[b & 1], *qd = a.qd[b & 1];
     float4 *qhit = a.qhit;
     auto view_of = [&](uint32_t i) -> const SceneView & { return a.jobs[__float_as_int(qd[i].w)].view; };
@@ -442,8 +454,8 @@ constexpr int kShadeTile = 256;
 // 3.18 / 3.30 / 3.47, textured 0.99 / 1.00 / 1.12.
 constexpr int kShadeMinBlocks = 3;
 
-// Light samples of a wave up to which traversals share launches (k_traverse)
-constexpr int64_t kMergeMaxSlots = (int64_t)1 << 22;
+// Light samples of a wave up to which its launches are chained, and traversals share them
+constexpr int64_t kSmallWaveSlots = (int64_t)1 << 22;
 
 // What a shading block keeps in shared memory: per warp the shadow rays that wait for a full 32 (or, while
 // the block traces its own rays, the traversal's records), the counts and the order of the tile's
@@ -585,6 +597,8 @@ __global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(const __g
                                                                        uint32_t whole) {
   extern __shared__ __align__(16) unsigned char shade_smem[];
   ShadeShared &sh = *reinterpret_cast<ShadeShared *>(shade_smem);
+  if (WHOLE) wide_tables(sh.tables);
+  chain();
   uint32_t n = a.counters[kCtrRay + b], base = blockIdx.x * kShadeTile;
   const uint32_t stride = gridDim.x * kShadeTile, total = n;
   const int b0 = b;
@@ -595,7 +609,6 @@ __global__ void __launch_bounds__(kShadeTile, kShadeMinBlocks) k_shade(const __g
   if (WHOLE) {
     base = blockIdx.x * whole;
     if (base >= total) return;
-    wide_tables(sh.tables);
     out = base;
     n = min(base + whole, total);
     next_ctr = &sh.rays;
@@ -850,6 +863,7 @@ __global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMi
   if constexpr (WIDE) {
     wide_shadow<COUNT, SPH>(a, b, wide_shared(), &c, rays);
   } else {
+    chain();
     const float4 *so = a.so, *sd = a.sd;
     float4 *slots = a.slots;
     auto view_of = [&](uint32_t i) -> const SceneView & {
@@ -980,7 +994,8 @@ __device__ void splat(const JobArgs &J, int x, int y, int s, V3 L) {
     }
 }
 
-__global__ void __launch_bounds__(kBlock) k_accumulate(RenderArgs a) {
+__global__ void __launch_bounds__(kBlock) k_accumulate(const __grid_constant__ RenderArgs a) {
+  chain();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     unsigned long long ext = 0, bounces = 0, sh = 0;
     for (int b = 0; b < a.max_b; ++b) {
@@ -1320,6 +1335,22 @@ static int grid_for(const void *kern, size_t smem, int block = kBlock) {
   return device_sm_count() * per_sm;
 }
 
+// A launch that, if chained, may overlap the end of the kernel before it on the stream (chain()).
+template <class... P, class... A>
+static void launch(bool chained, void (*kern)(P...), unsigned grid, int block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3((unsigned)block);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = chained ? 1 : 0;
+  cudaLaunchKernelEx(&c, kern, static_cast<P>(args)...);
+}
+
 static Camera make_camera(const float *c) {
   // ThinLensCamera::setOrientation (ThinLensCamera.cpp:241-259) and _computeMatrix (:204-210)
   double eye[3] = {c[0], c[1], c[2]}, look[3] = {c[3], c[4], c[5]}, up[3] = {c[6], c[7], c[8]};
@@ -1646,6 +1677,10 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
     k_generate<<<g_gen, kGenBlock, 0, st>>>(a);
     pf.end(m, st);
     ++launches;
+    // In waves of few light samples the starts and ends of launches count (851 paths 122 -> 112 us, 30,400 without
+    // allocation 424 -> 384, two passes of 0.97 M paths 2.65 -> 2.58 ms); in larger ones kernels that
+    // overlap gain nothing (ten scenes, 10 M paths: 4.69 / 4.68) or lose (textured, 5.3 M: 2.925 / 2.95).
+    const bool chained = wv.npaths * wv.nl_stride <= kSmallWaveSlots;
     auto kshd = surf ? k_shade<true, false> : k_shade<false, false>;
     auto kshp = surf ? k_shade<true, true> : k_shade<false, true>;
     int b = 0;
@@ -1664,7 +1699,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
       RenderArgs w1 = a;
       w1.bin_ext = 0;  // a block's next rays stay with the block
       const int mk = pf.begin(kProfShade, st);
-      kshp<<<(unsigned)((rays + per - 1) / per), kShadeTile, sizeof(ShadeShared), st>>>(w1, from, per);
+      launch(chained, kshp, (unsigned)((rays + per - 1) / per), kShadeTile, sizeof(ShadeShared), st, w1, from, per);
       pf.end(mk, st);
       ++launches;
     };
@@ -1678,7 +1713,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
     // plain box 0.866 / 0.840; 2.2 M, spheres without a depth cap 1.62 / 1.58; but 5.3 M textured 2.93 / 2.97 and
     // 64 M paths of the mid scene 109.2 / 112.0: two traversals in one kernel leave each fewer
     // registers, and the first bounce is the largest).  Per-kernel timing keeps them apart.
-    const bool merge = wide && !COUNT && !pf.enabled && wv.npaths * wv.nl_stride <= kMergeMaxSlots;
+    const bool merge = chained && wide && !COUNT && !pf.enabled;
     while (b < max_b && err == cudaSuccess) {
       // with a fixed depth cap every bounce is launched blind; without one, check the live
       // count every 4 bounces and stop when the wave has drained
@@ -1686,12 +1721,12 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
       for (int k = 0; k < chunk; ++k, ++b) {
         if (k == 0 || b < 2 || !merge) {
           m = pf.begin(kProfExtend, st);
-          kext<<<g_ext, tb, tsm, st>>>(a, b);
+          launch(chained, kext, g_ext, tb, tsm, st, a, b);
           pf.end(m, st);
           ++launches;
         }
         m = pf.begin(kProfShade, st);
-        kshd<<<g_sha, kShadeTile, sizeof(ShadeShared), st>>>(a, b, 0);
+        launch(chained, kshd, g_sha, kShadeTile, sizeof(ShadeShared), st, a, b, 0u);
         pf.end(m, st);
         if (a.bin_ext && b + 1 < max_b) {
           const int nx = (b + 1) & 1;
@@ -1705,8 +1740,8 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
           launches += 3;
         }
         m = pf.begin(kProfShadow, st);
-        if (merge && b > 0 && k + 1 < chunk) ktrv<<<g_ext, tb, tsm, st>>>(a, b);
-        else kshw<<<g_shw, tb, tsm, st>>>(a, b);
+        if (merge && b > 0 && k + 1 < chunk) launch(chained, ktrv, g_ext, tb, tsm, st, a, b);
+        else launch(chained, kshw, g_shw, tb, tsm, st, a, b);
         pf.end(m, st);
         launches += 2;
       }
@@ -1720,7 +1755,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
       }
     }
     m = pf.begin(kProfAccumulate, st);
-    k_accumulate<<<g_acc, kBlock, 0, st>>>(a);
+    launch(chained, k_accumulate, g_acc, kBlock, 0, st, a);
     pf.end(m, st);
     ++launches;
     if (err == cudaSuccess) err = cudaGetLastError();
