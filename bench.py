@@ -834,6 +834,7 @@ def run_profile_case(args):
     ds = pt.DeviceScene(s, pt.Accel(s))
     film = pt.Film(512, 512)
     st = pt.RenderSettings(512, 512, 4, max_depth=MAX_DEPTH, rr_start_depth=RR_START, seed=SEED)
+    pt.profile_enable(True)  # closest hits and occlusion queries in launches of their own, as in a large wave
     for _ in range(2):
         pt.render(ds, st, film)
     torch.cuda.synchronize()

@@ -1080,9 +1080,9 @@ struct Tuning {
   std::atomic<int> persistent{0}, coop_leaf{3}, trav_block{256};
   std::atomic<int> bin_extension{1};  // counting-sort extension rays by (octant, origin cell)
   // waves of fewer paths, and scenes of fewer than kBinMinTris triangles, skip the sort: it pays where
-  // tree and triangles are well beyond the L1s (64 M paths, sorted against not: 1 M triangles 117.5 / 120.5 ms,
-  // 300 k 81.8 / 82.3, 150 k 60.2 / 60.1, 50 k 31.8 / 30.8, 36 triangles 68.9 / 57.3; 16 M paths of 1 M
-  // triangles 30.95 / 31.02).  0: sort every wave.
+  // tree and triangles are well beyond the L1s (64 M paths, sorted against not: 2 M triangles 318.5 / 326.5 ms,
+  // 1 M 103.8 / 107.4, 300 k 70.3 / 71.2; with 8-bit nodes 150 k 60.2 / 60.1, 50 k 31.8 / 30.8, 36 triangles
+  // 68.9 / 57.3; 16 M paths of 2 M 82.0 / 83.6, 1 M 27.7 / 27.9, 300 k 18.8 / 18.6).  0: sort every wave.
   std::atomic<int64_t> bin_min_paths{(int64_t)1 << 25};
   // a sort of the shadow rays cost more than it saved and is no more (1 M triangles, 64 M paths: 6.1 ms of sorting
   // and key writes for 3.5 of traversal); kept for callers that set and read it back
@@ -1523,7 +1523,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
   for (const Job &j : jobs)
     nl_max = std::max(nl_max, std::max(1, job_args(j).nl_slots));
   // automatic wave: the largest power of two up to 2^26 paths whose workspace fits 40 GB (larger
-  // waves mean fewer bounce tails: mid frame 226 / 236 / 241 Mpaths/s at 2^24 / 2^25 / 2^26)
+  // waves mean fewer bounce tails: mid frame 606 / 634 / 647 Mpaths/s at 2^24 / 2^25 / 2^26)
   int64_t wave = wave_req;
   if (wave <= 0) {
     const double per_path = (double)workspace_bytes((int64_t)1 << 20, ((int64_t)1 << 20) * nl_max, 1) / (1 << 20);
