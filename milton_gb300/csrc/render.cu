@@ -996,18 +996,27 @@ __device__ void splat(const JobArgs &J, int x, int y, int s, V3 L) {
 
 __global__ void __launch_bounds__(kBlock) k_accumulate(const __grid_constant__ RenderArgs a) {
   chain();
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  // the wave's counts, by one warp (one thread took 43 us over the 1,024 bounces of a wave without a depth cap:
+  // analytic spheres, 1.08 M paths, 65 -> 22 us)
+  if (blockIdx.x == 0 && threadIdx.x < 32) {
     unsigned long long ext = 0, bounces = 0, sh = 0;
-    for (int b = 0; b < a.max_b; ++b) {
+    for (int b = threadIdx.x; b < a.max_b; b += 32) {
       uint32_t c = a.counters[kCtrRay + b];
       ext += c;
       bounces += c ? 1ull : 0ull;
       sh += a.counters[kCtrNee + b];
     }
-    a.stats[0] += ext;
-    a.stats[1] += sh;
-    a.stats[2] += a.counters[kCtrTrunc];
-    a.stats[3] += bounces;
+    for (int d = 16; d > 0; d >>= 1) {
+      ext += __shfl_xor_sync(0xFFFFFFFFu, ext, d);
+      sh += __shfl_xor_sync(0xFFFFFFFFu, sh, d);
+      bounces += __shfl_xor_sync(0xFFFFFFFFu, bounces, d);
+    }
+    if (threadIdx.x == 0) {
+      a.stats[0] += ext;
+      a.stats[1] += sh;
+      a.stats[2] += a.counters[kCtrTrunc];
+      a.stats[3] += bounces;
+    }
   }
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < a.nslots; q += stride) {
