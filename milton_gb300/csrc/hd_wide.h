@@ -44,13 +44,13 @@ constexpr uint32_t kWideRootBits = 0x101u;  // pending slots and inner mask of t
 // neighbours in the (sorted) queue and share its L1: mid frame, traversal 117 ms in blocks of 128,
 // 114 / 108 / 102 ms in blocks of 256 / 512 / 1024.
 constexpr int kWideBlock = 1024;
-// Rays that a block takes at a time; its warps take them 32 by 32 as they finish (mid frame: 97.0,
-// 96.3, 98.2, 101.1 ms at 1024, 512, 2048, 4096 against 102 in fixed grid-stride rounds; on the
-// present kernels 86.4, 86.0, 85.6 at 1024, 512, 256).
+// Rays that a block takes at a time; its warps take them 32 by 32 as they finish (against fixed grid-stride
+// rounds the mid frame's traversal went from 102 to 96 ms; now, whole frame: 103.7, 104.0, 104.3 ms at 128, 256,
+// 512, and 1 M ray queries 0.215, 0.211, 0.229).
 constexpr uint32_t kWideChunk = 256u;
 // Triangle tests waiting after a node step that are worth a round of their own: a full queue (32) keeps
 // every lane busy but lets the rays go on with a stale closest t (mid closest hits: 49.9 / 46.9 /
-// 46.5 ms at 32 / 16 / 8).
+// 46.5 ms at 32 / 16 / 8; now flat from 4 to 16, and 2 % slower at 24 in the textured scene).
 constexpr uint32_t kWideFlush = 8u;
 
 // Box tests are conservative.  The planes are rounded outward when they are stored.  What rounds relative
