@@ -242,7 +242,7 @@ __device__ __forceinline__ uint32_t ext_key(const JobArgs &J, V3 o, V3 d) {
   return (oct << (kBinBits - 3)) | (morton15(J, o) >> (18 - kBinBits));
 }
 
-// The kernels of a small wave are launched so that each may start while the one before it drains (programmatic
+// Most kernels of a small wave are launched so that they may start while the one before it drains (programmatic
 // stream serialization): every thread of every kernel calls chain() before it touches memory that another
 // kernel writes; it waits there until the kernel before has ended and its writes are visible.  Without
 // that launch attribute it returns at once.
@@ -1677,6 +1677,8 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
     a.max_b = wv.max_b;
     a.seq = sph ? 1 : 0;
     const int max_b = wv.max_b;
+    bool splats = false;  // a chunk's film has a reconstruction filter
+    for (const JobArgs &c : wv.chunks) splats = splats || c.film_fx != nullptr;
     bool surf = false;  // a chunk's scene has image maps, a background or analytic spheres
     for (const JobArgs &c : wv.chunks)
       surf = surf || c.texrec != nullptr || c.bg_tex != 0 || c.bg_le[0] != 0.0f || c.bg_le[1] != 0.0f ||
@@ -1686,9 +1688,12 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
     k_generate<<<g_gen, kGenBlock, 0, st>>>(a);
     pf.end(m, st);
     ++launches;
-    // In waves of few light samples the starts and ends of launches count (851 paths 122 -> 112 us, 30,400 without
-    // allocation 424 -> 384, two passes of 0.97 M paths 2.65 -> 2.58 ms); in larger ones kernels that
-    // overlap gain nothing (ten scenes, 10 M paths: 4.69 / 4.68) or lose (textured, 5.3 M: 2.925 / 2.95).
+    // In waves of few light samples the starts and ends of launches count (851 paths 118 -> 111 us, 30,400 without
+    // allocation 419 -> 386, two passes of 0.97 M paths 2.65 -> 2.585 ms); in larger ones kernels that overlap
+    // gain nothing (ten scenes, 10 M paths: 4.69 / 4.68) or lose (textured, 5.3 M: 2.925 / 2.95).  Blocks that come
+    // early fill the first SMs that come free instead of spreading over all, so a kernel whose work is in its
+    // first few blocks is not chained: shading (plain box 838 / 827 us chained / not, spheres 1.561 / 1.541 ms) and
+    // accumulation through a reconstruction filter (141 x 37 pixels of 64 samples 1.29 / 0.49 ms).
     const bool chained = wv.npaths * wv.nl_stride <= kSmallWaveSlots;
     auto kshd = surf ? k_shade<true, false> : k_shade<false, false>;
     auto kshp = surf ? k_shade<true, true> : k_shade<false, true>;
@@ -1735,7 +1740,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
           ++launches;
         }
         m = pf.begin(kProfShade, st);
-        launch(chained, kshd, g_sha, kShadeTile, sizeof(ShadeShared), st, a, b, 0u);
+        kshd<<<g_sha, kShadeTile, sizeof(ShadeShared), st>>>(a, b, 0);
         pf.end(m, st);
         if (a.bin_ext && b + 1 < max_b) {
           const int nx = (b + 1) & 1;
@@ -1764,7 +1769,7 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
       }
     }
     m = pf.begin(kProfAccumulate, st);
-    launch(chained, k_accumulate, g_acc, kBlock, 0, st, a);
+    launch(chained && !splats, k_accumulate, g_acc, kBlock, 0, st, a);
     pf.end(m, st);
     ++launches;
     if (err == cudaSuccess) err = cudaGetLastError();
