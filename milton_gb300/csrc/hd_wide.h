@@ -59,6 +59,18 @@ constexpr uint32_t kWideFlush = 8u;
 // 2 M) -- is covered by moving every plane outward by 1.5 x 2^-20 M, folded into the ray's constants.
 constexpr float kWideEps = 1.5f / 1048576.0f;
 
+// A direction component below 2^-40 of the ray's largest is taken as that in the box tests: the reciprocal of a
+// smaller one, multiplied by the origin, overflows, and boxes that the ray passes were missed (components
+// of 1e-38; and where the reciprocal itself is infinite every box was met: 200,000 rays 0.3 -> 611 ms).  It is
+// still conservative: through the scene such a ray moves at most 2^-38 M along that axis, and the planes
+// are 2^-19 M farther out.
+constexpr float kWideLeast = 1.0f / 1099511627776.0f;
+// ... and below this part of it the ray is one with a zero component to the kd-tree's rounding (kWideTie)
+constexpr float kWideZero = 1.0e-30f;
+// What the box tests multiply and add lies between 2^-20 and 2^41 times M / (largest component); where M / it is
+// beyond these, products overflow or lose bits below the normal numbers, and the kd-tree answers the ray.
+constexpr float kWideScaleMin = 1.0e-25f, kWideScaleMax = 1.0e25f;
+
 #if defined(__CUDACC__)
 
 // one half of w (which: the permute's selector) as the upper half of a float
@@ -192,8 +204,8 @@ __device__ __forceinline__ float wide_unorder(uint32_t u) {
 // once the best hit lies inside the current cell, widened by 2^-18), so such a ray is traced again
 // there.  It is a ray through an exact edge, or a surface laid on another: one in some 10^8 on scenes
 // without coincident surfaces.
-// So is a ray with a zero direction component: one that lies in a split plane sees only the cells on one
-// side of it in the kd-tree.
+// So is a ray with a zero direction component, or as good as zero: one that lies in a split plane sees only
+// the cells on one side of it in the kd-tree.
 constexpr float kWideTie = 1.0f / 131072.0f;
 
 // The kd-tree's answer for one ray: closest hit, or any (h.prim >= 0).  seq: a leaf's triangles one after
@@ -290,17 +302,24 @@ struct WideWarp {
       sh.sphere[lane] = sphere;
     }
     active = s.ntri > 0 && !(ANY && sphere >= 0);
-    kd = active && (r.d.x == 0.0f || r.d.y == 0.0f || r.d.z == 0.0f);
+    const V3 o = r.o - v3(s.wcentre[0], s.wcentre[1], s.wcentre[2]);
+    float m = fmaxf(fmaxf(s.wextent, fabsf(o.x)), fmaxf(fabsf(o.y), fabsf(o.z)));
+    const float dmax = fmaxf(fabsf(r.d.x), fmaxf(fabsf(r.d.y), fabsf(r.d.z))), scale = m / dmax;
+    const float zero = dmax * kWideZero;
+    kd = active && (fabsf(r.d.x) <= zero || fabsf(r.d.y) <= zero || fabsf(r.d.z) <= zero ||
+                    !(scale >= kWideScaleMin && scale <= kWideScaleMax));
     active = active && !kd;
     if (active) {
-      w.inv = v3(1.0f / r.d.x, 1.0f / r.d.y, 1.0f / r.d.z);
       float t0, t1;
-      active = clip_root(s, r, w.inv, t0, t1) && fmaxf(t0, r.tmin) <= fminf(t1, r.tmax);
+      active = clip_root(s, r, v3(1.0f / r.d.x, 1.0f / r.d.y, 1.0f / r.d.z), t0, t1) &&
+               fmaxf(t0, r.tmin) <= fminf(t1, r.tmax);
     }
     if (active) {
       const RayPre pre = precompute(r);
-      const V3 o = r.o - v3(s.wcentre[0], s.wcentre[1], s.wcentre[2]);
-      const float m = fmaxf(fmaxf(s.wextent, fabsf(o.x)), fmaxf(fabsf(o.y), fabsf(o.z))) * kWideEps;
+      const float least = dmax * kWideLeast;
+      w.inv = v3(1.0f / copysignf(fmaxf(fabsf(r.d.x), least), r.d.x), 1.0f / copysignf(fmaxf(fabsf(r.d.y), least), r.d.y),
+                 1.0f / copysignf(fmaxf(fabsf(r.d.z), least), r.d.z));
+      m *= kWideEps;
       const V3 e = v3(m * fabsf(w.inv.x), m * fabsf(w.inv.y), m * fabsf(w.inv.z));
       const V3 k = v3(-(o.x * w.inv.x), -(o.y * w.inv.y), -(o.z * w.inv.z));
       w.kn = k - e;

@@ -258,3 +258,42 @@ def test_traversals_that_share_a_launch_equal_separate_ones(cuda, kind, depth, b
         pt.tune("bin_min_paths", 1 << 25)
     assert all(np.array_equal(x.view(np.uint32), y.view(np.uint32)) for x, y in zip(*out))
     assert stats[0] == stats[1]
+
+
+@pytest.mark.parametrize("c", [1e-4, 1e-12, 2.0 ** -40, 1e-30, 1e-36, 1e-37, 1e-38, 3e-39, 2e-39, 1e-40, 1e-45])
+@pytest.mark.parametrize("offset", [0.0, 1000.0])
+def test_tiny_direction_components(cuda, c, offset):
+    # the reciprocal of such a component is huge, its product with the origin beyond the largest float, or the
+    # reciprocal itself infinite; origins on and off vertex planes, and far from the scene's centre
+    s = _scene("random")
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    rng = np.random.default_rng(17)
+    n = 20_000
+    v = s.tri_v.reshape(-1, 3)
+    o = np.where(rng.random((n, 3)) < 0.4, v[rng.integers(0, len(v), n)], rng.uniform(v.min(0), v.max(0), (n, 3)))
+    k = rng.integers(0, 3, n)
+    side = np.where(rng.random(n) < 0.5, -1.0, 1.0)
+    o[np.arange(n), k] += offset * side
+    d = np.where(rng.random((n, 3)) < 0.5, -c, c)
+    one = rng.random(n) < 0.3  # one component tiny, the other not
+    d[one, (k[one] + 1) % 3] = rng.uniform(-1, 1, one.sum())
+    d[np.arange(n), k] = -side
+    rays = np.concatenate([o, np.zeros((n, 1)), d, np.full((n, 1), np.inf)], 1).astype(np.float32)
+    kd, _ = gpu_trace(cuda, ds, rays, counts=True)
+    wide, _ = gpu_trace(cuda, ds, rays)
+    hit = kd[:, 1].view(np.int32) >= 0
+    assert hit.any()
+    assert np.array_equal(kd.view(np.uint32), wide.view(np.uint32))
+    assert np.array_equal(gpu_any(cuda, ds, rays) != 0, hit)
+
+
+@pytest.mark.parametrize("length", [1e-38, 1e-30, 1e-20, 1e20, 1e30, 1e38])
+def test_directions_of_any_length(cuda, length):
+    s = _soup(_random_tris(3000, 10, size=0.1) * 50)
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    rays = _rays(s, 4000, 19)
+    rays[:, 4:7] = (rays[:, 4:7].astype(np.float64) * length).astype(np.float32)
+    kd, _ = gpu_trace(cuda, ds, rays, counts=True)
+    wide, _ = gpu_trace(cuda, ds, rays)
+    assert np.array_equal(kd.view(np.uint32), wide.view(np.uint32))
+    assert np.array_equal(gpu_any(cuda, ds, rays) != 0, kd[:, 1].view(np.int32) >= 0)
