@@ -63,12 +63,12 @@ constexpr float kWideEps = 1.5f / 1048576.0f;
 // smaller one, multiplied by the origin, overflows, and boxes that the ray passes were missed (components
 // of 1e-38; and where the reciprocal itself is infinite every box was met: 200,000 rays 0.3 -> 611 ms).  It is
 // still conservative: through the scene such a ray moves at most 2^-38 M along that axis, and the planes
-// are 2^-19 M farther out.
-constexpr float kWideLeast = 1.0f / 1099511627776.0f;
-// ... and below this part of it the ray is one with a zero component to the kd-tree's rounding (kWideTie)
-constexpr float kWideZero = 1.0e-30f;
-// What the box tests multiply and add lies between 2^-20 and 2^41 times M / (largest component); where M / it is
-// beyond these, products overflow or lose bits below the normal numbers, and the kd-tree answers the ray.
+// are 2^-19 M farther out.  (All of it in reciprocals: least is that of the largest component.)
+constexpr float kWideMost = 1099511627776.0f;
+// ... and from this part of it on the ray is one with a zero component to the kd-tree's rounding (wide_beside)
+constexpr float kWideZero = 1.0e30f;
+// What the box tests multiply and add lies between 2^-20 and 2^41 times M x least; where that is beyond these,
+// products overflow or lose bits below the normal numbers, and the kd-tree answers the ray.
 constexpr float kWideScaleMin = 1.0e-25f, kWideScaleMax = 1.0e25f;
 
 #if defined(__CUDACC__)
@@ -188,7 +188,8 @@ struct WideShared {
   uint8_t own[64];           // ... and the lane it is for
   int32_t sphere[32];        // analytic sphere hit before the traversal, -1: none
   const F4 *tris[32];        // the lanes' scenes' triangle records (waves of several scenes)
-  uint32_t tie[32];          // ordered t of the nearest pair of hits within kWideTie of each other
+  uint8_t zero[32];          // axes of zero direction components
+  uint32_t tie[32];          // ordered t of the nearest hit that the kd-tree has to decide (kWideTie, wide_beside)
 };
 
 __device__ __forceinline__ uint32_t wide_order(float f) {
@@ -204,9 +205,25 @@ __device__ __forceinline__ float wide_unorder(uint32_t u) {
 // once the best hit lies inside the current cell, widened by 2^-18), so such a ray is traced again
 // there.  It is a ray through an exact edge, or a surface laid on another: one in some 10^8 on scenes
 // without coincident surfaces.
-// So is a ray with a zero direction component, or as good as zero: one that lies in a split plane sees only
-// the cells on one side of it in the kd-tree.
 constexpr float kWideTie = 1.0f / 131072.0f;
+
+// So is a ray with a zero direction component, or as good as zero, if its hit touches the plane through its
+// origin normal to that axis from one side: if that is a split plane the ray sees only the cells on one side
+// of it in the kd-tree, and the triangle may be listed on the other.  Split planes are triangle bounds and
+// triangles are listed by their bounds, so a triangle with vertices on both sides is in both cells.
+// axes: the mask of those components; within a t of 1e-29 of the plane counts, as the kd-tree takes
+// 1e30 for the reciprocal of a zero.
+// (Tracing all of them in the kd-tree, lane by lane: 1 M vertical rays from random points among 300 k triangles
+// 673 us, now 251; random rays of which 5 % have a zero component 358 us, now 178.)
+// Not inlined, and reads the triangle again, so that the tests' code keeps neither the mask nor the vertices.
+inline __device__ __noinline__ bool wide_beside(uint32_t axes, V3 o, float t, const F4 *tri) {
+  const F4 a = load_f4(tri, 0), b = load_f4(tri, 1), c = load_f4(tri, 2);
+  const float e = 1.0e-29f * fabsf(t);
+  const V3 lo = v3(fminf(a.x, fminf(b.x, c.x)), fminf(a.y, fminf(b.y, c.y)), fminf(a.z, fminf(b.z, c.z)));
+  const V3 hi = v3(fmaxf(a.x, fmaxf(b.x, c.x)), fmaxf(a.y, fmaxf(b.y, c.y)), fmaxf(a.z, fmaxf(b.z, c.z)));
+  return ((axes & 1u) && (o.x - e <= lo.x || o.x + e >= hi.x)) || ((axes & 2u) && (o.y - e <= lo.y || o.y + e >= hi.y)) ||
+         ((axes & 4u) && (o.z - e <= lo.z || o.z + e >= hi.z));
+}
 
 // The kd-tree's answer for one ray: closest hit, or any (h.prim >= 0).  seq: a leaf's triangles one after
 // another, each against the t before it; otherwise the smallest (t, leaf order) among those accepted
@@ -258,8 +275,11 @@ __device__ __noinline__ void kd_ray(const SceneView &s, const Ray &r, bool seq, 
 //   seq     which of the kd-tree's orders decides near ties (kd_ray)
 //   SINGLE  every ray is in the scene view(0), which the kernel passes from its parameter space
 //   TZERO   every ray starts at t = 0
+//   AXES    rays with zero direction components go through the hierarchy (wide_beside); otherwise the kd-tree
+//           answers them.  Ray queries along an axis are whole launches of such rays; a path meets one by
+//           chance, and the code of the test makes the render kernels spill.
 // All 32 lanes call round(), the other members are per lane or say so.
-template <bool ANY, bool COUNT, bool SPH, bool SINGLE, bool TZERO, class View, class Load, class Store>
+template <bool ANY, bool COUNT, bool SPH, bool SINGLE, bool TZERO, bool AXES, class View, class Load, class Store>
 struct WideWarp {
   static constexpr unsigned kFull = 0xFFFFFFFFu;
   View view;
@@ -304,21 +324,20 @@ struct WideWarp {
     active = s.ntri > 0 && !(ANY && sphere >= 0);
     const V3 o = r.o - v3(s.wcentre[0], s.wcentre[1], s.wcentre[2]);
     float m = fmaxf(fmaxf(s.wextent, fabsf(o.x)), fmaxf(fabsf(o.y), fabsf(o.z)));
-    const float dmax = fmaxf(fabsf(r.d.x), fmaxf(fabsf(r.d.y), fabsf(r.d.z))), scale = m / dmax;
-    const float zero = dmax * kWideZero;
-    kd = active && (fabsf(r.d.x) <= zero || fabsf(r.d.y) <= zero || fabsf(r.d.z) <= zero ||
-                    !(scale >= kWideScaleMin && scale <= kWideScaleMax));
+    const V3 inv = v3(1.0f / r.d.x, 1.0f / r.d.y, 1.0f / r.d.z);
+    const V3 ai = v3(fabsf(inv.x), fabsf(inv.y), fabsf(inv.z));
+    const float least = fminf(ai.x, fminf(ai.y, ai.z)), most = fmaxf(ai.x, fmaxf(ai.y, ai.z));
+    const float zero = least * kWideZero, scale = m * least;
+    kd = active && ((!AXES && most >= zero) || !(scale >= kWideScaleMin && scale <= kWideScaleMax));
     active = active && !kd;
     if (active) {
       float t0, t1;
-      active = clip_root(s, r, v3(1.0f / r.d.x, 1.0f / r.d.y, 1.0f / r.d.z), t0, t1) &&
-               fmaxf(t0, r.tmin) <= fminf(t1, r.tmax);
+      active = clip_root(s, r, inv, t0, t1) && fmaxf(t0, r.tmin) <= fminf(t1, r.tmax);
     }
     if (active) {
       const RayPre pre = precompute(r);
-      const float least = dmax * kWideLeast;
-      w.inv = v3(1.0f / copysignf(fmaxf(fabsf(r.d.x), least), r.d.x), 1.0f / copysignf(fmaxf(fabsf(r.d.y), least), r.d.y),
-                 1.0f / copysignf(fmaxf(fabsf(r.d.z), least), r.d.z));
+      const float cap = least * kWideMost;
+      w.inv = v3(copysignf(fminf(ai.x, cap), inv.x), copysignf(fminf(ai.y, cap), inv.y), copysignf(fminf(ai.z, cap), inv.z));
       m *= kWideEps;
       const V3 e = v3(m * fabsf(w.inv.x), m * fabsf(w.inv.y), m * fabsf(w.inv.z));
       const V3 k = v3(-(o.x * w.inv.x), -(o.y * w.inv.y), -(o.z * w.inv.z));
@@ -334,11 +353,12 @@ struct WideWarp {
       sh.b[lane] = make_float4(pre.sx, pre.sy, pre.sz, r.tmax);
       if (!SINGLE) sh.tris[lane] = s.wtris;
       sh.k[lane] = (uint32_t)pre.kx | ((uint32_t)pre.ky << 2) | ((uint32_t)pre.kz << 4);
+      if (AXES)
+        sh.zero[lane] = most < zero ? (uint8_t)0
+                                    : (uint8_t)((ai.x >= zero ? 1u : 0u) | (ai.y >= zero ? 2u : 0u) | (ai.z >= zero ? 4u : 0u));
     }
-    if (!ANY) {
-      sh.key[lane] = ((unsigned long long)wide_order(best) << 32) | (sphere >= 0 ? 0xFFFFFFFEu : 0xFFFFFFFFu);
-      sh.tie[lane] = 0xFFFFFFFFu;
-    }
+    if (!ANY) sh.key[lane] = ((unsigned long long)wide_order(best) << 32) | (sphere >= 0 ? 0xFFFFFFFEu : 0xFFFFFFFFu);
+    if (!ANY || AXES) sh.tie[lane] = 0xFFFFFFFFu;
   }
 
   // one node of the lane's ray: its triangles into tg, its inner children pending
@@ -387,8 +407,11 @@ struct WideWarp {
       float t, b1, b2;
       if (intersect_tri(p, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), (f_bits(b.w) & 1u) != 0u,
                         TZERO ? 0.0f : ra.w, rb.w, t, b1, b2)) {
+        const uint32_t axes = AXES ? sh.zero[o] : 0u;
+        const bool beside = axes != 0u && wide_beside(axes, p.o, t, lt + q);
+        if (beside) atomicMin(&sh.tie[o], wide_order(t));
         if (ANY) {
-          hit = 1u << o;
+          if (!beside) hit = 1u << o;
         } else {
           const unsigned long long old = atomicMin(&sh.key[o], ((unsigned long long)wide_order(t) << 32) | rec);
           const float told = wide_unorder((uint32_t)(old >> 32));
@@ -422,6 +445,7 @@ struct WideWarp {
     uint32_t rec = 0xFFFFFFFFu;
     if (ANY) {
       if (found) h.prim = 0;
+      if (AXES) kd = kd || (!found && sh.tie[lane] != 0xFFFFFFFFu);
     } else {
       const unsigned long long key = sh.key[lane];
       h.t = wide_unorder((uint32_t)(key >> 32));
@@ -487,7 +511,7 @@ __device__ __forceinline__ void wide_trace(const Rays &rays, View view, uint32_t
     if (first >= n) break;
     const uint32_t i = (uint32_t)first + lane;
     __syncwarp(kFull);  // the previous rays' readers are done with the shared records
-    WideWarp<ANY, COUNT, SPH, SINGLE, TZERO, View, Load, Store> t{view, load, store, sh, tab, cnt, lane, seq, stack};
+    WideWarp<ANY, COUNT, SPH, SINGLE, TZERO, false, View, Load, Store> t{view, load, store, sh, tab, cnt, lane, seq, stack};
     if (i < n) {
       t.start(i);
       ++rays_done;
@@ -518,12 +542,13 @@ __device__ __forceinline__ void wide_trace_refill(View view, uint32_t n, Load lo
   constexpr unsigned kFull = 0xFFFFFFFFu;
   uint2 stack[kWideMaxDepth];
   const WideChunks chunks(n);
-  WideWarp<ANY, false, SPH, true, false, View, Load, Store> t{view, load, store, sh, tab, nullptr, threadIdx.x & 31u, seq, stack};
+  WideWarp<ANY, false, SPH, true, false, true, View, Load, Store> t{view, load, store, sh, tab, nullptr, threadIdx.x & 31u, seq, stack};
   uint32_t i = 0u;
   bool have = false;  // the lane holds ray i
   bool more = true;   // the block has rays left (uniform over the warp)
   for (bool swap = true;;) {
     if (swap) {
+      __syncwarp(kFull);
       if (have && !t.active) {
         t.finish(i);
         have = false;

@@ -287,6 +287,40 @@ def test_tiny_direction_components(cuda, c, offset):
     assert np.array_equal(gpu_any(cuda, ds, rays) != 0, hit)
 
 
+@pytest.mark.parametrize("kind", ["flat", "plain", "random", "coincident", "points", "culled", "balls", "n7"])
+@pytest.mark.parametrize("zeros", [1, 2])
+def test_zero_components_in_vertex_planes(cuda, kind, zeros):
+    # a ray in a split plane sees the cells on one side of it only: rays through vertices, along edges and beside
+    # them, whose origin shares the vertex' coordinate along every axis that the direction does not have
+    s = _scene(kind)
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    rng = np.random.default_rng(23)
+    n = 30_000
+    v = s.tri_v.reshape(-1, 3)
+    t = s.tri_v[rng.integers(0, s.ntri, n)].astype(np.float64)
+    w = rng.dirichlet((1, 1, 1), n) * np.where(rng.random((n, 1)) < 0.2, 1.0, rng.integers(0, 2, (n, 3)))
+    w /= np.maximum(w.sum(1, keepdims=True), 1e-9)
+    at = (t * w[..., None]).sum(1).astype(np.float32)
+    at = np.where(w.max(1, keepdims=True) == 1.0, t[np.arange(n), w.argmax(1)].astype(np.float32), at)
+    o = rng.uniform(v.min(0) - 0.5, v.max(0) + 0.5, (n, 3)).astype(np.float32)
+    zero = np.zeros((n, 3), bool)
+    k = rng.integers(0, 3, n)
+    zero[np.arange(n), k] = True
+    if zeros == 2:
+        zero[np.arange(n), (k + 1) % 3] = True
+    o = np.where(zero, at, o)
+    rays = np.zeros((n, 8), np.float32)
+    rays[:, 0:3] = o
+    rays[:, 4:7] = np.where(zero, np.where(rng.random((n, 3)) < 0.5, -0.0, 0.0), at - o)
+    rays[:, 7] = np.where(rng.random(n) < 0.5, np.inf, rng.uniform(0.5, 1.5, n))
+    kd, _ = gpu_trace(cuda, ds, rays, counts=True)
+    wide, _ = gpu_trace(cuda, ds, rays)
+    assert (kd[:, 1].view(np.int32) >= 0).any()
+    same = np.all(kd.view(np.uint32) == wide.view(np.uint32), axis=1)
+    assert same.all(), (int((~same).sum()), rays[~same][:2], kd[~same][:2], wide[~same][:2])
+    assert np.array_equal(gpu_any(cuda, ds, rays) != 0, kd[:, 1].view(np.int32) >= 0)
+
+
 @pytest.mark.parametrize("length", [1e-38, 1e-30, 1e-20, 1e20, 1e30, 1e38])
 def test_directions_of_any_length(cuda, length):
     s = _soup(_random_tris(3000, 10, size=0.1) * 50)
