@@ -21,6 +21,7 @@ int fail(int code, const std::string &msg) {
 }
 int cuda_fail(cudaError_t e, const char *what) {
   t_last_error = std::string(what) + ": " + cudaGetErrorString(e);
+  cudaGetLastError();  // reported here: the next call's check of its launches does not find it again
   return e == cudaErrorMemoryAllocation ? MGPU_E_NOMEM : MGPU_E_CUDA;
 }
 

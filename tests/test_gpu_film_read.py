@@ -62,3 +62,28 @@ def test_pool_gives_blocks_back_and_stays_bounded(cuda):
     assert hostmem._total <= max(before, hostmem.LIMIT)
     p = C.c_void_p()
     assert N.load().mgpu_host_alloc(0, C.byref(p)) != N.MGPU_OK
+
+
+def test_a_failed_allocation_does_not_fail_the_next_call(cuda):
+    s = scenegen.plain(0)
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    st = pt.RenderSettings(64, 48, 2, max_depth=2, rr_start_depth=3, seed=3)
+    f, g = pt.Film(64, 48), pt.Film(64, 48)
+    pt.render(ds, st, f)
+    want = f.mean(), f.tonemap()
+    lib = N.load()
+
+    def fail():
+        p = C.c_void_p()
+        assert lib.mgpu_host_alloc(1 << 60, C.byref(p)) != N.MGPU_OK and not p.value
+
+    fail()
+    pt.render(ds, st, g)
+    fail()
+    assert np.array_equal(g.mean(), want[0])
+    fail()
+    assert np.array_equal(g.tonemap(), want[1])
+    fail()
+    assert pt.film_error([g])[0] == pt.film_error([f])[0]
+    fail()
+    assert pt.DeviceScene(s, pt.Accel(s)).nbytes == ds.nbytes
