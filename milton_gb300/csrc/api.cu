@@ -2,6 +2,7 @@
 #include <string.h>
 
 #include <cmath>
+#include <map>
 #include <mutex>
 #include <new>
 #include <vector>
@@ -341,14 +342,22 @@ struct ReadScratch {
 };
 static thread_local ReadScratch t_read;
 
-// the device's view of a page-locked host buffer, or nullptr for pageable memory
-static void *device_view(const void *p) {
-  cudaPointerAttributes at;
-  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
+// Blocks of mgpu_host_alloc that are not freed: address, bytes.
+static std::mutex g_host_mu;
+static std::map<uintptr_t, size_t> &g_host_blocks = *new std::map<uintptr_t, size_t>;  // outlives the program's statics
+
+// Whether the device may write the n bytes at p itself: they lie in one block of mgpu_host_alloc, aligned for
+// its stores.  Other page-locked memory is not asked for: the runtime tells what the first byte is, not how
+// far its registration reaches.  (Such a block has one address on host and device.)
+static bool device_writes(const void *p, size_t n, size_t align) {
+  const uintptr_t at = (uintptr_t)p;
+  if (at % align) return false;
+  std::lock_guard<std::mutex> lock(g_host_mu);
+  auto it = g_host_blocks.upper_bound(at);
+  if (it == g_host_blocks.begin()) return false;
+  --it;
+  const size_t off = at - it->first;
+  return off <= it->second && n <= it->second - off;
 }
 
 }  // namespace mgpu
@@ -772,8 +781,8 @@ int mgpu_film_read(mgpu_film *f, double *out_mean, void *stream) {
     return cudaGetLastError();
   };
   // into the caller's array where the device can write it
-  if (double *dst = (double *)device_view(out_mean)) {
-    MGPU_CUDA(launch(0, n, dst));
+  if (device_writes(out_mean, (size_t)n * 3 * sizeof(double), alignof(double))) {
+    MGPU_CUDA(launch(0, n, out_mean));
     MGPU_CUDA(cudaStreamSynchronize(st));
     return MGPU_OK;
   }
@@ -817,8 +826,7 @@ int mgpu_film_tonemap(mgpu_film *f, uint8_t *out_rgba, void *stream) {
   uchar4 *img = nullptr;
   MGPU_CUDA(t_read.device_buffer(kErrBlocks * sizeof(double2), (void **)&part));
   const size_t bytes = (size_t)npix * sizeof(uchar4);
-  void *dst = device_view(out_rgba);
-  if ((uintptr_t)dst & 3) dst = nullptr;
+  void *dst = device_writes(out_rgba, bytes, sizeof(uchar4)) ? out_rgba : nullptr;
   if (!dst) MGPU_CUDA(t_read.host_buffer(bytes, (void **)&img));
   cudaStream_t st = as_stream(stream);
   k_tonemap_reduce<<<kErrBlocks, kErrThreads, 0, st>>>(ref, part);
@@ -864,10 +872,22 @@ int mgpu_film_error(mgpu_film *const *films, int32_t n, double *out_rmse, void *
 int mgpu_host_alloc(uint64_t bytes, void **out) {
   if (!out || bytes == 0) return fail(MGPU_E_INVALID, "mgpu_host_alloc: bad argument");
   MGPU_CUDA(cudaHostAlloc(out, (size_t)bytes, cudaHostAllocPortable | cudaHostAllocMapped));
+  try {
+    std::lock_guard<std::mutex> lock(g_host_mu);
+    g_host_blocks[(uintptr_t)*out] = (size_t)bytes;
+  } catch (const std::bad_alloc &) {
+    cudaFreeHost(*out);
+    *out = nullptr;
+    return fail(MGPU_E_NOMEM, "mgpu_host_alloc: out of host memory");
+  }
   return MGPU_OK;
 }
 
 int mgpu_host_free(void *p) {
+  {
+    std::lock_guard<std::mutex> lock(g_host_mu);
+    g_host_blocks.erase((uintptr_t)p);
+  }
   if (p) MGPU_CUDA(cudaFreeHost(p));
   return MGPU_OK;
 }

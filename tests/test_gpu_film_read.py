@@ -87,3 +87,48 @@ def test_a_failed_allocation_does_not_fail_the_next_call(cuda):
     assert pt.film_error([g])[0] == pt.film_error([f])[0]
     fail()
     assert pt.DeviceScene(s, pt.Accel(s)).nbytes == ds.nbytes
+
+
+@pytest.mark.parametrize("kind", ["none", "triangle"])
+@pytest.mark.parametrize("part", ["pageable", "head", "tail", "whole", "two", "block", "inside", "beyond"])
+def test_arrays_of_which_a_part_is_page_locked(cuda, kind, part):
+    # the device writes only what lies in one block of mgpu_host_alloc; any other memory is filled by copies, be
+    # its first byte page-locked or not
+    page = 1 << 16
+    w, h = 173, 211
+    s = scenegen.plain(0)
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    f = pt.Film(w, h)
+    if kind != "none":
+        f.set_filter(kind, 2.0)
+    pt.render(ds, pt.RenderSettings(w, h, 2, max_depth=2, rr_start_depth=3, seed=3), f)
+    want = np.array(f.mean()), np.array(f.tonemap())
+    lib, rt = N.load(), cuda.cuda.cudart()
+    for img, read in zip(want, (lib.mgpu_film_read, lib.mgpu_film_tonemap)):
+        size = -(-img.nbytes // page) * page + 2 * page
+        block, ranges = C.c_void_p(), []
+        if part in ("block", "inside", "beyond"):
+            # the array: the whole block, its end, or ordinary memory
+            N.check(lib.mgpu_host_alloc(img.nbytes + (page if part == "inside" else 0), C.byref(block)))
+            at = block.value + (page if part == "inside" else 0)
+            if part == "beyond":
+                raw = np.zeros(size, np.uint8)
+                at = -(-raw.ctypes.data // page) * page
+        else:
+            raw = np.zeros(size, np.uint8)
+            at = -(-raw.ctypes.data // page) * page
+            half = img.nbytes // 2 // page * page
+            ranges = {"pageable": [], "head": [(0, half)], "tail": [(half, page)], "whole": [(0, size - page)],
+                      "two": [(0, half), (half, page)]}[part]
+        for first, n in ranges:
+            assert n > 0 and int(rt.cudaHostRegister(at + first, n, 0)) == 0
+        try:
+            N.check(read(f.handle, at, None))
+            got = np.ctypeslib.as_array((C.c_uint8 * img.nbytes).from_address(at)).view(img.dtype).reshape(img.shape)
+            assert np.array_equal(got, img)
+            del got
+        finally:
+            for first, _ in ranges:
+                rt.cudaHostUnregister(at + first)
+            if block:
+                N.check(lib.mgpu_host_free(block))
