@@ -270,9 +270,9 @@ int mgpu_film_clear(mgpu_film *film, void *stream);
 int mgpu_film_destroy(mgpu_film *film);
 /* The film's output in FP64: out = host array of width*height*3 doubles (synchronises): the
  * per-pixel mean, or with a reconstruction filter set, sum(w L) / sum(w) over the samples
- * splatted onto each pixel.  Taken on the device, which writes page-locked arrays (mgpu_host_alloc)
- * itself; a pageable one is filled through at most 12 MB of page-locked staging that the calling
- * thread keeps for its later reads (released when the thread exits).                          */
+ * splatted onto each pixel.  Taken on the device, which writes arrays of mgpu_host_alloc itself; any
+ * other is copied from at most 96 MB of device scratch that the calling thread keeps for its later
+ * reads (24 bytes per pixel; released when the thread exits).                                 */
 int mgpu_film_read(mgpu_film *film, double *out_mean, void *stream);
 /* Reconstruction filter of ReconstructionRenderOutput (ReconstructionRenderOutput.cpp:30-83):
  * every sample is splatted onto the pixels within (ceil(support) | 1) / 2 of its own with
@@ -385,7 +385,8 @@ int mgpu_tune_set(const char *key, int64_t value);
 int mgpu_tune_get(const char *key, int64_t *value);
 
 /* Page-locked host memory for results (film reads, tone maps): the device writes it without a
- * staging copy.  No counterpart in the reference. */
+ * copy.  Copies from it are asynchronous: they must have ended before it is read into again or
+ * freed.  No counterpart in the reference. */
 int mgpu_host_alloc(uint64_t bytes, void **out);
 int mgpu_host_free(void *p);
 

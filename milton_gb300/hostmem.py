@@ -1,39 +1,48 @@
-"""Result arrays in page-locked host memory, from a bounded pool.
+"""Result arrays in ordinary host memory whose pages exist already, from a bounded pool.
 
-The device writes such an array itself (mgpu_host_alloc), so a film read needs no staging copy and
-touches no fresh pages (256 x 256 means: 157 -> 40 us a read).  A block goes back to the pool when the
-last numpy view of it is gone; the pool holds at most LIMIT bytes, in use and free together, beyond
-which results are ordinary numpy arrays.  Safe with several threads.
+A fresh array's pages are made as it is filled (1024 x 1024 means: 1.7 ms of a read that takes 0.2 into
+pages that exist), so the memory of a result goes back to the pool when the last numpy view of it is gone, as
+malloc would take it, but stays mapped.  It is pageable: a copy to a device has read it when the call that
+starts it returns, whatever its stream does, and forked processes have their own.  (Page-locked blocks,
+which the device could write itself, gave neither: an asynchronous copy from a temporary result was still
+reading when the next result was written there.)  The pool holds at most LIMIT bytes, in use and free
+together, beyond which results are ordinary numpy arrays.  Safe with several threads.
 """
 from __future__ import annotations
 
 import ctypes as C
 import math
+import os
 import threading
 import weakref
 
 import numpy as np
 
-from . import _native as N
-
 LIMIT = 256 << 20
-MIN = 1 << 17    # smaller results are ordinary arrays: their copy costs less than the bookkeeping
+MIN = 1 << 17    # smaller results are ordinary arrays: malloc keeps their pages
 _GRAIN = 1 << 16
 
 _lock = threading.RLock()  # reentrant: a collection inside the lock may return a block
-_free: dict[int, list[int]] = {}
+_free: dict[int, list[np.ndarray]] = {}
 _total = 0
 
 
-def _release(size: int, addr: int) -> None:
+def _after_fork() -> None:
+    global _lock
+    _lock = threading.RLock()  # another thread may have held it
+
+
+os.register_at_fork(after_in_child=_after_fork)
+
+
+def _release(size: int, block: np.ndarray) -> None:
     with _lock:
-        _free.setdefault(size, []).append(addr)
+        _free.setdefault(size, []).append(block)
 
 
-def _take(size: int) -> int | None:
-    """A block of size bytes, or None: the pool is at its limit or page-locked memory is short."""
+def _take(size: int) -> np.ndarray | None:
+    """A block of size bytes, or None: the pool is at its limit."""
     global _total
-    lib = N.load()
     with _lock:
         blocks = _free.get(size)
         if blocks:
@@ -41,15 +50,13 @@ def _take(size: int) -> int | None:
         if _total + size > LIMIT:
             for s, bs in list(_free.items()):
                 while bs:
-                    lib.mgpu_host_free(bs.pop())
+                    bs.pop()
                     _total -= s
         if _total + size > LIMIT:
             return None
-        p = C.c_void_p()
-        if lib.mgpu_host_alloc(size, C.byref(p)) != N.MGPU_OK or not p.value:
-            return None
+        block = np.empty(size, np.uint8)
         _total += size
-        return p.value
+        return block
 
 
 def empty(shape, dtype) -> np.ndarray:
@@ -57,9 +64,9 @@ def empty(shape, dtype) -> np.ndarray:
     count = math.prod(shape)
     n = count * np.dtype(dtype).itemsize
     size = -(-n // _GRAIN) * _GRAIN
-    addr = _take(size) if n >= MIN else None
-    if addr is None:
+    block = _take(size) if n >= MIN else None
+    if block is None:
         return np.empty(shape, dtype)
-    owner = (C.c_byte * size).from_address(addr)
-    weakref.finalize(owner, _release, size, addr).atexit = False
+    owner = (C.c_byte * size).from_address(block.ctypes.data)
+    weakref.finalize(owner, _release, size, block).atexit = False
     return np.frombuffer(owner, dtype, count=count).reshape(shape)

@@ -132,3 +132,24 @@ def test_arrays_of_which_a_part_is_page_locked(cuda, kind, part):
                 rt.cudaHostUnregister(at + first)
             if block:
                 N.check(lib.mgpu_host_free(block))
+
+
+def test_a_copy_from_a_result_outlives_it(cuda):
+    # a copy that waits behind a frame on another stream; its source, a temporary result, is gone and the next
+    # result is read meanwhile
+    s = scenegen.random_scene(3, 20_000)
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    films = [pt.Film(256, 200) for _ in range(2)]
+    for k, f in enumerate(films):
+        pt.render(ds, pt.RenderSettings(256, 200, 2, max_depth=2, rr_start_depth=3, seed=k), f)
+    want = [np.array(f.mean()) for f in films]
+    assert not np.array_equal(*want)
+    side, big = cuda.cuda.Stream(), pt.Film(1024, 1024)
+    cuda.cuda.synchronize()
+    for read, want in ((pt.Film.mean, want), (pt.Film.raw, [np.array(f.raw()) for f in films])):
+        with cuda.cuda.stream(side):
+            pt.render(ds, pt.RenderSettings(1024, 1024, 16, max_depth=6, rr_start_depth=3, seed=5), big)
+            got = cuda.from_numpy(read(films[0], stream=cuda.cuda.default_stream())).to("cuda", non_blocking=True)
+        again = read(films[1], stream=cuda.cuda.default_stream())
+        cuda.cuda.synchronize()
+        assert np.array_equal(got.cpu().numpy(), want[0]) and np.array_equal(again, want[1])
