@@ -615,6 +615,7 @@ int mgpu_scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void
     delete s;
     return rc;
   }
+  if (!wide) s->view.wextent = INFINITY;
   s->view.wnodes = wide ? (const uint32_t *)(base + L.off_wnodes) : nullptr;
   s->view.wtris = wide ? (const F4 *)(base + L.off_wtris) : nullptr;
   // staging the top of the tree in shared memory costs more occupancy than it saves on GB300

@@ -55,7 +55,7 @@ struct SceneView {
   const uint32_t *wnodes;  // 8-wide hierarchy (hd_wide.h), nullptr: none
   const F4 *wtris;         // its triangle records, 3 per triangle
   float wcentre[3];        // what its node coordinates are relative to
-  float wextent;           // the largest coordinate of its box from there
+  float wextent;           // the largest coordinate of its box from there, infinite without a hierarchy
 #endif
 };
 

@@ -68,7 +68,9 @@ constexpr float kWideMost = 1099511627776.0f;
 // ... and from this part of it on the ray is one with a zero component to the kd-tree's rounding (wide_beside)
 constexpr float kWideZero = 1.0e30f;
 // What the box tests multiply and add lies between 2^-20 and 2^41 times M x least; where that is beyond these,
-// products overflow or lose bits below the normal numbers, and the kd-tree answers the ray.
+// products overflow or lose bits below the normal numbers, and the kd-tree answers the ray.  (A scene without
+// the hierarchy has an infinite extent, which takes its rays there where it shares a wave with scenes that
+// have one.)
 constexpr float kWideScaleMin = 1.0e-25f, kWideScaleMax = 1.0e25f;
 
 #if defined(__CUDACC__)
@@ -226,10 +228,11 @@ inline __device__ __noinline__ bool wide_beside(uint32_t axes, V3 o, float t, co
 }
 
 // The kd-tree's answer for one ray: closest hit, or any (h.prim >= 0).  seq: a leaf's triangles one after
-// another, each against the t before it; otherwise the smallest (t, leaf order) among those accepted
-// against the t before the leaf.
-template <bool ANY, bool SPH>
-__device__ __noinline__ void kd_ray(const SceneView &s, const Ray &r, bool seq, Hit &h) {
+// another, each against the t before it (ray queries, scenes with analytic spheres); otherwise the
+// smallest (t, leaf order) among those accepted against the t before the leaf.  The two differ where
+// triangles coincide, so the rule belongs to the scene, not to the launch.
+template <bool ANY, bool SPH, bool COUNT>
+__device__ __forceinline__ void kd_trace(const SceneView &s, const Ray &r, bool seq, Hit &h, TraceCounts *cnt) {
   TravState st;
   TravEntry stack[kMaxStack];
   if (trav_init<SPH>(s, r, nullptr, 0, st, ANY)) {
@@ -237,10 +240,11 @@ __device__ __noinline__ void kd_ray(const SceneView &s, const Ray &r, bool seq, 
     while (!done) {
       uint32_t w0, w1;
       float tmax;
-      trav_descend<false>(s, st, stack, nullptr, 0, nullptr, w0, w1, tmax);
+      trav_descend<COUNT>(s, st, stack, nullptr, 0, cnt, w0, w1, tmax);
       const float best0 = st.best;
       bool took = false;
       for (uint32_t i = 0; i < (w0 >> 2) && !(ANY && took); ++i) {
+        if (COUNT) cnt->tris++;
         const int64_t q = 3 * ((int64_t)w1 + i);
         const F4 a = load_f4(s.ltris, q), b = load_f4(s.ltris, q + 1), c = load_f4(s.ltris, q + 2);
         float t, b1, b2;
@@ -251,13 +255,33 @@ __device__ __noinline__ void kd_ray(const SceneView &s, const Ray &r, bool seq, 
           st.best = t; st.best_prim = (int32_t)f_bits(a.w); st.bb1 = b1; st.bb2 = b2;
         }
       }
-      done = (ANY && took) || trav_after_leaf<false>(st, stack, tmax);
+      done = (ANY && took) || trav_after_leaf<ANY>(st, stack, tmax);
     }
   }
   h.t = st.best;
   h.prim = st.best_prim;
   h.b1 = st.bb1;
   h.b2 = st.bb2;
+}
+
+template <bool ANY, bool SPH, bool QUERY>
+__device__ __noinline__ void kd_ray(const SceneView &s, const Ray &r, Hit &h) {
+  kd_trace<ANY, SPH, false>(s, r, QUERY || (SPH && s.nsphere > 0), h, nullptr);
+}
+
+// Rays 0 .. n - 1 through the kd-tree, one per lane, grid-stride: scenes without the hierarchy.
+template <bool ANY, bool COUNT, bool SPH, class View, class Load, class Store>
+__device__ __forceinline__ void kd_grid(View view, uint32_t n, Load load, Store store, TraceCounts *cnt,
+                                        uint32_t &rays_done) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const SceneView &s = view(i);
+    Ray r;
+    load(i, r);
+    ++rays_done;
+    Hit h;
+    kd_trace<ANY, SPH, COUNT>(s, r, SPH && s.nsphere > 0, h, cnt);
+    store(i, h.prim >= 0, h);
+  }
 }
 
 // The traversal of one warp.  Every lane steps through the nodes of its own ray; the triangles it meets go
@@ -272,14 +296,14 @@ __device__ __noinline__ void kd_ray(const SceneView &s, const Ray &r, bool seq, 
 // queries): kd-tree 187.7 ms of traversal, nodes of 80 bytes with per-node slack and child order by mask
 // permutation 95.0, nodes of 96 bytes on an 8-bit grid 83.7, as it is now 77.9.
 //   ANY     occlusion: the first hit ends the ray; otherwise the closest
-//   seq     which of the kd-tree's orders decides near ties (kd_ray)
+//   QUERY   a ray query, whose near ties are decided in leaf order (seq of kd_trace) whatever the scene; otherwise
+//           the scene's rule decides
 //   SINGLE  every ray is in the scene view(0), which the kernel passes from its parameter space
-//   TZERO   every ray starts at t = 0
-//   AXES    rays with zero direction components go through the hierarchy (wide_beside); otherwise the kd-tree
-//           answers them.  Ray queries along an axis are whole launches of such rays; a path meets one by
-//           chance, and the code of the test makes the render kernels spill.
+//           and its rays with zero direction components go through the hierarchy (wide_beside): queries along an
+//           axis are whole launches of such rays.  A path meets one by chance, the kd-tree answers it, and
+//           the render kernels, whose rays all start at t = 0, are spared code that makes them spill.
 // All 32 lanes call round(), the other members are per lane or say so.
-template <bool ANY, bool COUNT, bool SPH, bool SINGLE, bool TZERO, bool AXES, class View, class Load, class Store>
+template <bool ANY, bool COUNT, bool SPH, bool SINGLE, bool QUERY, class View, class Load, class Store>
 struct WideWarp {
   static constexpr unsigned kFull = 0xFFFFFFFFu;
   View view;
@@ -289,7 +313,6 @@ struct WideWarp {
   const WideTables &tab;
   TraceCounts *cnt;
   const uint32_t lane;
-  const bool seq;
   uint2 *stack;
   WideRay w{};
   WideGroup ng{0u, 0u}, tg{0u, 0u};
@@ -328,7 +351,7 @@ struct WideWarp {
     const V3 ai = v3(fabsf(inv.x), fabsf(inv.y), fabsf(inv.z));
     const float least = fminf(ai.x, fminf(ai.y, ai.z)), most = fmaxf(ai.x, fmaxf(ai.y, ai.z));
     const float zero = least * kWideZero, scale = m * least;
-    kd = active && ((!AXES && most >= zero) || !(scale >= kWideScaleMin && scale <= kWideScaleMax));
+    kd = active && ((!QUERY && most >= zero) || !(scale >= kWideScaleMin && scale <= kWideScaleMax));
     active = active && !kd;
     if (active) {
       float t0, t1;
@@ -353,12 +376,12 @@ struct WideWarp {
       sh.b[lane] = make_float4(pre.sx, pre.sy, pre.sz, r.tmax);
       if (!SINGLE) sh.tris[lane] = s.wtris;
       sh.k[lane] = (uint32_t)pre.kx | ((uint32_t)pre.ky << 2) | ((uint32_t)pre.kz << 4);
-      if (AXES)
+      if (QUERY)
         sh.zero[lane] = most < zero ? (uint8_t)0
                                     : (uint8_t)((ai.x >= zero ? 1u : 0u) | (ai.y >= zero ? 2u : 0u) | (ai.z >= zero ? 4u : 0u));
     }
     if (!ANY) sh.key[lane] = ((unsigned long long)wide_order(best) << 32) | (sphere >= 0 ? 0xFFFFFFFEu : 0xFFFFFFFFu);
-    if (!ANY || AXES) sh.tie[lane] = 0xFFFFFFFFu;
+    if (!ANY || QUERY) sh.tie[lane] = 0xFFFFFFFFu;
   }
 
   // one node of the lane's ray: its triangles into tg, its inner children pending
@@ -368,7 +391,7 @@ struct WideWarp {
     ng.bits &= ~(1u << slot);
     if (ng.bits & 0xFFu) stack[sp++] = make_uint2(ng.base, ng.bits);
     if (COUNT) cnt->nodes++;
-    wide_node(SINGLE ? view(0u).wnodes : nodes, idx, w, TZERO ? 0.0f : w.tmin, tab, ng, tg, tvalid);
+    wide_node(SINGLE ? view(0u).wnodes : nodes, idx, w, QUERY ? w.tmin : 0.0f, tab, ng, tg, tvalid);
     if (!(ng.bits & 0xFFu)) {
       if (sp == 0) {
         active = false;
@@ -406,8 +429,8 @@ struct WideWarp {
       if (COUNT) cnt->tris++;
       float t, b1, b2;
       if (intersect_tri(p, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), (f_bits(b.w) & 1u) != 0u,
-                        TZERO ? 0.0f : ra.w, rb.w, t, b1, b2)) {
-        const uint32_t axes = AXES ? sh.zero[o] : 0u;
+                        QUERY ? ra.w : 0.0f, rb.w, t, b1, b2)) {
+        const uint32_t axes = QUERY ? sh.zero[o] : 0u;
         const bool beside = axes != 0u && wide_beside(axes, p.o, t, lt + q);
         if (beside) atomicMin(&sh.tie[o], wide_order(t));
         if (ANY) {
@@ -445,7 +468,7 @@ struct WideWarp {
     uint32_t rec = 0xFFFFFFFFu;
     if (ANY) {
       if (found) h.prim = 0;
-      if (AXES) kd = kd || (!found && sh.tie[lane] != 0xFFFFFFFFu);
+      if (QUERY) kd = kd || (!found && sh.tie[lane] != 0xFFFFFFFFu);
     } else {
       const unsigned long long key = sh.key[lane];
       h.t = wide_unorder((uint32_t)(key >> 32));
@@ -457,7 +480,7 @@ struct WideWarp {
       Ray r;
       load(i, r);
       if (kd) {
-        kd_ray<ANY, SPH>(s, r, seq, h);
+        kd_ray<ANY, SPH, QUERY>(s, r, h);
       } else {
         // the winner again, for its barycentrics: the same inputs, the same result
         const int64_t q = 3 * (int64_t)rec;
@@ -497,8 +520,8 @@ struct WideAll {
 // lie in a queue with their neighbours: a lane that ends early waits, which costs less than what the other
 // shape (below) adds to the node loop's registers (mid frame 83.7 against 92 ms).
 // All 32 lanes of every warp must call this.
-template <bool ANY, bool COUNT, bool SPH, bool SINGLE, bool TZERO, class Rays, class View, class Load, class Store>
-__device__ __forceinline__ void wide_trace(const Rays &rays, View view, uint32_t n, Load load, Store store, bool seq,
+template <bool ANY, bool COUNT, bool SPH, bool SINGLE, class Rays, class View, class Load, class Store>
+__device__ __forceinline__ void wide_trace(const Rays &rays, View view, uint32_t n, Load load, Store store,
                                            WideShared &sh, const WideTables &tab, uint32_t *next, TraceCounts *cnt,
                                            uint32_t &rays_done) {
   constexpr unsigned kFull = 0xFFFFFFFFu;
@@ -511,7 +534,7 @@ __device__ __forceinline__ void wide_trace(const Rays &rays, View view, uint32_t
     if (first >= n) break;
     const uint32_t i = (uint32_t)first + lane;
     __syncwarp(kFull);  // the previous rays' readers are done with the shared records
-    WideWarp<ANY, COUNT, SPH, SINGLE, TZERO, false, View, Load, Store> t{view, load, store, sh, tab, cnt, lane, seq, stack};
+    WideWarp<ANY, COUNT, SPH, SINGLE, false, View, Load, Store> t{view, load, store, sh, tab, cnt, lane, stack};
     if (i < n) {
       t.start(i);
       ++rays_done;
@@ -537,12 +560,12 @@ __device__ __forceinline__ void wide_trace(const Rays &rays, View view, uint32_t
 constexpr uint32_t kWideRefill = 16u;
 
 template <bool ANY, bool SPH, class View, class Load, class Store>
-__device__ __forceinline__ void wide_trace_refill(View view, uint32_t n, Load load, Store store, bool seq, WideShared &sh,
+__device__ __forceinline__ void wide_trace_refill(View view, uint32_t n, Load load, Store store, WideShared &sh,
                                                   const WideTables &tab, uint32_t *next) {
   constexpr unsigned kFull = 0xFFFFFFFFu;
   uint2 stack[kWideMaxDepth];
   const WideChunks chunks(n);
-  WideWarp<ANY, false, SPH, true, false, true, View, Load, Store> t{view, load, store, sh, tab, nullptr, threadIdx.x & 31u, seq, stack};
+  WideWarp<ANY, false, SPH, true, true, View, Load, Store> t{view, load, store, sh, tab, nullptr, threadIdx.x & 31u, stack};
   uint32_t i = 0u;
   bool have = false;  // the lane holds ray i
   bool more = true;   // the block has rays left (uniform over the warp)

@@ -95,7 +95,6 @@ struct RenderArgs {
   unsigned long long *stats;     // [0] extension rays, [1] shadow rays, [2] truncated paths, [3] bounces
   unsigned long long *tcount;    // counted mode: ext nodes, refs, tris, rays; shadow nodes, refs, tris, rays
   int32_t max_b;
-  int32_t seq;                   // near ties are decided as the one-ray-per-lane kd-tree kernels do
   SceneView view0;               // the scene of a wave of one scene (njobs == 1)
 };
 
@@ -317,8 +316,8 @@ __global__ void __launch_bounds__(kGenBlock) k_generate(const __grid_constant__ 
 }
 
 // extend: closest hit for the live queue of bounce b
-// Traversal: the 8-wide hierarchy (hd_wide.h), or the kd-tree, one ray per lane, for a scene that has
-// none and with mgpu_tune_set("wide", 0).
+// Traversal: the 8-wide hierarchy (hd_wide.h), or the kd-tree, one ray per lane, where no scene of a render has
+// one and with mgpu_tune_set("wide", 0).
 struct WideBlockShared {
   WideShared warp[kWideBlock / 32];
   WideTables tables;
@@ -358,9 +357,9 @@ __device__ __forceinline__ void wide_extend(const RenderArgs &a, int b, WideBloc
   WideShared &sh = ws.warp[threadIdx.x >> 5];
   uint32_t *next = &ws.next_extend;
   if (a.njobs == 1)
-    wide_trace<false, COUNT, SPH, true, true>(WideChunks(n), view0, n, load, store, SPH, sh, ws.tables, next, c, rays);
+    wide_trace<false, COUNT, SPH, true>(WideChunks(n), view0, n, load, store, sh, ws.tables, next, c, rays);
   else
-    wide_trace<false, COUNT, SPH, false, true>(WideChunks(n), view_of, n, load, store, SPH, sh, ws.tables, next, c, rays);
+    wide_trace<false, COUNT, SPH, false>(WideChunks(n), view_of, n, load, store, sh, ws.tables, next, c, rays);
 }
 
 // occlusion of bounce b's light samples, by the hierarchy; an occluded sample's slot is zeroed
@@ -387,9 +386,9 @@ __device__ __forceinline__ void wide_shadow(const RenderArgs &a, int b, WideBloc
   WideShared &sh = ws.warp[threadIdx.x >> 5];
   uint32_t *next = &ws.next;
   if (a.njobs == 1)
-    wide_trace<true, COUNT, SPH, true, true>(WideChunks(n), view0, n, load, store, SPH, sh, ws.tables, next, c, rays);
+    wide_trace<true, COUNT, SPH, true>(WideChunks(n), view0, n, load, store, sh, ws.tables, next, c, rays);
   else
-    wide_trace<true, COUNT, SPH, false, true>(WideChunks(n), view_of, n, load, store, SPH, sh, ws.tables, next, c, rays);
+    wide_trace<true, COUNT, SPH, false>(WideChunks(n), view_of, n, load, store, sh, ws.tables, next, c, rays);
 }
 
 // Bounce b + 1's closest hits and bounce b's occlusion queries, which do not depend on each other: one launch,
@@ -422,11 +421,10 @@ __global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMi
       r.d = v3(d.x, d.y, d.z);
       r.tmax = INFINITY;
     };
-    auto store = [&](uint32_t i, bool hit, const TravState &st) {
-      qhit[i] = make_float4(hit ? st.best : INFINITY, __int_as_float(hit ? st.best_prim : -1), hit ? st.bb1 : 0.0f,
-                            hit ? st.bb2 : 0.0f);
+    auto store = [&](uint32_t i, bool hit, const Hit &h) {
+      qhit[i] = make_float4(hit ? h.t : INFINITY, __int_as_float(hit ? h.prim : -1), hit ? h.b1 : 0.0f, hit ? h.b2 : 0.0f);
     };
-    grid_trace<false, COUNT, SPH>(view_of, nullptr, 0, a.counters[kCtrRay + b], load, store, &c, rays);
+    kd_grid<false, COUNT, SPH>(view_of, a.counters[kCtrRay + b], load, store, &c, rays);
   }
   if (COUNT && rays + c.nodes + c.tris) {
     atomicAdd(&a.tcount[0], (unsigned long long)c.nodes);
@@ -543,7 +541,7 @@ template <bool SPH>
 __device__ __noinline__ void block_extend(const RenderArgs &a, ShadeShared &sh, int b, uint32_t base, uint32_t n) {
   const float4 *qo = a.qo[b & 1] + base, *qd = a.qd[b & 1] + base;
   uint32_t done = 0u;
-  wide_trace<false, false, SPH, false, true>(
+  wide_trace<false, false, SPH, false>(
       WideAll(), [&](uint32_t i) -> const SceneView & { return a.jobs[__float_as_int(qd[i].w)].view; }, n - base,
       [&](uint32_t i, Ray &r) {
         const float4 o = qo[i], d = qd[i];
@@ -556,14 +554,14 @@ __device__ __noinline__ void block_extend(const RenderArgs &a, ShadeShared &sh, 
         a.qhit[base + i] = make_float4(hit ? h.t : INFINITY, __int_as_float(hit ? h.prim : -1), hit ? h.b1 : 0.0f,
                                        hit ? h.b2 : 0.0f);
       },
-      a.seq != 0, sh.wide[threadIdx.x >> 5], sh.tables, &sh.next, nullptr, done);
+      sh.wide[threadIdx.x >> 5], sh.tables, &sh.next, nullptr, done);
 }
 
 template <bool SPH>
 __device__ __noinline__ void block_shadow(const RenderArgs &a, ShadeShared &sh, const float4 *so, const float4 *sd,
                                           uint32_t n) {
   uint32_t done = 0u;
-  wide_trace<true, false, SPH, false, true>(
+  wide_trace<true, false, SPH, false>(
       WideAll(),
       [&](uint32_t i) -> const SceneView & {
         return a.njobs == 1 ? a.jobs[0].view : a.jobs[a.path_job[__float_as_uint(so[i].w) / (uint32_t)a.nl_stride]].view;
@@ -579,7 +577,7 @@ __device__ __noinline__ void block_shadow(const RenderArgs &a, ShadeShared &sh, 
       [&](uint32_t i, bool hit, const Hit &) {
         if (hit) a.slots[__float_as_uint(so[i].w)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       },
-      a.seq != 0, sh.wide[threadIdx.x >> 5], sh.tables, &sh.next, nullptr, done);
+      sh.wide[threadIdx.x >> 5], sh.tables, &sh.next, nullptr, done);
 }
 
 // SURF: the wave has a scene with image maps, a background or analytic spheres.  Scenes without
@@ -877,10 +875,10 @@ __global__ void __launch_bounds__(WIDE ? kWideBlock : kBlock, WIDE ? 1 : kTravMi
       r.d = v3(d.x, d.y, d.z);
       r.tmax = d.w;
     };
-    auto store = [&](uint32_t i, bool hit, const TravState &) {
+    auto store = [&](uint32_t i, bool hit, const Hit &) {
       if (hit) slots[__float_as_uint(so[i].w)] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     };
-    grid_trace<true, COUNT, SPH>(view_of, nullptr, 0, a.counters[kCtrNee + b], load, store, &c, rays);
+    kd_grid<true, COUNT, SPH>(view_of, a.counters[kCtrNee + b], load, store, &c, rays);
   }
   if (COUNT && rays + c.nodes + c.tris) {
     atomicAdd(&a.tcount[4], (unsigned long long)c.nodes);
@@ -1602,24 +1600,11 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
     MGPU_CUDA(cudaMemcpyAsync(w->jobs, all.data(), all.size() * sizeof(JobArgs), cudaMemcpyHostToDevice, st));
   }
 
-  bool sph = false;  // a job's scene has analytic spheres: the traversal kernels that test them
   bool sort_hits = false;
-  bool wide = g_tune.wide.load() != 0;  // every scene has the 8-wide hierarchy
-  for (const Job &j : jobs) {
-    sort_hits = sort_hits || j.scene->mixed;
-    sph = sph || j.scene->view.nsphere > 0;
-    wide = wide && (j.scene->view.wnodes != nullptr || j.scene->view.ntri == 0);
-  }
-  auto kext = !wide ? k_extend<COUNT, false, true> : sph ? k_extend<COUNT, true, true> : k_extend<COUNT, true, false>;
-  auto kshw = !wide ? k_shadow<COUNT, false, true> : sph ? k_shadow<COUNT, true, true> : k_shadow<COUNT, true, false>;
-  auto ktrv = sph ? k_traverse<true> : k_traverse<false>;
-  const int tb = wide ? kWideBlock : kBlock;
-  const size_t tsm = wide ? (size_t)kWideSmem : 0;
+  for (const Job &j : jobs) sort_hits = sort_hits || j.scene->mixed;
   MGPU_CUDA(kernel_attributes());
   const int g_gen = grid_for((const void *)k_generate, 0, kGenBlock);
-  const int g_ext = grid_for((const void *)kext, tsm, tb);
   const int g_sha = grid_for((const void *)k_shade<true, false>, sizeof(ShadeShared), kShadeTile);
-  const int g_shw = grid_for((const void *)kshw, tsm, tb);
   const int g_acc = grid_for((const void *)k_accumulate, 0);
   const int g_bin = device_sm_count() * 4;
   const int bin_ext = g_tune.bin_extension.load();
@@ -1675,8 +1660,21 @@ static int render_jobs(const std::vector<Job> &jobs, void *stream, bool noalloc,
     a.stats = w->stats;
     a.tcount = w->tcount;
     a.max_b = wv.max_b;
-    a.seq = sph ? 1 : 0;
     const int max_b = wv.max_b;
+    bool sph = false;   // a chunk's scene has analytic spheres: the traversal kernels that test them
+    bool wide = false;  // ... has the hierarchy, or no triangles; the rays of one that has not take the kd-tree
+    for (const JobArgs &c : wv.chunks) {
+      sph = sph || c.view.nsphere > 0;
+      wide = wide || c.view.wnodes != nullptr || c.view.ntri == 0;
+    }
+    wide = wide && g_tune.wide.load() != 0;
+    auto kext = !wide ? k_extend<COUNT, false, true> : sph ? k_extend<COUNT, true, true> : k_extend<COUNT, true, false>;
+    auto kshw = !wide ? k_shadow<COUNT, false, true> : sph ? k_shadow<COUNT, true, true> : k_shadow<COUNT, true, false>;
+    auto ktrv = sph ? k_traverse<true> : k_traverse<false>;
+    const int tb = wide ? kWideBlock : kBlock;
+    const size_t tsm = wide ? (size_t)kWideSmem : 0;
+    const int g_ext = grid_for((const void *)kext, tsm, tb);
+    const int g_shw = grid_for((const void *)kshw, tsm, tb);
     bool splats = false;  // a chunk's film has a reconstruction filter
     for (const JobArgs &c : wv.chunks) splats = splats || c.film_fx != nullptr;
     bool surf = false;  // a chunk's scene has image maps, a background or analytic spheres

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(kTraceWideBlock, 4)
     if (ANY) occ[i] = hit ? 1 : 0;
     else hits[i] = make_float4(hit ? h.t : INFINITY, __int_as_float(hit ? h.prim : -1), hit ? h.b1 : 0.0f, hit ? h.b2 : 0.0f);
   };
-  wide_trace_refill<ANY, true>([&](uint32_t) -> const SceneView & { return s; }, n, load, store, true,
+  wide_trace_refill<ANY, true>([&](uint32_t) -> const SceneView & { return s; }, n, load, store,
                                wsh[threadIdx.x >> 5], tables, &next);
 }
 

@@ -331,3 +331,55 @@ def test_directions_of_any_length(cuda, length):
     wide, _ = gpu_trace(cuda, ds, rays)
     assert np.array_equal(kd.view(np.uint32), wide.view(np.uint32))
     assert np.array_equal(gpu_any(cuda, ds, rays) != 0, kd[:, 1].view(np.int32) >= 0)
+
+
+def _overlaid(kind):
+    """Every triangle twice, with two materials; "none": and one whose coordinates the hierarchy does not hold."""
+    b = SceneBuilder()
+    m = [b.material(diffuse(0.8)), b.material(diffuse(0.1)), b.material(dielectric(1.5))]
+    t = _random_tris(300, 5, size=0.4).astype(np.float32)
+    n = np.broadcast_to(np.float32([0, 0, 1]), t.shape)
+    for k in (0, 1, 0, 2):
+        b.add(f"t{k}", t[::-1] if k else t, n, m[k])
+    b.add_quad_light("l", (0.0, 0.0, 2.5), (0.5, 0.0, 0.0), (0.0, 0.5, 0.0), 8.0, m[0])
+    if kind == "none":
+        b.add("far", np.float32([[[2e37, 0, 0], [2e37, 1, 0], [2e37, 0, 1]]]), np.float32([[[1, 0, 0]] * 3]), m[0])
+    if kind == "spheres":
+        b.add_sphere((0.2, 0.1, 0.3), 0.2, m[1])
+    return b.build(camera(eye=(0, 0, 3), look=(0, 0, -1), up=(0, 1, 0), height_angle=40.0, aspect=1.0))
+
+
+@pytest.mark.parametrize("whole", [0, -1])
+def test_overlaid_surfaces_do_not_depend_on_the_batch(cuda, whole):
+    # which of two coincident triangles a ray reports is decided by its scene, whatever shares the wave and
+    # whichever structure the scene's rays traverse
+    scenes = {k: _overlaid(k) for k in ("plain", "spheres", "none")}
+    ds = {k: pt.DeviceScene(s, pt.Accel(s)) for k, s in scenes.items()}
+    st = pt.RenderSettings(45, 37, 4, max_depth=4, rr_start_depth=3, seed=12)
+
+    def films(kinds, batch):
+        out = [pt.Film(45, 37) for _ in kinds]
+        if batch:
+            b = pt.Batch()
+            for k, f in zip(kinds, out):
+                b.add(ds[k], st, f)
+            b.render()
+        else:
+            for k, f in zip(kinds, out):
+                pt.render(ds[k], st, f)
+        return {k: np.array(f.raw()).view(np.uint32) for k, f in zip(kinds, out)}
+
+    try:
+        pt.tune("whole_paths", whole)
+        alone = films(scenes, False)
+        assert all(a.any() for a in alone.values())
+        groups = [films(g, True) for g in (("plain", "spheres"), ("plain", "none"), ("spheres", "none"),
+                                           ("plain", "spheres", "none"))]
+        pt.tune("wide", 0)
+        groups += [films(scenes, False), films(scenes, True)]
+    finally:
+        pt.tune("wide", 1)
+        pt.tune("whole_paths", -1)
+    for i, g in enumerate(groups):
+        for k, a in g.items():
+            assert np.array_equal(alone[k], a), (i, k, int((alone[k] != a).sum()))
