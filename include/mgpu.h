@@ -239,6 +239,8 @@ int mgpu_accel_destroy(mgpu_accel *accel);
 int mgpu_scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void *stream, mgpu_scene **out);
 int mgpu_scene_destroy(mgpu_scene *scene);
 int mgpu_scene_bytes(const mgpu_scene *scene, uint64_t *out);
+/* Nodes of the scene's 8-wide hierarchy; 0: it has none and its rays traverse the kd-tree. */
+int mgpu_scene_hierarchy(const mgpu_scene *scene, uint64_t *out_nodes);
 /* Device bytes mgpu_scene_create would allocate for this accel with nmat materials and nlight
  * lights (admission against a memory budget before uploading).  No reference counterpart. */
 int mgpu_accel_device_bytes(const mgpu_accel *accel, int32_t nmat, int32_t nlight, uint64_t *out);

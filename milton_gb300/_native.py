@@ -91,6 +91,7 @@ SIGNATURES = [
     ("mgpu_accel_destroy", C.c_int, [C.c_void_p]),
     ("mgpu_scene_create", C.c_int, [C.POINTER(SceneDesc), C.c_void_p, C.c_void_p, C.POINTER(C.c_void_p)]),
     ("mgpu_scene_destroy", C.c_int, [C.c_void_p]),
+    ("mgpu_scene_hierarchy", C.c_int, [C.c_void_p, C.POINTER(C.c_uint64)]),
     ("mgpu_scene_bytes", C.c_int, [C.c_void_p, C.POINTER(C.c_uint64)]),
     ("mgpu_scene_set_top_pairs", C.c_int, [C.c_void_p, C.c_uint32]),
     ("mgpu_accel_device_bytes", C.c_int, [C.c_void_p, C.c_int32, C.c_int32, C.POINTER(C.c_uint64)]),

@@ -602,20 +602,24 @@ int mgpu_scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void
   for (int i = 1; i < desc->nmat; ++i) s->mixed = s->mixed || desc->materials[16 * i] != desc->materials[0];
   s->nlight = desc->nlight;
   bool wide = false;
-  uint32_t wide_nodes = 0;
   s->view.wextent = 0.0f;
   for (int k = 0; k < 3; ++k) {
     const float c = 0.5f * s->view.bmin[k] + 0.5f * s->view.bmax[k];
     s->view.wcentre[k] = std::isfinite(c) ? c : 0.0f;
-    s->view.wextent = std::max(s->view.wextent, std::max(s->view.bmax[k] - s->view.wcentre[k], s->view.wcentre[k] - s->view.bmin[k]));
+    // (a scene of points only has no bounds)
+    const float lo = std::min(s->view.bmin[k], (float)tr.tmin[k]), hi = std::max(s->view.bmax[k], (float)tr.tmax[k]);
+    s->view.wextent = std::max(s->view.wextent, std::max(hi - s->view.wcentre[k], s->view.wcentre[k] - lo));
   }
   if (int rc = wide_build(s->view.tris, T, s->view, base + L.off_wnodes, (F4 *)(base + L.off_wtris), base + L.off_wscratch, st,
-                          &wide_nodes, &wide)) {
+                          &s->wide_nodes, &wide)) {
     cudaFree(s->d_block);
     delete s;
     return rc;
   }
-  if (!wide) s->view.wextent = INFINITY;
+  if (!wide) {
+    s->view.wextent = INFINITY;
+    s->wide_nodes = 0;
+  }
   s->view.wnodes = wide ? (const uint32_t *)(base + L.off_wnodes) : nullptr;
   s->view.wtris = wide ? (const F4 *)(base + L.off_wtris) : nullptr;
   // staging the top of the tree in shared memory costs more occupancy than it saves on GB300
@@ -651,6 +655,12 @@ int mgpu_scene_set_top_pairs(mgpu_scene *s, uint32_t n) {
 int mgpu_scene_bytes(const mgpu_scene *s, uint64_t *out) {
   if (!s || !out) return fail(MGPU_E_INVALID, "mgpu_scene_bytes: null argument");
   *out = s->bytes;
+  return MGPU_OK;
+}
+
+int mgpu_scene_hierarchy(const mgpu_scene *s, uint64_t *out) {
+  if (!s || !out) return fail(MGPU_E_INVALID, "mgpu_scene_hierarchy: null argument");
+  *out = s->wide_nodes;
   return MGPU_OK;
 }
 

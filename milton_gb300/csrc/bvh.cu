@@ -115,12 +115,25 @@ __device__ __forceinline__ float unorder_bits(uint32_t u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
 }
 
-__device__ __forceinline__ Box tri_box(const F4 *tris, int64_t t) {
-  const F4 a = load_f4(tris, 3 * t), b = load_f4(tris, 3 * t + 1), c = load_f4(tris, 3 * t + 2);
+// Whether a triangle reaches out of the kd-tree's root box.  The root box leaves out triangles whose bounds compare
+// equal under Milton's fuzzy comparison (flat ones from -1 to 1, kdbuild.cpp); rays find such a triangle only
+// where a leaf on their way through the root box lists it, wherever they hit it.  Its records carry
+// kWideOutside, and the kd-tree decides a ray that hits one before anything else.
+__device__ __forceinline__ bool sticks_out(const Build &B, const Box &b) {
+  bool out = false;
+  for (int k = 0; k < 3; ++k) out = out || b.lo[k] < B.bmin[k] || b.hi[k] > B.bmax[k];
+  return out;
+}
+
+__device__ __forceinline__ Box tri_box(const Build &B, int64_t t) {
+  const F4 a = load_f4(B.tris, 3 * t), b = load_f4(B.tris, 3 * t + 1), c = load_f4(B.tris, 3 * t + 2);
   Box r;
   r.lo[0] = fminf(a.x, fminf(b.x, c.x)); r.hi[0] = fmaxf(a.x, fmaxf(b.x, c.x));
   r.lo[1] = fminf(a.y, fminf(b.y, c.y)); r.hi[1] = fmaxf(a.y, fmaxf(b.y, c.y));
   r.lo[2] = fminf(a.z, fminf(b.z, c.z)); r.hi[2] = fmaxf(a.z, fmaxf(b.z, c.z));
+  // nothing hits a point, and the kd-tree's bounds leave it out: it must not widen the hierarchy's
+  if (r.lo[0] == r.hi[0] && r.lo[1] == r.hi[1] && r.lo[2] == r.hi[2])
+    for (int k = 0; k < 3; ++k) r.lo[k] = r.hi[k] = fminf(fmaxf(r.lo[k], B.bmin[k]), B.bmax[k]);
   return r;
 }
 
@@ -140,7 +153,7 @@ __global__ void k_bvh_init(Build B) {
 __device__ void centre_bounds(const Build &B, int64_t first, int64_t stride, uint32_t *g) {
   float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (int64_t t = first; t < B.n; t += stride) {
-    const Box b = tri_box(B.tris, t);
+    const Box b = tri_box(B, t);
     for (int k = 0; k < 3; ++k) {
       const float c = 0.5f * b.lo[k] + 0.5f * b.hi[k];
       lo[k] = fminf(lo[k], c);
@@ -179,7 +192,7 @@ __device__ __forceinline__ uint64_t morton_key(const Build &B, const uint32_t *g
     ext = fmaxf(ext, unorder_bits(g[3 + k]) - lo[k]);
   }
   const float scale = ext > 0.0f ? 65535.0f / ext : 0.0f;
-  const Box b = tri_box(B.tris, t);
+  const Box b = tri_box(B, t);
   uint32_t c[3];
   for (int k = 0; k < 3; ++k)
     c[k] = (uint32_t)fminf(fmaxf((0.5f * b.lo[k] + 0.5f * b.hi[k] - lo[k]) * scale, 0.0f), 65535.0f);
@@ -305,7 +318,7 @@ __global__ void __launch_bounds__(256) k_bvh_radix_scatter(const uint64_t *__res
 
 __device__ __forceinline__ Box make_leaf(const Build &B, int64_t i, int32_t t) {
   BNode nd;
-  nd.box = tri_box(B.tris, t);
+  nd.box = tri_box(B, t);
   nd.left = t;
   nd.right = -1;
   B.node[i] = nd;
@@ -764,11 +777,6 @@ __device__ void emit_node(const Build &B, uint32_t w, bool valid, int32_t *xn, i
     mid[k] = 0.5f * lo + 0.5f * hi;
     fits = fits && fmaxf(fabsf(lo), fabsf(hi)) <= 1.0e37f;  // the stored planes are finite
   }
-  // The kd-tree's root box leaves out triangles whose bounds compare equal under Milton's fuzzy comparison (flat
-  // ones from -1 to 1, kdbuild.cpp), and rays find such a triangle only inside that box.  A scene with one
-  // that sticks out keeps the kd-tree's answers, and its traversal.
-  if (w == 0u)
-    for (int k = 0; k < 3; ++k) fits = fits && box.lo[k] >= B.bmin[k] && box.hi[k] <= B.bmax[k];
   const int cnt = x < 0 || !leaf ? 0 : (x < B.n ? 1 : (int)B.cut[x - B.n].prims);
   const uint32_t imask = __reduce_or_sync(group, x >= 0 && !leaf ? 1u << slot : 0u);
   const uint32_t tvalid = __reduce_or_sync(group, cnt ? ((1u << cnt) - 1u) << (3 * slot) : 0u);
@@ -812,7 +820,7 @@ __device__ void emit_node(const Build &B, uint32_t w, bool valid, int32_t *xn, i
         const int64_t t = B.node[y].left;
         F4 a = load_f4(B.tris, 3 * t), bb = load_f4(B.tris, 3 * t + 1);
         const F4 c = load_f4(B.tris, 3 * t + 2);
-        bb.w = a.w;  // flags
+        bb.w = __uint_as_float((__float_as_uint(a.w) & 1u) | (sticks_out(B, B.node[y].box) ? kWideOutside : 0u));
         a.w = __int_as_float((int)t);
         B.wtris[3 * (size_t)at] = a;
         B.wtris[3 * (size_t)at + 1] = bb;

@@ -87,6 +87,7 @@ struct mgpu_scene {
   uint32_t top_pairs_max = 0;   // breadth-first pairs available for staging
   void *d_block = nullptr;      // one allocation holding everything above
   uint64_t bytes = 0;
+  uint32_t wide_nodes = 0;      // nodes of the 8-wide hierarchy, 0: none
   uint32_t *d_err = nullptr;    // device error word
 };
 

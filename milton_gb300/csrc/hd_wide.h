@@ -25,7 +25,7 @@
 //   7      unused
 //   8 + 3 s + k   slot s's planes along axis k, relative to the centre: the upper halves of two floats, low
 //          plane in bits 0..15, high plane in bits 16..31
-// Triangle record: 3 x float4 as a kd leaf's (v0 + primitive id, v1 + flags, v2).
+// Triangle record: 3 x float4 as a kd leaf's (v0 + primitive id, v1 + flags, v2); flags: 1 = culled, kWideOutside.
 //
 // A slot's number says where its child lies: bit k set = the upper side along axis k.  A ray visits
 // the children it meets in the order of slot XOR octant (its negative directions), which is front to
@@ -39,6 +39,7 @@ namespace mgpu {
 constexpr int kWideWords = 32;       // 32-bit words per node
 constexpr int kWideLeafTris = 3;     // triangles per leaf child
 constexpr int kWideMaxDepth = 30;    // levels of node below the root that the traversal stack holds
+constexpr uint32_t kWideOutside = 2u;  // flag of a triangle record: it reaches out of the kd-tree's root box (bvh.cu)
 constexpr uint32_t kWideRootBits = 0x101u;  // pending slots and inner mask of the root's pseudo parent
 // Threads per block: one block per SM at 64 registers a thread.  The rays of one SM are then
 // neighbours in the (sorted) queue and share its L1: mid frame, traversal 117 ms in blocks of 128,
@@ -191,7 +192,8 @@ struct WideShared {
   int32_t sphere[32];        // analytic sphere hit before the traversal, -1: none
   const F4 *tris[32];        // the lanes' scenes' triangle records (waves of several scenes)
   uint8_t zero[32];          // axes of zero direction components
-  uint32_t tie[32];          // ordered t of the nearest hit that the kd-tree has to decide (kWideTie, wide_beside)
+  uint32_t tie[32];          // ordered t of the nearest hit that the kd-tree has to decide (kWideTie, wide_beside);
+                             // any hit: 0, if there is one (kWideOutside, wide_beside)
 };
 
 __device__ __forceinline__ uint32_t wide_order(float f) {
@@ -381,7 +383,7 @@ struct WideWarp {
                                     : (uint8_t)((ai.x >= zero ? 1u : 0u) | (ai.y >= zero ? 2u : 0u) | (ai.z >= zero ? 4u : 0u));
     }
     if (!ANY) sh.key[lane] = ((unsigned long long)wide_order(best) << 32) | (sphere >= 0 ? 0xFFFFFFFEu : 0xFFFFFFFFu);
-    if (!ANY || QUERY) sh.tie[lane] = 0xFFFFFFFFu;
+    sh.tie[lane] = 0xFFFFFFFFu;
   }
 
   // one node of the lane's ray: its triangles into tg, its inner children pending
@@ -431,11 +433,12 @@ struct WideWarp {
       if (intersect_tri(p, v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z), (f_bits(b.w) & 1u) != 0u,
                         QUERY ? ra.w : 0.0f, rb.w, t, b1, b2)) {
         const uint32_t axes = QUERY ? sh.zero[o] : 0u;
-        const bool beside = axes != 0u && wide_beside(axes, p.o, t, lt + q);
-        if (beside) atomicMin(&sh.tie[o], wide_order(t));
+        const bool doubt = (ANY && (f_bits(b.w) & kWideOutside) != 0u) || (axes != 0u && wide_beside(axes, p.o, t, lt + q));
         if (ANY) {
-          if (!beside) hit = 1u << o;
+          hit = 1u << o;
+          if (doubt) sh.tie[o] = 0u;
         } else {
+          if (doubt) atomicMin(&sh.tie[o], wide_order(t));
           const unsigned long long old = atomicMin(&sh.key[o], ((unsigned long long)wide_order(t) << 32) | rec);
           const float told = wide_unorder((uint32_t)(old >> 32));
           if ((uint32_t)old != 0xFFFFFFFFu && fabsf(t - told) <= kWideTie * fabsf(t))
@@ -468,13 +471,19 @@ struct WideWarp {
     uint32_t rec = 0xFFFFFFFFu;
     if (ANY) {
       if (found) h.prim = 0;
-      if (QUERY) kd = kd || (!found && sh.tie[lane] != 0xFFFFFFFFu);
+      kd = kd || sh.tie[lane] == 0u;
     } else {
       const unsigned long long key = sh.key[lane];
       h.t = wide_unorder((uint32_t)(key >> 32));
       rec = (uint32_t)key;
       // (a pair behind the final hit is no tie)
       kd = kd || (sh.tie[lane] != 0xFFFFFFFFu && wide_unorder(sh.tie[lane]) - h.t <= kWideTie * fabsf(h.t));
+    }
+    const int64_t q = 3 * (int64_t)rec;
+    F4 b = {};
+    if (!ANY && rec < 0xFFFFFFFEu) {
+      b = load_f4(s.wtris, q + 1);
+      kd = kd || (f_bits(b.w) & kWideOutside) != 0u;
     }
     if (kd || (!ANY && rec < 0xFFFFFFFEu)) {
       Ray r;
@@ -483,8 +492,7 @@ struct WideWarp {
         kd_ray<ANY, SPH, QUERY>(s, r, h);
       } else {
         // the winner again, for its barycentrics: the same inputs, the same result
-        const int64_t q = 3 * (int64_t)rec;
-        const F4 a = load_f4(s.wtris, q), b = load_f4(s.wtris, q + 1), c = load_f4(s.wtris, q + 2);
+        const F4 a = load_f4(s.wtris, q), c = load_f4(s.wtris, q + 2);
         float t;
         intersect_tri(precompute(r), v3(a.x, a.y, a.z), v3(b.x, b.y, b.z), v3(c.x, c.y, c.z),
                       (f_bits(b.w) & 1u) != 0u, r.tmin, r.tmax, t, h.b1, h.b2);
@@ -549,6 +557,7 @@ __device__ __forceinline__ void wide_trace(const Rays &rays, View view, uint32_t
       if (t.qn >= kWideFlush) t.round(t.qn);
     }
     if (t.qn) t.round(t.qn);
+    if (ANY) __syncwarp(kFull);  // sh.tie (a round of closest hits ends with one)
     if (i < n) t.finish(i);
   }
 }
@@ -571,7 +580,7 @@ __device__ __forceinline__ void wide_trace_refill(View view, uint32_t n, Load lo
   bool more = true;   // the block has rays left (uniform over the warp)
   for (bool swap = true;;) {
     if (swap) {
-      __syncwarp(kFull);
+      if (ANY) __syncwarp(kFull);  // sh.tie
       if (have && !t.active) {
         t.finish(i);
         have = false;

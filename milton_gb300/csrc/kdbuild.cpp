@@ -376,7 +376,10 @@ bool kd_build(const float *v, int64_t ntri, const KdParams &p, KdTree &out, cons
   std::vector<float> tmn((size_t)ntri * 3), tmx((size_t)ntri * 3);
   std::vector<uint8_t> point((size_t)ntri);
   Box root;
-  for (int k = 0; k < 3; ++k) { root.mn[k] = INFINITY; root.mx[k] = -INFINITY; }
+  for (int k = 0; k < 3; ++k) {
+    root.mn[k] = out.tmin[k] = INFINITY;
+    root.mx[k] = out.tmax[k] = -INFINITY;
+  }
   for (int64_t t = 0; t < ntri; ++t) {
     float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (int j = 0; j < 3; ++j)
@@ -394,6 +397,8 @@ bool kd_build(const float *v, int64_t ntri, const KdParams &p, KdTree &out, cons
     if (!is_point) {
       bool same = true;
       for (int k = 0; k < 3; ++k) {
+        out.tmin[k] = std::min(out.tmin[k], (double)mn[k]);
+        out.tmax[k] = std::max(out.tmax[k], (double)mx[k]);
         double a = mn[k], b = mx[k];
         bool eq = fabs(a - b) < 1e-7 || (fabs(a - b / ((fabs(b) > fabs(a)) ? b : a)) <= 1e-7);
         same = same && eq;

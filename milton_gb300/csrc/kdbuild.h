@@ -27,7 +27,8 @@ struct KdLog {
 struct KdTree {
   std::vector<Pair> pairs;      // pair 0 = {root, unused}
   std::vector<uint32_t> refs;   // reversed leaf lists (count > 1 only)
-  double bmin[3], bmax[3];
+  double bmin[3], bmax[3];      // the root box
+  double tmin[3], tmax[3];      // bounds of all triangles but those that are points: the root box leaves some out
   uint32_t top_pairs = 0;       // pairs [0, top_pairs) are the breadth-first top of the tree
   KdLog log;
   double build_seconds = 0;

@@ -144,6 +144,13 @@ class DeviceScene:
         N.check(self._lib.mgpu_scene_bytes(self.handle, C.byref(v)))
         return v.value
 
+    @property
+    def hierarchy_nodes(self) -> int:
+        """Nodes of the 8-wide hierarchy, 0 if the scene's rays traverse the kd-tree (mgpu_scene_hierarchy)."""
+        v = C.c_uint64()
+        N.check(self._lib.mgpu_scene_hierarchy(self.handle, C.byref(v)))
+        return v.value
+
     def texels(self, tex: int, stream=None) -> np.ndarray:
         """Texture tex as the device holds it: (H, W, 4) float32 (filtered rgb, or bump gx, gy)."""
         h, w, _ = self.scene.textures[tex].rgb.shape

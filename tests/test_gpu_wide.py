@@ -202,6 +202,77 @@ def test_a_triangle_outside_the_kd_trees_root_box(cuda):
     assert np.array_equal(gpu_any(cuda, ds, rays) != 0, kd[:, 1].view(np.int32) >= 0)
 
 
+def _outside(kind):
+    """Scenes with triangles that the kd-tree's root box leaves out: flat ones from -1 to 1, and points."""
+    b = SceneBuilder()
+    m = b.material(diffuse(0.6))
+    t = (_random_tris(1500, 12, size=0.08) * 0.6).astype(np.float32)
+    up = np.float32([0, 1, 0])
+    b.add("t", t, np.broadcast_to(up, t.shape), m)
+    y = float(t[..., 1].min())
+
+    def quad(name, *c):
+        v = scenegen.quad_tris(*c)
+        b.add(name, np.asarray(v, np.float32), np.broadcast_to(up, (2, 3, 3)), m, culled=kind == "culled floor")
+
+    if kind in ("floor", "culled floor"):
+        quad("floor", (-1, y, 1), (1, y, 1), (1, y, -1), (-1, y, -1))
+    if kind == "room":
+        quad("floor", (-1, -1, 1), (1, -1, 1), (1, -1, -1), (-1, -1, -1))
+        quad("top", (-1, 1, 1), (1, 1, 1), (1, 1, -1), (-1, 1, -1))
+        quad("left", (-1, -1, 1), (-1, 1, 1), (-1, 1, -1), (-1, -1, -1))
+        quad("right", (1, -1, 1), (1, 1, 1), (1, 1, -1), (1, -1, -1))
+        quad("back", (-1, -1, -1), (1, -1, -1), (1, 1, -1), (-1, 1, -1))
+    if kind == "inside":
+        quad("cut", (-1, 0.1, 1), (1, 0.1, 1), (1, 0.1, -1), (-1, 0.1, -1))
+    if kind == "points":
+        p = np.float32([[50, 0, 0], [-3e7, 1, 2], [0.1, 0.1, 0.1], [0, 1e30, 0]])
+        b.add("points", np.repeat(p[:, None], 3, 1), np.broadcast_to(up, (4, 3, 3)), m)
+    b.add_quad_light("light", (0.0, 0.45, 0.0), (0.1, 0.0, 0.0), (0.0, 0.0, 0.12), 15.0, m)
+    return b.build(camera(eye=(0, 0.2, 1.7), look=(0, -0.1, -1), up=(0, 1, 0), height_angle=50.0, aspect=1.0))
+
+
+@pytest.mark.parametrize("kind", ["floor", "culled floor", "room", "inside", "points"])
+def test_triangles_that_the_root_box_leaves_out(cuda, kind):
+    # the scene keeps its hierarchy; what such a triangle hides, and where it can be hit, is the kd-tree's answer
+    s = _outside(kind)
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    assert ds.hierarchy_nodes > 0
+    box = _outside("none")
+    for seed in (13, 14):
+        rays = _rays(box, 6000, seed)
+        out = sphere_rays(np.full(3, -1.3), np.full(3, 1.3), 20_000, seed + 10)
+        rays = np.concatenate([rays, out]).astype(np.float32)
+        kd, _ = gpu_trace(cuda, ds, rays, counts=True)
+        wide, _ = gpu_trace(cuda, ds, rays)
+        prim = kd[:, 1].view(np.int32)
+        if kind != "points":
+            assert (prim >= 1500).any()
+        same = np.all(kd.view(np.uint32) == wide.view(np.uint32), axis=1)
+        assert same.all(), (kind, int((~same).sum()), rays[~same][:2], kd[~same][:2], wide[~same][:2])
+        assert np.array_equal(gpu_any(cuda, ds, rays) != 0, prim >= 0)
+    films = []
+    try:
+        for wide, whole in ((1, -1), (1, 0), (0, 0)):
+            pt.tune("wide", wide)
+            pt.tune("whole_paths", whole)
+            f = pt.Film(70, 50)
+            pt.render(ds, pt.RenderSettings(70, 50, 9, max_depth=5, rr_start_depth=3, seed=7), f)
+            films.append(np.array(f.raw()).view(np.uint32))
+    finally:
+        pt.tune("wide", 1)
+        pt.tune("whole_paths", -1)
+    assert all(np.array_equal(films[0], f) for f in films[1:])
+
+
+def test_which_scenes_have_the_hierarchy(cuda):
+    for kind in KINDS:
+        s = _scene(kind)
+        assert pt.DeviceScene(s, pt.Accel(s)).hierarchy_nodes > 0, kind
+    s = _overlaid("none")  # coordinates beyond what its nodes hold
+    assert pt.DeviceScene(s, pt.Accel(s)).hierarchy_nodes == 0
+
+
 @pytest.mark.parametrize("scale,nudge", [(1.0, 0), (1.0, 1), (1.0, -1), (1e9, 1), (1e-9, -1)])
 def test_planes_at_the_roundings_of_16_bit_floats(cuda, scale, nudge):
     # axis-aligned quads on, just above and just below values that the nodes store exactly (eight leading
@@ -343,7 +414,8 @@ def _overlaid(kind):
         b.add(f"t{k}", t[::-1] if k else t, n, m[k])
     b.add_quad_light("l", (0.0, 0.0, 2.5), (0.5, 0.0, 0.0), (0.0, 0.5, 0.0), 8.0, m[0])
     if kind == "none":
-        b.add("far", np.float32([[[2e37, 0, 0], [2e37, 1, 0], [2e37, 0, 1]]]), np.float32([[[1, 0, 0]] * 3]), m[0])
+        for x in (-2.9e37, 2.9e37):
+            b.add(f"far{x}", np.float32([[[x, 0, 0], [x, 1, 0], [x, 0, 1]]]), np.float32([[[1, 0, 0]] * 3]), m[0])
     if kind == "spheres":
         b.add_sphere((0.2, 0.1, 0.3), 0.2, m[1])
     return b.build(camera(eye=(0, 0, 3), look=(0, 0, -1), up=(0, 1, 0), height_angle=40.0, aspect=1.0))
