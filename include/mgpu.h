@@ -231,8 +231,8 @@ int mgpu_accel_serialize(const mgpu_accel *accel, int32_t *kind, float *split, i
 int mgpu_accel_destroy(mgpu_accel *accel);
 
 /* Upload accel + scene to the current device and build the 8-wide hierarchy that rays traverse there
- * (device scratch of about 170 bytes per triangle for the duration of the call; a scene whose
- * scratch does not fit is traversed through its kd-tree).  The triangle arrays uploaded are the ones the
+ * (its scratch lies where other arrays of the scene are uploaded afterwards; where scene and hierarchy
+ * do not fit the free memory the scene is traversed through its kd-tree).  The triangle arrays uploaded are the ones the
  * accel captured at build time (tree layout with leaf-ordered triangle records, triangles by id,
  * shading records; page-locked on the first upload); desc supplies the materials and lights and
  * must describe the same triangles.  Returns after the copies complete.                   */

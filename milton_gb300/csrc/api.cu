@@ -88,28 +88,30 @@ static void register_staging(mgpu_accel *a) {
 // Offsets of the arrays in a scene's one device allocation (256-byte aligned each).
 struct SceneLayout {
   size_t off_pairs, off_refs, off_tris, off_shade, off_mats, off_lights, off_uv, off_texrec, off_texels, off_sph,
-      off_wnodes, off_wtris, off_wscratch, off_err, total;
+      off_wnodes, off_wtris, off_err, total;
 };
 // uv_tris: triangles with uploaded uvs (0 or all); ntex textures holding texels texels in all;
-// nsph analytic spheres (2 float4 each, and 3 shading records after the triangles')
+// nsph analytic spheres (2 float4 each, and 3 shading records after the triangles'); wide: with the 8-wide
+// hierarchy, whose build takes its scratch where the kd-tree and the shading records (off_pairs to off_mats)
+// are uploaded afterwards: nothing is allocated for it, and freed, which would wait for the whole device
 static SceneLayout scene_layout(const mgpu_accel *a, int32_t nmat, int32_t nlight, int64_t uv_tris = 0,
-                                int32_t ntex = 0, uint64_t texels = 0, int32_t nsph = 0) {
+                                int32_t ntex = 0, uint64_t texels = 0, int32_t nsph = 0, bool wide = true) {
   SceneLayout L;
-  L.off_pairs = 0;
+  L.off_tris = 0;
+  L.off_pairs = align_up(L.off_tris + std::max<size_t>(a->tris.size(), 1) * sizeof(F4), 256);
   L.off_refs = align_up(L.off_pairs + a->dpairs.size() * sizeof(Pair), 256);
-  L.off_tris = align_up(L.off_refs + std::max<size_t>(a->ltris.size(), 1) * sizeof(F4), 256);
-  L.off_shade = align_up(L.off_tris + std::max<size_t>(a->tris.size(), 1) * sizeof(F4), 256);
+  L.off_shade = align_up(L.off_refs + std::max<size_t>(a->ltris.size(), 1) * sizeof(F4), 256);
   L.off_mats = align_up(L.off_shade + std::max<size_t>(a->shade.size() + 3 * (size_t)std::max(nsph, 0), 1) *
                                           sizeof(float4), 256);
+  if (wide) L.off_mats = std::max(L.off_mats, align_up(L.off_pairs + wide_scratch(a->ntri), 256));
   L.off_lights = align_up(L.off_mats + (size_t)std::max(nmat, 0) * 16 * sizeof(float), 256);
   L.off_uv = align_up(L.off_lights + std::max<size_t>((size_t)std::max(nlight, 0), 1) * 32 * sizeof(float), 256);
   L.off_texrec = align_up(L.off_uv + (size_t)std::max<int64_t>(uv_tris, 0) * 3 * sizeof(float2), 256);
   L.off_texels = align_up(L.off_texrec + (size_t)std::max(ntex, 0) * 2 * sizeof(float4), 256);
   L.off_sph = align_up(L.off_texels + (size_t)texels * sizeof(float4), 256);
   L.off_wnodes = align_up(L.off_sph + (size_t)std::max(nsph, 0) * 2 * sizeof(float4), 256);
-  L.off_wtris = align_up(L.off_wnodes + (size_t)wide_node_cap(a->ntri) * kWideWords * sizeof(uint32_t), 256);
-  L.off_wscratch = align_up(L.off_wtris + (size_t)a->ntri * 3 * sizeof(F4), 256);
-  L.off_err = align_up(L.off_wscratch + wide_scratch(a->ntri), 256);
+  L.off_wtris = align_up(L.off_wnodes + (wide ? (size_t)wide_node_cap(a->ntri) * kWideWords * sizeof(uint32_t) : 0), 256);
+  L.off_err = align_up(L.off_wtris + (wide ? (size_t)a->ntri * 3 * sizeof(F4) : 0), 256);
   L.total = L.off_err + 256;
   return L;
 }
@@ -529,16 +531,19 @@ int mgpu_scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void
   const std::vector<Pair> &dpairs = accel->dpairs;
   const std::vector<F4> &ltris = accel->ltris, &tris = accel->tris;
   const std::vector<float4> &shade = accel->shade;
-  const SceneLayout L = scene_layout(accel, desc->nmat, desc->nlight, tp.uv ? T : 0, desc->ntex, tp.texels,
-                                     desc->nsphere);
-  const size_t off_pairs = L.off_pairs, off_refs = L.off_refs, off_tris = L.off_tris, off_shade = L.off_shade,
-               off_mats = L.off_mats, off_lights = L.off_lights, off_err = L.off_err, total = L.total;
-  const size_t sz_pairs = dpairs.size() * sizeof(Pair), sz_mats = (size_t)desc->nmat * 16 * sizeof(float);
+  SceneLayout L = scene_layout(accel, desc->nmat, desc->nlight, tp.uv ? T : 0, desc->ntex, tp.texels, desc->nsphere);
 
   mgpu_scene *s = new (std::nothrow) mgpu_scene();
   if (!s) return fail(MGPU_E_NOMEM, "mgpu_scene_create: out of host memory");
   cudaGetDevice(&s->device);
-  cudaError_t e = cudaMalloc(&s->d_block, total);
+  bool wide = true;
+  cudaError_t e = cudaMalloc(&s->d_block, L.total);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();  // no room for the hierarchy: the kd-tree alone
+    wide = false;
+    L = scene_layout(accel, desc->nmat, desc->nlight, tp.uv ? T : 0, desc->ntex, tp.texels, desc->nsphere, false);
+    e = cudaMalloc(&s->d_block, L.total);
+  }
   if (e != cudaSuccess) {
     delete s;
     return cuda_fail(e, "mgpu_scene_create: cudaMalloc");
@@ -549,19 +554,46 @@ int mgpu_scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void
     if (n == 0) return cudaSuccess;
     return cudaMemcpyAsync(base + off, src, n, cudaMemcpyHostToDevice, st);
   };
-  e = up(off_pairs, dpairs.data(), sz_pairs);
-  if (e == cudaSuccess) e = up(off_refs, ltris.data(), ltris.size() * sizeof(F4));
-  if (e == cudaSuccess) e = up(off_tris, tris.data(), tris.size() * sizeof(F4));
-  if (e == cudaSuccess) e = up(off_shade, shade.data(), shade.size() * sizeof(float4));
-  if (e == cudaSuccess) e = up(off_mats, desc->materials, sz_mats);
-  if (e == cudaSuccess && desc->nlight > 0) e = up(off_lights, lrec.data(), lrec.size() * sizeof(float));
+  s->view.tris = (const F4 *)(base + L.off_tris);
+  s->view.ntri = T;
+  s->view.wextent = 0.0f;
+  for (int k = 0; k < 3; ++k) {
+    s->view.bmin[k] = (float)tr.bmin[k];
+    s->view.bmax[k] = (float)tr.bmax[k];
+    const float c = 0.5f * s->view.bmin[k] + 0.5f * s->view.bmax[k];
+    s->view.wcentre[k] = std::isfinite(c) ? c : 0.0f;
+    // (a scene of points only has no bounds)
+    const float lo = std::min(s->view.bmin[k], (float)tr.tmin[k]), hi = std::max(s->view.bmax[k], (float)tr.tmax[k]);
+    s->view.wextent = std::max(s->view.wextent, std::max(hi - s->view.wcentre[k], s->view.wcentre[k] - lo));
+  }
+  e = up(L.off_tris, tris.data(), tris.size() * sizeof(F4));
+  if (e == cudaSuccess && wide) {
+    if (int rc = wide_build(s->view.tris, T, s->view, base + L.off_wnodes, (F4 *)(base + L.off_wtris), base + L.off_pairs, st,
+                            &s->wide_nodes, &wide)) {
+      cudaFree(s->d_block);
+      delete s;
+      return rc;
+    }
+  }
+  if (wide) {
+    s->view.wnodes = (const uint32_t *)(base + L.off_wnodes);
+    s->view.wtris = (const F4 *)(base + L.off_wtris);
+  } else {
+    s->view.wextent = INFINITY;
+    s->wide_nodes = 0;
+  }
+  if (e == cudaSuccess) e = up(L.off_pairs, dpairs.data(), dpairs.size() * sizeof(Pair));
+  if (e == cudaSuccess) e = up(L.off_refs, ltris.data(), ltris.size() * sizeof(F4));
+  if (e == cudaSuccess) e = up(L.off_shade, shade.data(), shade.size() * sizeof(float4));
+  if (e == cudaSuccess) e = up(L.off_mats, desc->materials, (size_t)desc->nmat * 16 * sizeof(float));
+  if (e == cudaSuccess && desc->nlight > 0) e = up(L.off_lights, lrec.data(), lrec.size() * sizeof(float));
   if (e == cudaSuccess && tp.uv) e = up(L.off_uv, desc->tri_uv, (size_t)T * 6 * sizeof(float));
   if (e == cudaSuccess && desc->nsphere > 0) {
     e = up(L.off_sph, sph.data(), sph.size() * sizeof(float4));
     if (e == cudaSuccess)
-      e = up(off_shade + shade.size() * sizeof(float4), sph_shade.data(), sph_shade.size() * sizeof(float4));
+      e = up(L.off_shade + shade.size() * sizeof(float4), sph_shade.data(), sph_shade.size() * sizeof(float4));
   }
-  if (e == cudaSuccess) e = cudaMemsetAsync(base + off_err, 0, 256, st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(base + L.off_err, 0, 256, st);
   // materials and lights are the caller's pageable arrays: wait for the copies
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) {
@@ -586,48 +618,24 @@ int mgpu_scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void
   if (tp.uv) s->d_uv = (float2 *)(base + L.off_uv);
   s->bg_tex = desc->background_tex;
   for (int k = 0; k < 3; ++k) s->bg_le[k] = desc->background_le[k];
-  s->view.pairs = (const Pair *)(base + off_pairs);
-  s->view.ltris = (const F4 *)(base + off_refs);
-  s->view.tris = (const F4 *)(base + off_tris);
-  for (int k = 0; k < 3; ++k) { s->view.bmin[k] = (float)tr.bmin[k]; s->view.bmax[k] = (float)tr.bmax[k]; }
-  s->view.ntri = T;
+  s->view.pairs = (const Pair *)(base + L.off_pairs);
+  s->view.ltris = (const F4 *)(base + L.off_refs);
   s->view.npairs = tr.pairs.size();
   s->view.nrefs = ltris.size() / 3;
   s->view.spheres = desc->nsphere > 0 ? (const F4 *)(base + L.off_sph) : nullptr;
   s->view.nsphere = desc->nsphere;
-  s->d_shade = (float4 *)(base + off_shade);
-  s->d_mats = (float *)(base + off_mats);
-  s->d_lights = (float *)(base + off_lights);
+  s->d_shade = (float4 *)(base + L.off_shade);
+  s->d_mats = (float *)(base + L.off_mats);
+  s->d_lights = (float *)(base + L.off_lights);
   s->nmat = desc->nmat;
   for (int i = 1; i < desc->nmat; ++i) s->mixed = s->mixed || desc->materials[16 * i] != desc->materials[0];
   s->nlight = desc->nlight;
-  bool wide = false;
-  s->view.wextent = 0.0f;
-  for (int k = 0; k < 3; ++k) {
-    const float c = 0.5f * s->view.bmin[k] + 0.5f * s->view.bmax[k];
-    s->view.wcentre[k] = std::isfinite(c) ? c : 0.0f;
-    // (a scene of points only has no bounds)
-    const float lo = std::min(s->view.bmin[k], (float)tr.tmin[k]), hi = std::max(s->view.bmax[k], (float)tr.tmax[k]);
-    s->view.wextent = std::max(s->view.wextent, std::max(hi - s->view.wcentre[k], s->view.wcentre[k] - lo));
-  }
-  if (int rc = wide_build(s->view.tris, T, s->view, base + L.off_wnodes, (F4 *)(base + L.off_wtris), base + L.off_wscratch, st,
-                          &s->wide_nodes, &wide)) {
-    cudaFree(s->d_block);
-    delete s;
-    return rc;
-  }
-  if (!wide) {
-    s->view.wextent = INFINITY;
-    s->wide_nodes = 0;
-  }
-  s->view.wnodes = wide ? (const uint32_t *)(base + L.off_wnodes) : nullptr;
-  s->view.wtris = wide ? (const F4 *)(base + L.off_wtris) : nullptr;
   // staging the top of the tree in shared memory costs more occupancy than it saves on GB300
   // (the L1 keeps those pairs anyway); mgpu_scene_set_top_pairs turns it on
   s->top_pairs = 0;
   s->top_pairs_max = tr.top_pairs;
-  s->d_err = (uint32_t *)(base + off_err);
-  s->bytes = total;
+  s->d_err = (uint32_t *)(base + L.off_err);
+  s->bytes = L.total;
   *out = s;
   return MGPU_OK;
 }

@@ -961,11 +961,10 @@ size_t place_scratch(Build &B, int64_t n, char *base) {
 }
 }  // namespace
 
-// Scratch that a scene keeps beside its arrays, so that creating a small scene allocates once; a larger
-// one's is allocated for the duration of the build.
+// Bytes of scratch that the build of n triangles takes.
 size_t wide_scratch(int64_t n) {
   Build B;
-  return n > 0 && n <= kSmall ? place_scratch(B, n, nullptr) : 0;
+  return n > 0 ? place_scratch(B, n, nullptr) : 0;
 }
 
 int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F4 *wtris, void *scratch, cudaStream_t st,
@@ -986,18 +985,8 @@ int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F
   }
   B.cap_nodes = (uint32_t)wide_node_cap(n);
   const int radix_blocks = (int)((n + kRadixTile - 1) / kRadixTile);
-  const size_t bytes = place_scratch(B, n, nullptr);
-  char *base = (char *)scratch;
   cudaError_t e = cudaSuccess;
-  if (n > kSmall) {
-    e = cudaMalloc((void **)&base, bytes);
-    if (e == cudaErrorMemoryAllocation) {
-      cudaGetLastError();  // no room for the scratch: the scene keeps the kd-tree traversal
-      return MGPU_OK;
-    }
-    if (e != cudaSuccess) return cuda_fail(e, "wide hierarchy build: scratch");
-  }
-  place_scratch(B, n, base);
+  place_scratch(B, n, (char *)scratch);
   const int sms = device_sm_count();
   uint64_t launches = 0;
   auto grid = [&](int64_t items, int block) {
@@ -1076,7 +1065,6 @@ int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F
     }
   }
   g_launches.fetch_add(launches);
-  if (n > kSmall) cudaFree(base);
   if (e != cudaSuccess) return cuda_fail(e, "wide hierarchy build");
   return MGPU_OK;
 }

@@ -45,9 +45,9 @@ struct TexPlan {
 int tex_plan(const mgpu_scene_desc *desc, TexPlan &plan);
 int tex_upload(const mgpu_scene_desc *desc, const TexPlan &plan, float4 *d_texrec, float4 *d_texels, cudaStream_t st);
 
-// 8-wide hierarchy over the uploaded triangles (bvh.cu): node capacity of n triangles, and the build
-// into wnodes / wtris (3 records of 16 bytes per triangle) with wide_scratch(n) bytes of scratch.  ok = false: none was built (no
-// scratch memory, or a hierarchy beyond the traversal's limits) and the kd-tree is used.
+// 8-wide hierarchy over the uploaded triangles (bvh.cu): node capacity of n triangles, and the build into wnodes /
+// wtris (3 records of 16 bytes per triangle) with wide_scratch(n) bytes of scratch.  ok = false: none was
+// built (a hierarchy beyond the traversal's limits) and the kd-tree is used.
 int64_t wide_node_cap(int64_t ntri);
 size_t wide_scratch(int64_t n);
 int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F4 *wtris, void *scratch, cudaStream_t st,
