@@ -266,9 +266,20 @@ def test_triangles_that_the_root_box_leaves_out(cuda, kind):
 
 
 def test_which_scenes_have_the_hierarchy(cuda):
-    for kind in KINDS:
-        s = _scene(kind)
-        assert pt.DeviceScene(s, pt.Accel(s)).hierarchy_nodes > 0, kind
+    for kind in KINDS + ["pile", "strip", "needles"]:
+        if kind == "pile":       # one triangle many times: every area in the hierarchy is the same
+            s = _soup(np.repeat(_random_tris(1, 3), 3000, 0))
+        elif kind == "strip":    # copies of one in a row, a power of two apart
+            t = np.float32([[0, 0, 0], [1, 0, 0], [0, 1, 0]])
+            s = _soup(t + np.float32([1, 0, 0]) * 2.0 ** np.arange(-12, 12, 0.005)[:, None, None])
+        elif kind == "needles":  # thin and long, side by side
+            t = _random_tris(3000, 4, size=1e-4)
+            t[:, 2, 0] += 3.0
+            s = _soup(t)
+        else:
+            s = _scene(kind)
+        n = pt.DeviceScene(s, pt.Accel(s)).hierarchy_nodes
+        assert 0 < n <= 5 * s.ntri / 16 + 8, (kind, s.ntri, n)
     s = _overlaid("none")  # coordinates beyond what its nodes hold
     assert pt.DeviceScene(s, pt.Accel(s)).hierarchy_nodes == 0
 
