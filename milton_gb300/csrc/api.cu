@@ -125,11 +125,13 @@ struct FilmRef {
   const float4 *sum;
   const float4 *c;
   int64_t npix;
+  int64_t first = 0;  // its first block among those of all films
 };
 constexpr int kErrBlocks = 64, kErrThreads = 256;
 
 // Blocks that reduce one film: one per 2,048 pixels within [64, 1024] (by the film alone, so that its value does
-// not depend on the films beside it).  64 for every film left the GPU idle on large ones (483,003
+// not depend on the films beside it; each film has its own number, or one large film would make a
+// thousand idle blocks and 16 KB of partial sums of every small one).  64 for every film left the GPU idle on large ones (483,003
 // pixels: 212 -> 87 us a call, with two divisions a pixel instead of five).
 constexpr int kErrMaxBlocks = 1024;
 __host__ __device__ inline int err_blocks(int64_t npix) {
@@ -154,12 +156,16 @@ __device__ __forceinline__ void err_reduce(double &a, double &c) {
   c = sc[0];
 }
 
-__global__ void __launch_bounds__(kErrThreads) k_film_error_partial(const FilmRef *films, double2 *partial) {
-  const FilmRef f = films[blockIdx.y];
+__global__ void __launch_bounds__(kErrThreads) k_film_error_partial(const FilmRef *films, int n, double2 *partial) {
+  int at = 0;  // the film of this block: the last that begins no later
+  for (int hi = n - 1; at < hi;) {
+    const int mid = (at + hi + 1) >> 1;
+    if (films[mid].first <= (int64_t)blockIdx.x) at = mid; else hi = mid - 1;
+  }
+  const FilmRef f = films[at];
   const int nb = err_blocks(f.npix);
-  if ((int)blockIdx.x >= nb) return;
   double acc = 0.0, cnt = 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * kErrThreads + threadIdx.x; i < f.npix; i += (int64_t)nb * kErrThreads) {
+  for (int64_t i = ((int64_t)blockIdx.x - f.first) * kErrThreads + threadIdx.x; i < f.npix; i += (int64_t)nb * kErrThreads) {
     const float4 S = f.sum[i], C = f.c[i];
     const double n = S.w;
     if (n > 1.0) {
@@ -172,15 +178,16 @@ __global__ void __launch_bounds__(kErrThreads) k_film_error_partial(const FilmRe
     }
   }
   err_reduce(acc, cnt);
-  if (threadIdx.x == 0) partial[(int64_t)blockIdx.y * gridDim.x + blockIdx.x] = make_double2(acc, cnt);
+  if (threadIdx.x == 0) partial[blockIdx.x] = make_double2(acc, cnt);
 }
 
 __global__ void __launch_bounds__(kErrThreads) k_film_error_final(const FilmRef *films, const double2 *partial,
-                                                                  int stride, double *out) {
-  const int nb = err_blocks(films[blockIdx.x].npix);
+                                                                  double *out) {
+  const FilmRef f = films[blockIdx.x];
+  const int nb = err_blocks(f.npix);
   double a = 0.0, c = 0.0;
   for (int b = threadIdx.x; b < nb; b += kErrThreads) {
-    const double2 p = partial[(int64_t)blockIdx.x * stride + b];
+    const double2 p = partial[f.first + b];
     a += p.x;
     c += p.y;
   }
@@ -841,7 +848,7 @@ int mgpu_film_read(mgpu_film *f, double *out_mean, void *stream) {
 int mgpu_film_tonemap(mgpu_film *f, uint8_t *out_rgba, void *stream) {
   if (!f || !out_rgba) return fail(MGPU_E_INVALID, "mgpu_film_tonemap: null argument");
   const int64_t npix = (int64_t)f->width * f->height;
-  ToneSrc ref{FilmRef{f->d_sum, f->d_c, npix}, f->d_fx};
+  ToneSrc ref{FilmRef{f->d_sum, f->d_c, npix, 0}, f->d_fx};
   const size_t bytes = (size_t)npix * sizeof(uchar4), b_part = align_up(kErrBlocks * sizeof(double2), 256);
   const bool direct = device_writes(out_rgba, bytes, sizeof(uchar4));
   char *d = nullptr;
@@ -868,19 +875,18 @@ int mgpu_film_error(mgpu_film *const *films, int32_t n, double *out_rmse, void *
   MGPU_CUDA(t_read.host_buffer(b_refs + (size_t)n * sizeof(double), (void **)&h));
   FilmRef *refs = (FilmRef *)h;
   double *est = (double *)(h + b_refs);
-  int blocks = kErrBlocks;
+  int64_t blocks = 0;
   for (int32_t i = 0; i < n; ++i) {
     if (!films[i]) return fail(MGPU_E_INVALID, "mgpu_film_error: null film");
-    refs[i].sum = films[i]->d_sum;
-    refs[i].c = films[i]->d_c;
-    refs[i].npix = (int64_t)films[i]->width * films[i]->height;
-    blocks = std::max(blocks, err_blocks(refs[i].npix));
+    const int64_t npix = (int64_t)films[i]->width * films[i]->height;
+    refs[i] = FilmRef{films[i]->d_sum, films[i]->d_c, npix, blocks};
+    blocks += err_blocks(npix);
   }
   double2 *part = nullptr;
-  MGPU_CUDA(t_read.device_buffer((size_t)n * blocks * sizeof(double2), (void **)&part));
+  MGPU_CUDA(t_read.device_buffer((size_t)blocks * sizeof(double2), (void **)&part));
   cudaStream_t st = as_stream(stream);
-  k_film_error_partial<<<dim3(blocks, n), kErrThreads, 0, st>>>(refs, part);
-  k_film_error_final<<<n, kErrThreads, 0, st>>>(refs, part, blocks, est);
+  k_film_error_partial<<<(unsigned)blocks, kErrThreads, 0, st>>>(refs, n, part);
+  k_film_error_final<<<n, kErrThreads, 0, st>>>(refs, part, est);
   g_launches.fetch_add(2);
   MGPU_CUDA(cudaGetLastError());
   MGPU_CUDA(cudaStreamSynchronize(st));

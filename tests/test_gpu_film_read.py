@@ -153,3 +153,22 @@ def test_a_copy_from_a_result_outlives_it(cuda):
         again = read(films[1], stream=cuda.cuda.default_stream())
         cuda.cuda.synchronize()
         assert np.array_equal(got.cpu().numpy(), want[0]) and np.array_equal(again, want[1])
+
+
+def test_error_estimates_of_films_of_uneven_size(cuda):
+    # each film by itself and all in one call give the same bits, and the scratch follows the sum of the sizes
+    s = scenegen.plain(0)
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    films = []
+    for k, (w, h) in enumerate([(1, 1), (37, 23), (1600, 1400), (256, 513), (2, 3)] + [(8, 8)] * 60):
+        films.append(pt.Film(w, h))
+        pt.render(ds, pt.RenderSettings(w, h, 4, max_depth=2, rr_start_depth=3, seed=k), films[-1])
+    alone = [pt.film_error([f])[0] for f in films]
+    assert np.array_equal(pt.film_error(films), alone)
+    assert np.array_equal(pt.film_error(films[::-1]), alone[::-1])
+    many = [films[2]] + [films[5]] * 20_000
+    free = cuda.cuda.mem_get_info()[0]
+    pt.film_error(many)
+    assert free - cuda.cuda.mem_get_info()[0] < 64 << 20  # 21 MB, not a row of the largest film's blocks for each
+    got = pt.film_error(many)
+    assert got[0] == alone[2] and (got[1:] == alone[5]).all()
