@@ -821,6 +821,15 @@ int mgpu_film_read(mgpu_film *f, double *out_mean, void *stream) {
   if (!f || !out_mean) return fail(MGPU_E_INVALID, "mgpu_film_read: null argument");
   const int64_t n = (int64_t)f->width * f->height;
   cudaStream_t st = as_stream(stream);
+  int cur = 0;
+  MGPU_CUDA(cudaGetDevice(&cur));
+  if (cur != f->device) {  // the kernel runs where the film is, after what the caller's stream holds
+    MGPU_CUDA(cudaStreamSynchronize(st));
+    MGPU_CUDA(cudaSetDevice(f->device));
+    const int rc = mgpu_film_read(f, out_mean, nullptr);
+    cudaSetDevice(cur);
+    return rc;
+  }
   auto launch = [&](int64_t first, int64_t count, double *dst) {
     const unsigned grid = (unsigned)std::min<int64_t>((count + 255) / 256, (int64_t)device_sm_count() * 8);
     k_film_mean<<<grid, 256, 0, st>>>(f->d_sum, f->d_c, f->d_fx, first, count, dst);

@@ -172,3 +172,24 @@ def test_error_estimates_of_films_of_uneven_size(cuda):
     assert free - cuda.cuda.mem_get_info()[0] < 64 << 20  # 21 MB, not a row of the largest film's blocks for each
     got = pt.film_error(many)
     assert got[0] == alone[2] and (got[1:] == alone[5]).all()
+
+
+@pytest.mark.parametrize("w,h", [(2048, 2048), (2048, 2049), (2897, 2897)])
+@pytest.mark.parametrize("kind", ["none", "box"])
+def test_means_of_more_pixels_than_the_scratch_holds(cuda, w, h, kind):
+    # one piece exactly, one row more, two pieces and a remainder, against the one store of a page-locked array
+    s = scenegen.plain(0)
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    f = pt.Film(w, h)
+    if kind != "none":
+        f.set_filter(kind, 1.0)
+    pt.render(ds, pt.RenderSettings(w, h, 1, max_depth=1, rr_start_depth=3, seed=3), f)
+    lib, p = N.load(), C.c_void_p()
+    N.check(lib.mgpu_host_alloc(w * h * 24, C.byref(p)))
+    try:
+        N.check(lib.mgpu_film_read(f.handle, p, None))
+        direct = np.ctypeslib.as_array((C.c_double * (w * h * 3)).from_address(p.value)).reshape(h, w, 3)
+        assert direct.any() and np.array_equal(f.mean(), direct)
+        del direct
+    finally:
+        N.check(lib.mgpu_host_free(p))
