@@ -131,9 +131,12 @@ __device__ __forceinline__ Box tri_box(const Build &B, int64_t t) {
   r.lo[0] = fminf(a.x, fminf(b.x, c.x)); r.hi[0] = fmaxf(a.x, fmaxf(b.x, c.x));
   r.lo[1] = fminf(a.y, fminf(b.y, c.y)); r.hi[1] = fmaxf(a.y, fmaxf(b.y, c.y));
   r.lo[2] = fminf(a.z, fminf(b.z, c.z)); r.hi[2] = fmaxf(a.z, fmaxf(b.z, c.z));
-  // nothing hits a point, and the kd-tree's bounds leave it out: it must not widen the hierarchy's
+  // nothing hits a point, and the kd-tree's bounds leave it out: it must not widen the hierarchy's.  (Bounds of
+  // nothing, where the kd-tree leaves out every triangle, would make it infinite and its areas NaN, which
+  // no order of neighbours survives.)
   if (r.lo[0] == r.hi[0] && r.lo[1] == r.hi[1] && r.lo[2] == r.hi[2])
-    for (int k = 0; k < 3; ++k) r.lo[k] = r.hi[k] = fminf(fmaxf(r.lo[k], B.bmin[k]), B.bmax[k]);
+    for (int k = 0; k < 3; ++k)
+      r.lo[k] = r.hi[k] = B.bmin[k] <= B.bmax[k] ? fminf(fmaxf(r.lo[k], B.bmin[k]), B.bmax[k]) : 0.0f;
   return r;
 }
 
@@ -580,7 +583,7 @@ __device__ void cluster_tail(const Build &B, TailShared &S, int count, uint32_t 
     if (f1 != 2) { S.id[k] = ni[1]; S.sb[k] = nb[1]; }
     if (threadIdx.x == 0) {
       S.next = next + tm;
-      S.force = tm < (uint32_t)count / 10u ? 1 : 0;
+      S.force = tm == 0u || tm < (uint32_t)count / 10u ? 1 : 0;  // the next round merges, whatever the areas
     }
     count = (int)tk;
     __syncthreads();

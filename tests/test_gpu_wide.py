@@ -265,6 +265,22 @@ def test_triangles_that_the_root_box_leaves_out(cuda, kind):
     assert all(np.array_equal(films[0], f) for f in films[1:])
 
 
+@pytest.mark.parametrize("points", [1, 2, 3, 9, 40, 3000])
+@pytest.mark.parametrize("floors", [0, 1, 3])
+def test_scenes_of_which_the_root_box_leaves_out_everything(cuda, points, floors):
+    # points, and flat triangles from -1 to 1: the root box is empty, and no bounds of it take part in the build
+    rng = np.random.default_rng(points)
+    t = [np.repeat(rng.uniform(-1, 1, (points, 1, 3)), 3, 1)]
+    for y in np.linspace(-0.5, 0.5, floors):
+        t.insert(rng.integers(len(t) + 1), scenegen.quad_tris((-1, y, 1), (1, y, 1), (1, y, -1), (-1, y, -1)))
+    s = _soup(np.concatenate(t))
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    rays = sphere_rays(np.full(3, -1.3), np.full(3, 1.3), 5000, points).astype(np.float32)
+    kd, _ = gpu_trace(cuda, ds, rays, counts=True)
+    assert np.array_equal(kd.view(np.uint32), gpu_trace(cuda, ds, rays)[0].view(np.uint32))
+    assert np.array_equal(gpu_any(cuda, ds, rays) != 0, kd[:, 1].view(np.int32) >= 0)
+
+
 def test_which_scenes_have_the_hierarchy(cuda):
     for kind in KINDS + ["pile", "strip", "needles"]:
         if kind == "pile":       # one triangle many times: every area in the hierarchy is the same
