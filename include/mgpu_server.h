@@ -13,8 +13,9 @@
  *      otherwise it is admitted while an active slot is free and its film -- plus its scene,
  *      if that is not resident -- fits the device-memory budget.  Idle resident scenes (no
  *      active job) are evicted least recently used first to make room; a job that still does
- *      not fit stops admission for this tick.  Trees and films stay on the device between
- *      ticks.
+ *      not fit stops admission for this tick.  A scene that the whole budget holds beside the
+ *      job's film only without its 8-wide hierarchy is uploaded without it.  Trees and films
+ *      stay on the device between ticks.
  *   2. Rendering: active jobs get sample passes up to the tick's path budget -- under the fair
  *      policy first one sample each, least recently served first, then the rest of the budget
  *      oldest job first; under the oldest-first policy only the latter; under the rotating

@@ -474,6 +474,14 @@ int mgpu_accel_destroy(mgpu_accel *a) {
 }
 
 int mgpu_scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void *stream, mgpu_scene **out) {
+  return scene_create(desc, accel, stream, UINT64_MAX, out);
+}
+
+}  // extern "C"
+
+namespace mgpu {
+
+int scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void *stream, uint64_t limit, mgpu_scene **out) {
   if (!desc || !accel || !out) return fail(MGPU_E_INVALID, "mgpu_scene_create: null argument");
   if (desc->ntri != accel->ntri) return fail(MGPU_E_INVALID, "mgpu_scene_create: accel built for another triangle count");
   if (desc->ntri > 0 && (!desc->tri_v || !desc->tri_mat)) return fail(MGPU_E_INVALID, "mgpu_scene_create: missing arrays");
@@ -548,8 +556,8 @@ int mgpu_scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void
   mgpu_scene *s = new (std::nothrow) mgpu_scene();
   if (!s) return fail(MGPU_E_NOMEM, "mgpu_scene_create: out of host memory");
   cudaGetDevice(&s->device);
-  bool wide = true;
-  cudaError_t e = cudaMalloc(&s->d_block, L.total);
+  bool wide = L.total <= limit;
+  cudaError_t e = wide ? cudaMalloc(&s->d_block, L.total) : cudaErrorMemoryAllocation;
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();  // no room for the hierarchy: the kd-tree alone
     wide = false;
@@ -652,6 +660,18 @@ int mgpu_scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void
   return MGPU_OK;
 }
 
+int scene_device_bytes(const mgpu_scene_desc *desc, const mgpu_accel *a, bool wide, uint64_t *out) {
+  TexPlan tp;
+  if (int rc = tex_plan(desc, tp)) return rc;
+  *out = scene_layout(a, desc->nmat, desc->nlight, tp.uv ? desc->ntri : 0, desc->ntex, tp.texels,
+                      std::max(desc->nsphere, 0), wide).total;
+  return MGPU_OK;
+}
+
+}  // namespace mgpu
+
+extern "C" {
+
 int mgpu_scene_destroy(mgpu_scene *s) {
   if (!s) return MGPU_OK;
   int cur = 0;
@@ -693,11 +713,7 @@ int mgpu_accel_device_bytes(const mgpu_accel *a, int32_t nmat, int32_t nlight, u
 int mgpu_scene_device_bytes(const mgpu_scene_desc *desc, const mgpu_accel *a, uint64_t *out) {
   if (!desc || !a || !out || desc->nmat < 0 || desc->nlight < 0)
     return fail(MGPU_E_INVALID, "mgpu_scene_device_bytes: bad argument");
-  TexPlan tp;
-  if (int rc = tex_plan(desc, tp)) return rc;
-  *out = scene_layout(a, desc->nmat, desc->nlight, tp.uv ? desc->ntri : 0, desc->ntex, tp.texels,
-                      std::max(desc->nsphere, 0)).total;
-  return MGPU_OK;
+  return scene_device_bytes(desc, a, true, out);
 }
 
 int mgpu_scene_read_texels(const mgpu_scene *s, int32_t tex, float *out, void *stream) {

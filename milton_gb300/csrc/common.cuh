@@ -53,6 +53,11 @@ size_t wide_scratch(int64_t n);
 int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F4 *wtris, void *scratch, cudaStream_t st,
                uint32_t *nodes_out, bool *ok);
 
+// mgpu_scene_create, without the hierarchy if the scene would exceed `limit` device bytes with it; and the device
+// bytes of a scene with it or without (api.cu)
+int scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void *stream, uint64_t limit, mgpu_scene **out);
+int scene_device_bytes(const mgpu_scene_desc *desc, const mgpu_accel *a, bool wide, uint64_t *out);
+
 }  // namespace mgpu
 
 struct mgpu_accel {

@@ -24,6 +24,8 @@
 
 namespace mgpu {
 int fail(int code, const std::string &msg);
+int scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void *stream, uint64_t limit, mgpu_scene **out);
+int scene_device_bytes(const mgpu_scene_desc *desc, const mgpu_accel *a, bool wide, uint64_t *out);
 }
 
 namespace {
@@ -46,9 +48,10 @@ struct SrvScene {
   int state = kIdle;
   std::string error;
   mgpu_accel *accel = nullptr;
-  uint64_t dev_bytes = 0;
+  uint64_t dev_bytes = 0, lean_bytes = 0;  // with the 8-wide hierarchy, and without
   // stepping thread only
   mgpu_scene *dev = nullptr;
+  uint64_t held = 0;  // device bytes of dev
   int active = 0;
   uint64_t last_use = 0;
 
@@ -141,14 +144,16 @@ void build_worker(mgpu_server *s) {
     }
     const mgpu_scene_desc d = sc->desc();
     mgpu_accel *acc = nullptr;
-    uint64_t bytes = 0;
+    uint64_t bytes = 0, lean = 0;
     int rc = mgpu_accel_build(&d, &s->p.kd, &acc);
-    if (rc == MGPU_OK) rc = mgpu_scene_device_bytes(&d, acc, &bytes);
+    if (rc == MGPU_OK) rc = mgpu::scene_device_bytes(&d, acc, true, &bytes);
+    if (rc == MGPU_OK) rc = mgpu::scene_device_bytes(&d, acc, false, &lean);
     const std::string err = rc == MGPU_OK ? std::string() : std::string(mgpu_last_error());
     std::lock_guard<std::mutex> lk(s->mu);
     if (rc == MGPU_OK) {
       sc->accel = acc;
       sc->dev_bytes = bytes;
+      sc->lean_bytes = lean;
       sc->state = kBuilt;
       ++s->builds;
     } else {
@@ -181,6 +186,14 @@ void account(mgpu_server *s) {
   s->peak = std::max(s->peak, s->resident);
 }
 
+void evict(mgpu_server *s, SrvScene *sc) {
+  mgpu_scene_destroy(sc->dev);
+  sc->dev = nullptr;
+  s->scene_bytes -= sc->held;
+  ++s->evictions;
+  account(s);
+}
+
 // frees idle resident scenes, least recently used first, until `need` more bytes fit
 void evict_idle(mgpu_server *s, uint64_t need, int32_t keep) {
   while (s->resident + need > s->p.hbm_budget) {
@@ -191,11 +204,7 @@ void evict_idle(mgpu_server *s, uint64_t need, int32_t keep) {
       if (!victim || sc->last_use < victim->last_use) victim = sc;
     }
     if (!victim) return;
-    mgpu_scene_destroy(victim->dev);
-    victim->dev = nullptr;
-    s->scene_bytes -= victim->dev_bytes;
-    ++s->evictions;
-    account(s);
+    evict(s, victim);
   }
 }
 
@@ -240,7 +249,12 @@ int admit(mgpu_server *s, void *stream, double now) {
       fail_job(s, j, "kd-tree build failed: " + sc->error, now);
       continue;
     }
-    const uint64_t need = j->film_bytes() + (sc->dev ? 0 : sc->dev_bytes);
+    // a budget that holds the film and the scene only without the 8-wide hierarchy takes the scene without (it
+    // renders the same image on the kd-tree); one that is resident with it, for smaller films, is made anew
+    const uint64_t budget = s->p.hbm_budget, film = j->film_bytes();
+    const uint64_t bytes = sc->dev_bytes <= budget && film <= budget - sc->dev_bytes ? sc->dev_bytes : sc->lean_bytes;
+    if (sc->dev && sc->active == 0 && sc->held > bytes && film + bytes <= budget) evict(s, sc);
+    const uint64_t need = film + (sc->dev ? 0 : bytes);
     if (need > s->p.hbm_budget) {
       s->queue.erase(s->queue.begin() + qi);
       fail_job(s, j, "film and scene exceed the whole memory budget", now);
@@ -250,14 +264,15 @@ int admit(mgpu_server *s, void *stream, double now) {
     if (s->resident + need > s->p.hbm_budget) break;  // wait for running jobs to free memory
     if (!sc->dev) {
       const mgpu_scene_desc d = sc->desc();
-      int rc = mgpu_scene_create(&d, sc->accel, stream, &sc->dev);
+      int rc = mgpu::scene_create(&d, sc->accel, stream, bytes, &sc->dev);
       if (rc == MGPU_E_NOMEM) break;
       if (rc != MGPU_OK) {
         s->queue.erase(s->queue.begin() + qi);
         fail_job(s, j, std::string("scene upload failed: ") + mgpu_last_error(), now);
         continue;
       }
-      s->scene_bytes += sc->dev_bytes;
+      sc->held = bytes;
+      s->scene_bytes += bytes;
       ++s->uploads;
       account(s);
     }

@@ -163,6 +163,20 @@ def test_admission_respects_the_memory_budget(cuda):
         assert srv.job(j)["state"] == "failed"
 
 
+def test_a_budget_that_holds_a_scene_only_without_its_hierarchy(cuda):
+    # the first job leaves room for the scene with its hierarchy, the second's film does not: both are served
+    scene = scenegen.random_scene(22, 20000)
+    full = pt.DeviceScene(scene, pt.Accel(scene)).nbytes
+    jobs = [(0, 16, 4, 4, 0.0), (0, 96, 4, 4, 0.0), (0, 16, 1, 2, 0.0)]
+    films = [side * side * 32 for _, side, *_ in jobs]
+    solo = [_run([scene], [j], keys=[k])[0][0] for k, j in enumerate(jobs)]
+    for budget in (full + films[1] - 1, full + films[0], full - 1):
+        served, st, peak = _run([scene], jobs, ServerSettings(hbm_budget=budget, tick_paths=20000, max_active=1))
+        assert st["finished"] == len(jobs) and peak <= budget
+        for (ia, a), (ib, b) in zip(solo, served):
+            assert ia["state"] == ib["state"] == "done" and np.array_equal(a, b)
+
+
 def test_film_error_matches_host_model_and_measured_error(cuda):
     s = scenegen.plain(0)
     acc = pt.Accel(s)
