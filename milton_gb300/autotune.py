@@ -2,8 +2,8 @@
 capacity) and queue binning by timing a short calibration render of the actual requests, and caches
 the choice per workload size class.  Results never depend on these knobs (every path draws its
 own counter-based random numbers and each film sums its samples in sample order), only speed does.
-The "persistent", "bin_shadow" and "trav_block" entries select nothing any more (include/mgpu.h); they
-are kept at one value so that a configuration still names them."""
+The "persistent", "bin_shadow" and "trav_block" entries of a configuration select nothing
+(include/mgpu.h); they are neither searched nor set."""
 from __future__ import annotations
 
 import itertools
@@ -13,7 +13,7 @@ from . import pathtracer as pt
 
 WAVES = (1 << 21, 1 << 22, 1 << 23, 1 << 24, 1 << 25, 1 << 26)
 SHAPES = ((0, 1, 1), (0, 1, 0))  # (persistent, bin_shadow, bin_extension)
-BLOCKS = (256,)
+BLOCKS = (256,)  # accepted; there is one traversal block size
 
 _cache: dict = {}
 
@@ -27,7 +27,7 @@ def _size_class(requests) -> tuple:
 def tune(requests, stream=None, calib_samples: int = 4, waves=WAVES, shapes=SHAPES, blocks=BLOCKS) -> dict:
     """requests: list of (DeviceScene, RenderSettings).  Returns {"wave_paths", "persistent",
     "bin_shadow", "bin_extension", "trav_block", "ms"} for the fastest calibration render and
-    applies the kernel-shape knobs process-wide."""
+    sets queue binning process-wide."""
     key = _size_class(requests)
     if key in _cache:
         best = _cache[key]
@@ -40,15 +40,6 @@ def tune(requests, stream=None, calib_samples: int = 4, waves=WAVES, shapes=SHAP
         ms = _time(requests, films, wave, cfg, stream, calib_samples)
         if ms is not None and (best is None or ms < best["ms"]):
             best = {"wave_paths": wave, **cfg, "ms": ms}
-    if best is not None and not best["persistent"]:
-        for blk in blocks:
-            if blk == 256:
-                continue
-            cfg = {k: best[k] for k in ("persistent", "bin_shadow", "bin_extension")}
-            cfg["trav_block"] = blk
-            ms = _time(requests, films, best["wave_paths"], cfg, stream, calib_samples)
-            if ms is not None and ms < best["ms"]:
-                best = {"wave_paths": best["wave_paths"], **cfg, "ms": ms}
     for f in films:
         f.close()
     _cache[key] = best
@@ -81,5 +72,4 @@ def _time(requests, films, wave, cfg, stream, calib_samples):
 
 
 def _apply(cfg: dict) -> None:
-    for k in ("persistent", "bin_shadow", "bin_extension", "trav_block"):
-        pt.tune(k, int(cfg.get(k, 256 if k == "trav_block" else 0)))
+    pt.tune("bin_extension", int(cfg.get("bin_extension", 0)))
