@@ -193,3 +193,21 @@ def test_means_of_more_pixels_than_the_scratch_holds(cuda, w, h, kind):
         del direct
     finally:
         N.check(lib.mgpu_host_free(p))
+
+
+@pytest.mark.parametrize("off", [0, 8, 24])
+@pytest.mark.parametrize("new", [False, True])
+def test_a_result_inside_a_larger_array(cuda, off, new):
+    # the pages of a result are made before the copy: with the bytes beside it in them, new and old ones
+    w, h = 150, 111
+    ds = pt.DeviceScene(scenegen.plain(0), pt.Accel(scenegen.plain(0)))
+    f = pt.Film(w, h)
+    pt.render(ds, pt.RenderSettings(w, h, 1, max_depth=2), f)
+    want, n = f.mean(), h * w * 3
+    lib = pt.N.load()
+    big = np.zeros(n + 4 * 16384) if new else np.full(n + 4 * 16384, 7.0)
+    keep = 0.0 if new else 7.0
+    part = big[16384 + off // 8:][:n]
+    pt.N.check(lib.mgpu_film_read(f.handle, pt.N.ptr(part), None))
+    assert np.array_equal(part.reshape(h, w, 3), want)
+    assert np.all(big[:16384 + off // 8] == keep) and np.all(big[16384 + off // 8 + n:] == keep)
