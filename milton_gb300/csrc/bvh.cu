@@ -118,7 +118,8 @@ __device__ __forceinline__ float unorder_bits(uint32_t u) {
 // Whether a triangle reaches out of the kd-tree's root box.  The root box leaves out triangles whose bounds compare
 // equal under Milton's fuzzy comparison (flat ones from -1 to 1, kdbuild.cpp); rays find such a triangle only
 // where a leaf on their way through the root box lists it, wherever they hit it.  Its records carry
-// kWideOutside, and the kd-tree decides a ray that hits one before anything else.
+// kWideOutside, and the kd-tree decides a ray that hits one before anything else, unless it is certain
+// to find that hit (wide_listed).
 __device__ __forceinline__ bool sticks_out(const Build &B, const Box &b) {
   bool out = false;
   for (int k = 0; k < 3; ++k) out = out || b.lo[k] < B.bmin[k] || b.hi[k] > B.bmax[k];

@@ -265,6 +265,40 @@ def test_triangles_that_the_root_box_leaves_out(cuda, kind):
     assert all(np.array_equal(films[0], f) for f in films[1:])
 
 
+@pytest.mark.parametrize("gap", [0.0, 1e-7, 1e-4, 0.05, -0.1])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+def test_hits_on_triangles_that_the_root_box_leaves_out(cuda, gap, axis):
+    # flat ones from -1 to 1 on both sides, on the root box's faces, beyond them and cutting through it: rays from
+    # inside and outside that leave through the face before them, through another, or miss the box
+    t = (_random_tris(1500, 21, size=0.08) * 0.6).astype(np.float32)
+    box = t.reshape(-1, 3).min(0), t.reshape(-1, 3).max(0)
+    q = []
+    for v in (np.float32(box[0][axis] - gap), np.float32(box[1][axis] + gap)):
+        f = np.asarray(scenegen.quad_tris((-1, v, 1), (1, v, 1), (1, v, -1), (-1, v, -1)), np.float32)
+        q.append(np.roll(f, axis - 1, axis=-1))
+    s = _soup(np.concatenate([q[0], t, q[1]]))
+    ds = pt.DeviceScene(s, pt.Accel(s))
+    assert ds.hierarchy_nodes > 0
+    n = 20_000
+    rng = np.random.default_rng(22)
+    r = np.concatenate([sphere_rays(np.full(3, a), np.full(3, -a), n, 23 + k) for k, a in enumerate((-0.5, -1.1, -3.0))])
+    r[::3, 4 + axis] *= 8.0           # steep
+    r[1::3, 4 + axis] *= 0.05         # grazing
+    r[::7, 4:7] = 0.0                 # along the axis
+    r[::7, 4 + axis] = np.where(rng.random(len(r[::7])) < 0.5, -1.0, 1.0)
+    r[::11, 0:3] = box[0] + (box[1] - box[0]) * rng.integers(0, 2, (len(r[::11]), 3))  # from the box's corners
+    r[::5, 3] = rng.uniform(-0.5, 1.0, len(r[::5]))
+    r[::10, 7] = r[::10, 3] + rng.uniform(0, 2.0, len(r[::10]))
+    rays = r.astype(np.float32)
+    kd, _ = gpu_trace(cuda, ds, rays, counts=True)
+    wide, _ = gpu_trace(cuda, ds, rays)
+    prim = kd[:, 1].view(np.int32)
+    assert ((prim >= 0) & (prim < 2)).any() and (prim >= s.ntri - 2).any()
+    same = np.all(kd.view(np.uint32) == wide.view(np.uint32), axis=1)
+    assert same.all(), (int((~same).sum()), rays[~same][:2], kd[~same][:2], wide[~same][:2])
+    assert np.array_equal(gpu_any(cuda, ds, rays) != 0, prim >= 0)
+
+
 @pytest.mark.parametrize("points", [1, 2, 3, 9, 40, 3000])
 @pytest.mark.parametrize("floors", [0, 1, 3])
 def test_scenes_of_which_the_root_box_leaves_out_everything(cuda, points, floors):
