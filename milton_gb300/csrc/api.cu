@@ -605,7 +605,7 @@ int scene_create(const mgpu_scene_desc *desc, const mgpu_accel *accel, void *str
   e = up(L.off_tris, tris.data(), tris.size() * sizeof(F4));
   if (e == cudaSuccess && wide) {
     if (int rc = wide_build(s->view.tris, T, s->view, base + L.off_wnodes, (F4 *)(base + L.off_wtris), base + L.off_pairs, st,
-                            &s->wide_nodes, &wide)) {
+                            &s->wide_nodes, &wide, &s->outside)) {
       cudaFree(s->d_block);
       delete s;
       return rc;

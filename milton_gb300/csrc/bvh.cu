@@ -104,6 +104,7 @@ constexpr int kCParity = 3;   // which cluster array is current
 constexpr int kCNodes = 4;    // wide nodes
 constexpr int kCTris = 5;     // triangle records
 constexpr int kCFail = 6;
+constexpr int kCOut = 7;      // a triangle sticks out
 constexpr int kCLevel = 8;    // first wide node of each level (kMaxLevels + 2)
 constexpr int kNumC = kCLevel + kMaxLevels + 8;
 
@@ -824,7 +825,9 @@ __device__ void emit_node(const Build &B, uint32_t w, bool valid, int32_t *xn, i
         const int64_t t = B.node[y].left;
         F4 a = load_f4(B.tris, 3 * t), bb = load_f4(B.tris, 3 * t + 1);
         const F4 c = load_f4(B.tris, 3 * t + 2);
-        bb.w = __uint_as_float((__float_as_uint(a.w) & 1u) | (sticks_out(B, B.node[y].box) ? kWideOutside : 0u));
+        const bool out = sticks_out(B, B.node[y].box);
+        if (out) B.ctr[kCOut] = 1u;
+        bb.w = __uint_as_float((__float_as_uint(a.w) & 1u) | (out ? kWideOutside : 0u));
         a.w = __int_as_float((int)t);
         B.wtris[3 * (size_t)at] = a;
         B.wtris[3 * (size_t)at + 1] = bb;
@@ -976,8 +979,8 @@ size_t wide_scratch(int64_t n) {
 }
 
 int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F4 *wtris, void *scratch, cudaStream_t st,
-               uint32_t *nodes_out, bool *ok) {
-  *ok = false;
+               uint32_t *nodes_out, bool *ok, bool *outside) {
+  *ok = *outside = false;
   *nodes_out = 0;
   if (n <= 0) return MGPU_OK;
   Build B;
@@ -1009,6 +1012,7 @@ int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F
   auto finished = [&]() {
     *ok = h[kCFail] == 0u && h[kCTris] == (uint32_t)n;
     *nodes_out = h[kCNodes];
+    *outside = h[kCOut] != 0u;
   };
   if (n <= kSmall) {
     e = cudaFuncSetAttribute((const void *)k_bvh_small, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -47,11 +47,11 @@ int tex_upload(const mgpu_scene_desc *desc, const TexPlan &plan, float4 *d_texre
 
 // 8-wide hierarchy over the uploaded triangles (bvh.cu): node capacity of n triangles, and the build into wnodes /
 // wtris (3 records of 16 bytes per triangle) with wide_scratch(n) bytes of scratch.  ok = false: none was
-// built (a hierarchy beyond the traversal's limits) and the kd-tree is used.
+// built (a hierarchy beyond the traversal's limits) and the kd-tree is used.  outside: a record has kWideOutside.
 int64_t wide_node_cap(int64_t ntri);
 size_t wide_scratch(int64_t n);
 int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F4 *wtris, void *scratch, cudaStream_t st,
-               uint32_t *nodes_out, bool *ok);
+               uint32_t *nodes_out, bool *ok, bool *outside);
 
 // mgpu_scene_create, without the hierarchy if the scene would exceed `limit` device bytes with it; and the device
 // bytes of a scene with it or without (api.cu)
@@ -93,6 +93,7 @@ struct mgpu_scene {
   void *d_block = nullptr;      // one allocation holding everything above
   uint64_t bytes = 0;
   uint32_t wide_nodes = 0;      // nodes of the 8-wide hierarchy, 0: none
+  bool outside = false;         // a triangle of it reaches out of the kd-tree's root box (kWideOutside)
   uint32_t *d_err = nullptr;    // device error word
 };
 

@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace(SceneView s, uint32_t nto
 // nothing from holding neighbours, and a small query ends sooner in small blocks.
 constexpr int kTraceWideBlock = 256;
 
-template <bool ANY>
+template <bool ANY, bool OUT>
 __global__ void __launch_bounds__(kTraceWideBlock, 4)
     k_trace_wide(const __grid_constant__ SceneView s, const float4 *__restrict__ rays, float4 *__restrict__ hits,
                  uint8_t *__restrict__ occ, uint32_t n) {
@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(kTraceWideBlock, 4)
     if (ANY) occ[i] = hit ? 1 : 0;
     else hits[i] = make_float4(hit ? h.t : INFINITY, __int_as_float(hit ? h.prim : -1), hit ? h.b1 : 0.0f, hit ? h.b2 : 0.0f);
   };
-  wide_trace_refill<ANY, true>([&](uint32_t) -> const SceneView & { return s; }, n, load, store,
+  wide_trace_refill<ANY, true, OUT>([&](uint32_t) -> const SceneView & { return s; }, n, load, store,
                                wsh[threadIdx.x >> 5], tables, &next);
 }
 
@@ -83,7 +83,7 @@ static int launch_trace(const mgpu_scene *s, const float *rays, float *hits, uin
   if (((uintptr_t)rays & 15) || (!ANY && ((uintptr_t)hits & 15)) || (COUNT && ((uintptr_t)counts & 15)))
     return fail(MGPU_E_INVALID, "trace: ray/hit/count buffers must be 16-byte aligned");
   if (!COUNT && s->view.wnodes != nullptr) {
-    auto kern = k_trace_wide<ANY>;
+    auto kern = s->outside ? k_trace_wide<ANY, true> : k_trace_wide<ANY, false>;
     int per_sm = 0;
     MGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kTraceWideBlock, 0));
     const int64_t grid = std::min<int64_t>((n + 31) / 32, (int64_t)device_sm_count() * std::max(per_sm, 1));
