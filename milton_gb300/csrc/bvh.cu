@@ -107,6 +107,7 @@ constexpr int kCFail = 6;
 constexpr int kCOut = 7;      // a triangle sticks out
 constexpr int kCLevel = 8;    // first wide node of each level (kMaxLevels + 2)
 constexpr int kNumC = kCLevel + kMaxLevels + 8;
+static_assert(kNumC <= kWideCounters, "the caller's counters");
 
 __device__ __forceinline__ uint32_t order_bits(float f) {
   const uint32_t u = __float_as_uint(f);
@@ -952,7 +953,6 @@ size_t place_scratch(Build &B, int64_t n, char *base) {
   const size_t radix_blocks = (N + kRadixTile - 1) / kRadixTile;
   size_t off = 0;
   auto take = [&](size_t bytes) { char *p = base + off; off += up256(bytes); return p; };
-  B.ctr = (uint32_t *)take(kNumC * 4);
   B.node = (BNode *)take(2 * N * sizeof(BNode));
   B.parent = (int32_t *)take(2 * N * 4);
   B.arrived = (uint32_t *)take(N * 4);
@@ -978,13 +978,18 @@ size_t wide_scratch(int64_t n) {
   return n > 0 ? place_scratch(B, n, nullptr) : 0;
 }
 
-int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F4 *wtris, void *scratch, cudaStream_t st,
-               uint32_t *nodes_out, bool *ok, bool *outside) {
-  *ok = *outside = false;
-  *nodes_out = 0;
+void wide_result(const uint32_t *h, int64_t n, uint32_t *nodes, bool *ok, bool *outside) {
+  *ok = h[kCFail] == 0u && h[kCTris] == (uint32_t)n;  // (a tree deeper than the traversal's stack lacks triangles)
+  *nodes = *ok ? h[kCNodes] : 0u;
+  *outside = *ok && h[kCOut] != 0u;
+}
+
+int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F4 *wtris, void *scratch, uint32_t *ctr,
+               cudaStream_t st) {
   if (n <= 0) return MGPU_OK;
   Build B;
   memset(&B, 0, sizeof(B));
+  B.ctr = ctr;
   B.n = (int32_t)n;
   B.tris = tris;
   B.wnodes = (uint32_t *)wnodes;
@@ -1009,20 +1014,14 @@ int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F
     if (r == cudaSuccess) r = cudaMemcpyAsync(h, B.ctr, sizeof(h), cudaMemcpyDeviceToHost, st);
     return r == cudaSuccess ? cudaStreamSynchronize(st) : r;
   };
-  auto finished = [&]() {
-    *ok = h[kCFail] == 0u && h[kCTris] == (uint32_t)n;
-    *nodes_out = h[kCNodes];
-    *outside = h[kCOut] != 0u;
-  };
   if (n <= kSmall) {
     e = cudaFuncSetAttribute((const void *)k_bvh_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sizeof(SmallShared));
     if (e == cudaSuccess) {
       k_bvh_small<<<1, 1024, sizeof(SmallShared), st>>>(B);
       ++launches;
-      e = counters();
+      e = cudaGetLastError();
     }
-    if (e == cudaSuccess) finished();
   } else {
     k_bvh_init<<<1, 128, 0, st>>>(B);
     k_bvh_bounds<<<grid(n, 256), 256, 0, st>>>(B);
@@ -1069,10 +1068,7 @@ int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F
           launches += 2;
         }
         e = counters();
-        if (e == cudaSuccess) {
-          more = h[kCLevel + level] != h[kCLevel + level + 1] && h[kCFail] == 0u;
-          if (!more) finished();
-        }
+        if (e == cudaSuccess) more = h[kCLevel + level] != h[kCLevel + level + 1] && h[kCFail] == 0u;
       }
     }
   }

@@ -46,12 +46,15 @@ int tex_plan(const mgpu_scene_desc *desc, TexPlan &plan);
 int tex_upload(const mgpu_scene_desc *desc, const TexPlan &plan, float4 *d_texrec, float4 *d_texels, cudaStream_t st);
 
 // 8-wide hierarchy over the uploaded triangles (bvh.cu): node capacity of n triangles, and the build into wnodes /
-// wtris (3 records of 16 bytes per triangle) with wide_scratch(n) bytes of scratch.  ok = false: none was
+// wtris (3 records of 16 bytes per triangle) with wide_scratch(n) bytes of scratch.  It may still run when the call
+// returns; wide_result tells from the kWideCounters words at ctr, copied after it, how it ended.  ok = false: none was
 // built (a hierarchy beyond the traversal's limits) and the kd-tree is used.  outside: a record has kWideOutside.
+constexpr int kWideCounters = 48;
 int64_t wide_node_cap(int64_t ntri);
 size_t wide_scratch(int64_t n);
-int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F4 *wtris, void *scratch, cudaStream_t st,
-               uint32_t *nodes_out, bool *ok, bool *outside);
+int wide_build(const F4 *tris, int64_t n, const SceneView &view, void *wnodes, F4 *wtris, void *scratch, uint32_t *ctr,
+               cudaStream_t st);
+void wide_result(const uint32_t *ctr, int64_t n, uint32_t *nodes, bool *ok, bool *outside);
 
 // mgpu_scene_create, without the hierarchy if the scene would exceed `limit` device bytes with it; and the device
 // bytes of a scene with it or without (api.cu)
