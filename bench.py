@@ -11,9 +11,9 @@ Printed JSON line (rank 0):
   value       Mpaths/s with the scene resident in HBM (device-timed, max over ranks)
   e2e         the same through the public API with host buffers: per step the scene upload
               (host -> device), the render and the film read-back (device -> host)
-  roofline    the dominant kernel's algorithmic bytes (traversal counters x bytes per node,
-              leaf reference and triangle) over its CUDA-event time, against the measured
-              HBM copy bandwidth
+  roofline    of the dominant kernel, over its CUDA-event time: L2 and DRAM traffic against their
+              measured bandwidths, busy issue slots (what bounds it), and the rate of its algorithmic bytes
+              (traversal counters x bytes per node and triangle)
   cpu_baseline  the FP64 oracle (port of Milton's PathTracer) on a bounded pixel subset
 
 `--impl reference` times the CPU implementation of the path -- the FP64 oracle port of Milton's
@@ -477,26 +477,27 @@ def run_ours(args):
     dom = max(kern, key=lambda k: kern[k][0])
     kms, kn, kbytes = kern[dom]
     achieved = (kbytes / max(kn, 1)) / ((kms / max(kn, 1)) / 1e3) / 1e9
-    # DRAM traffic per launch: the ncu capture of the same kernel on the small case gives DRAM
-    # bytes per ray (profiles/traffic_per_ray.json); scaled here by the rays of an average launch
-    traffic = None
-    l2 = None
+    # mid scene: the same kernel's DRAM and L2 bytes per ray and its busy issue slots, from ncu captures of
+    # that scene (profiles/traffic_per_ray.json), scaled by the rays of an average launch.  The algorithmic bytes
+    # are mostly L1 hits, so they are a rate ("served_gbs") and no fraction of a memory's peak; the L2
+    # carries what the L1s miss, and its measured read bandwidth (of an L2-resident buffer) is the denominator.
+    roofline = {"kernel": dom, "bound": "instruction issue", "served_gbs": achieved,
+                "bytes_per_ray": {"extend": ext_ray, "shadow": sh_ray}}
     tfile = ROOT / "profiles" / "traffic_per_ray.json"
-    if tfile.exists():
-        tr = json.loads(tfile.read_text()).get(dom, {})
-        per_ray = tr.get("dram_bytes_per_ray")
-        rays_total = ext_rays_total if dom == "extend" else sh_rays_total
-        if per_ray:
-            traffic = per_ray * rays_total / max(kn, 1)
-        # the L2 roofline: the kernel's L2 traffic (ncu lts__t_bytes per ray of the same kernel on
-        # the small case, times the rays of an average launch) over its launch time, against the
-        # measured copy bandwidth of an L2-resident buffer
-        l2_per_ray = tr.get("l2_bytes_per_ray")
-        if l2_per_ray:
-            l2_peak = _l2_read_peak()
-            l2_ach = (l2_per_ray * rays_total / max(kn, 1)) / ((kms / max(kn, 1)) / 1e3) / 1e9
-            l2 = {"achieved": l2_ach, "peak": l2_peak, "unit": "GB/s", "frac": l2_ach / l2_peak,
-                  "bytes_per_ray": l2_per_ray, "peak_source": "measured: reads of a 32 MiB L2-resident buffer, one launch"}
+    if tfile.exists() and args.workload == "mid":
+        tr = json.loads(tfile.read_text())[dom]
+        rays_per_launch = (ext_rays_total if dom == "extend" else sh_rays_total) / max(kn, 1)
+        launch_s = (kms / max(kn, 1)) / 1e3
+        l2_peak = _l2_read_peak()
+        l2_ach = tr["l2_bytes_per_ray"] * rays_per_launch / launch_s / 1e9
+        traffic = tr["dram_bytes_per_ray"] * rays_per_launch
+        roofline.update({
+            "issue_active": tr["issue_active"], "achieved": l2_ach, "peak": l2_peak, "unit": "GB/s",
+            "frac": l2_ach / l2_peak, "peak_source": "measured: reads of a 32 MiB L2-resident buffer, one launch",
+            "traffic": traffic,
+            "hbm": {"achieved": traffic / launch_s / 1e9, "peak": peaks["hbm_gbs"], "unit": "GB/s",
+                    "frac": traffic / launch_s / 1e9 / peaks["hbm_gbs"],
+                    "peak_source": peaks["source"] + " copy bandwidth"}})
 
     out = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps, "warmup": args.warmup,
@@ -512,10 +513,7 @@ def run_ours(args):
         "e2e_with_init": e2e_init,
         "gpu_launches": int(launches),
         "kernels_ms": {k: round(v[0], 3) for k, v in prof.items()},
-        "roofline": {"kernel": dom, "bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
-                     "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
-                     "peak_source": peaks["source"] + " copy bandwidth",
-                     "bytes_per_ray": {"extend": ext_ray, "shadow": sh_ray}, "l2": l2},
+        "roofline": roofline,
         "clocks": clk,
     }
     if rank == 0 and ws == 1 and not args.no_cpu_baseline:
