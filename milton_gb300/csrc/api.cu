@@ -359,16 +359,19 @@ static thread_local ReadScratch t_read;
 constexpr size_t kStageBytes = (size_t)1 << 17;
 
 // Makes the pages of a result array, while the stream still works; the array keeps its contents.  A copy by the
-// device into new memory faults page by page (24 MB: 2.0 to 7 ms).  Not by reading and writing a byte of
-// each: a page that is first mapped to read is replaced at the write, which the GPU's translations
-// wait for (9 ms).  Kernels that do not know the request refuse it, and the copy faults as before.
+// device faults at every page that is not there, at 20 us each (24 MB: 2 to 9 ms), and at pages that are but
+// that nobody has touched for a while (10 MB into memory of a result a second old: 2 to 3.4 ms, now 0.3).  So
+// they are made in one request and then touched.  (Touched by a read first, a new page would be mapped
+// twice, for reading and at the write, and the GPU's translations wait for that: 9 ms too.)  A system that
+// does not know the request refuses it, and the copy faults as before.
 static void make_pages(void *dst, size_t n) {
 #ifndef MADV_POPULATE_WRITE
   constexpr int MADV_POPULATE_WRITE = 23;
 #endif
   static const uintptr_t page = (uintptr_t)std::max(sysconf(_SC_PAGESIZE), 4096L);
   const uintptr_t first = (uintptr_t)dst / page * page, end = ((uintptr_t)dst + n + page - 1) / page * page;
-  if (n >= kStageBytes) madvise((void *)first, end - first, MADV_POPULATE_WRITE);
+  if (n < kStageBytes || madvise((void *)first, end - first, MADV_POPULATE_WRITE) != 0) return;
+  for (uintptr_t p = first; p < end; p += page) (void)*(const volatile char *)std::max(p, (uintptr_t)dst);
 }
 
 // Device memory into the caller's array; returns when it is there.  Into ordinary memory whose pages exist a GB300
