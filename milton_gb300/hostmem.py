@@ -1,6 +1,6 @@
 """Result arrays in ordinary host memory whose pages exist already, from a bounded pool.
 
-A fresh array's pages are made as it is filled (1024 x 1024 means: 1.7 ms of a read that takes 0.2 into
+A fresh array's pages have to be made first (1024 x 1024 means: 0.8 ms of a read that takes 0.3 into
 pages that exist), so the memory of a result goes back to the pool when the last numpy view of it is gone, as
 malloc would take it, but stays mapped.  It is pageable: a copy to a device has read it when the call that
 starts it returns, whatever its stream does, and forked processes have their own.  (Page-locked blocks,
